@@ -63,7 +63,7 @@ int default_piece_max(const Geometry& g, int64_t N) {
 }
 
 size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws, bool multi,
-                        int tc_maps) {
+                        int tc_maps, int fp64_maps) {
   size_t off = 0;
   auto take = [&](size_t bytes) -> uint8_t* {
     uint8_t* p = base ? base + off : nullptr;
@@ -81,8 +81,6 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
     extra = std::max<int64_t>(extra, std::max<int64_t>(2048, (direct_n + 2047) / 2048));
   }
   const int64_t pmax = std::min<int64_t>(g.nkeys, n) + extra;
-  const int tile = 128;
-  const int ntile = (g.Nx + tile - 1) / tile;
   Workspace w{};
   w.key = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * n));
   w.pay = reinterpret_cast<double*>(take(sizeof(double) * kRec * n));
@@ -106,18 +104,17 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
     w.all_flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
   }
   w.partial = reinterpret_cast<double*>(take(sizeof(double) * 8 * (size_t)g.Nl * pmax));
-  // The FP64 fold of one map, or the tensor-core route's fold digits ([Nl][2][4][4 tc_maps]
+  // The FP64 folds of a contraction pass, or the tensor-core route's fold digits ([Nl][2][4][4 tc_maps]
   // [Kp] int8), whichever is larger: a call's route uses one of them.
   w.tc_maps = std::max(1, std::min(tc_maps, kTcMaxMaps));
-  const size_t fold_bytes = sizeof(double) * 16 * (size_t)g.Nl * g.Nx;
+  const size_t fold_bytes = sizeof(double) * fold_stride(g.Nx) * (size_t)g.Nl * fp64_maps;
   const size_t fdig_bytes = (size_t)g.Nl * 8 * 4 * w.tc_maps * (size_t)digit_kp(g.Nx);
   w.fold = reinterpret_cast<double*>(take(std::max(fold_bytes, fdig_bytes)));
+  w.fp64_maps = fp64_maps;
+  w.live = take((size_t)fp64_maps * ((g.Nx + 15) / 16));
   w.cexp = reinterpret_cast<int16_t*>(take(sizeof(int16_t) * 2 * w.tc_maps));
   w.cmax = reinterpret_cast<unsigned long long*>(take(sizeof(unsigned long long) * 2 * w.tc_maps));
   w.tc_next = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
-  w.tile_live = reinterpret_cast<uint8_t*>(take(2 * (size_t)ntile));
-  w.tile_live2 = reinterpret_cast<uint8_t*>(take(2 * (size_t)((g.Nx + 255) / 256)));
-  w.alm_equ = reinterpret_cast<double*>(take(sizeof(double) * 2 * (size_t)g.Nlm));
   w.alm_pol = reinterpret_cast<double*>(take(sizeof(double) * 2 * (size_t)g.Nlm * (maps ? kMaxRot : 1)));
   w.npts = n;
   w.pmax = pmax;
@@ -179,7 +176,6 @@ Route plan_route(const dsht_plan_s* p, int64_t N) {
   // The digit tables serve tensor-core transforms at the MIXED level and every transform
   // of a plan that holds no FP64 tables; everything else contracts the FP64 tables.
   r.digits = p->tmdig && ((r.tc && p->precision == DSHT_PREC_MIXED) || !p->Yv);
-  r.streamed = r.digits || p->tm64;
   return r;
 }
 
@@ -219,7 +215,7 @@ static int build_digits(dsht_plan_s* p) {
     digits_from_rows(p, 0, g.Nlm, p->Yv, p->Yd, 0);
   } else {
     // columns m0 .. m1 - 1 with at most ~2^26 table entries per pass through the buffers
-    const int64_t cap = std::max<int64_t>((int64_t)1 << 26, (int64_t)g.Nl * g.Nx);
+    const int64_t cap = std::max<int64_t>((int64_t)1 << 26, (int64_t)g.Nl * g.pitch);
     double *tv = nullptr, *td = nullptr;
     e = cudaMalloc(&tv, sizeof(double) * cap);
     if (e == cudaSuccess) e = cudaMalloc(&td, sizeof(double) * cap);
@@ -231,7 +227,7 @@ static int build_digits(dsht_plan_s* p) {
     }
     for (int m0 = 0; m0 < g.Nl;) {
       int m1 = m0 + 1;
-      while (m1 < g.Nl && (hp_index(m1 + 1, m1 + 1, g.Nl) - hp_index(m0, m0, g.Nl)) * g.Nx <= cap) ++m1;
+      while (m1 < g.Nl && (hp_index(m1 + 1, m1 + 1, g.Nl) - hp_index(m0, m0, g.Nl)) * g.pitch <= cap) ++m1;
       const int64_t r0 = hp_index(m0, m0, g.Nl), r1 = hp_index(m1, m1, g.Nl);
       launch_tables_cols(g, m0, m1, tv, td, 0);
       digits_from_rows(p, r0, r1 - r0, tv, td, 0);
@@ -249,10 +245,16 @@ static int build_digits(dsht_plan_s* p) {
   return DSHT_OK;
 }
 
+FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol) {
+  return FoldOut{ws.fold + (size_t)k * fold_stride(g.Nx) * g.Nl, ws.live + (size_t)k * ((g.Nx + 15) / 16), equ, pol,
+                 ws.tc_next};
+}
+
 Geometry make_geometry(int Nl, int Nx, double xmax) {
   Geometry g{};
   g.Nl = Nl;
   g.Nx = Nx;
+  g.pitch = Nx + (Nx & 1);
   g.xmax = xmax;
   g.dx = xmax / (double)(Nx - 1);
   g.acos_xmax = std::acos(xmax);
@@ -288,26 +290,21 @@ int run_after_sort(dsht_plan_s* p, int64_t N, int mode, double* alm, const Works
     launch_fold_digits(g, w2, ws.cmax, ws.cexp, 0, 4, fdig, s);
     mark(DSHT_STAGE_CONTRACT);
     TcOut out{};
-    out.equ[0] = ws.alm_equ;
+    out.equ[0] = alm;
     out.pol[0] = ws.alm_pol;
     if (int rc = launch_contract_tc(g, p->tmDig, p->tc_items, p->tc_nitems, p->rexp, fdig, 4, ws.cexp, 1, out,
                                     ws.flags, ws.tc_next, s))
       return rc;
   } else {
     mark(DSHT_STAGE_FOLD);
-    launch_fold(g, w2, s);
+    FoldIn in{};
+    in.map[0] = fold_slot(g, ws, 0, alm, ws.alm_pol);
+    launch_fold(g, w2, in.map[0], s);
     mark(DSHT_STAGE_CONTRACT);
-    if (p->tm64)
-      launch_contract_stream(g, p->tmYv, p->tmYd, ws.fold, ws.tile_live2, ws.alm_equ, ws.alm_pol, ws.flags, s);
-    else
-      launch_contract_fp64(g, p->Yv, p->Yd, ws, s);
+    launch_contract_fp64(g, p->tmY64, p->tmY8, in, 1, ws.tc_next, ws.flags, s);
   }
   mark(DSHT_STAGE_ROTATE);
-  if (mode == DSHT_MODE_CALL) {
-    launch_rotate_back(g, ws.alm_pol, ws.alm_equ, alm, ws.flags, s);
-  } else {
-    DSHT_CUDA_OK(cudaMemcpyAsync(alm, ws.alm_equ, sizeof(double) * 2 * g.Nlm, cudaMemcpyDeviceToDevice, s));
-  }
+  if (mode == DSHT_MODE_CALL) launch_rotate_back(g, ws.alm_pol, alm, alm, ws.flags, s);
   mark(-1);
   if (int rc = launch_error("kernel launch")) return rc;
   DSHT_CUDA_OK(cudaGetLastError());
@@ -391,6 +388,72 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
   return DSHT_OK;
 }
 
+// Items of one class on the FP64 tables: contracted up to ws.fp64_maps per read of the table,
+// rotations batched up to kMaxRot items.
+static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<int>& list, int mode,
+                          const Workspace& ws, cudaStream_t s, int* sorted_item) {
+  const Geometry& g = p->g;
+  const int64_t nlm2 = 2 * g.Nlm;
+  const bool mixed = plan_route(p, items[list[0]].N).tc;
+  std::vector<int> pend;  // items awaiting rotation; item pend[k] in slot k
+  FoldIn in{};
+  int nfold = 0;  // folds awaiting contraction
+  for (size_t li = 0; li < list.size(); ++li) {
+    const int i = list[li];
+    const Item& item = items[i];
+    const int slot = (int)pend.size();
+    const bool more = li + 1 < list.size() && items[list[li + 1]].same_points;
+    Workspace w2 = ws;
+    w2.flags = ws.slot_flags + slot;
+    if (item.same_points && *sorted_item >= 0) {
+      prof_mark(p, DSHT_STAGE_BIN_SUMS, s);  // the weight gather counts with the bin sums
+      launch_gather(g, item.w, item.w_f32, item.N, ws, s);
+    } else {
+      prof_mark(p, DSHT_STAGE_POINTS, s);
+      // The sort keeps the input index of every slot when later items share it.
+      Workspace wp = ws;
+      wp.piece_max = plan_piece_max(p, item.N);
+      if (!more) wp.sidx = nullptr;
+      launch_points(g, item.theta, item.phi, item.w, item.w_f32, item.N, mode, wp, s, plan_uses_nufft(p, item.N));
+      *sorted_item = i;
+    }
+    prof_mark(p, DSHT_STAGE_BIN_SUMS, s);
+    DSHT_CUDA_OK(cudaMemcpyAsync(w2.flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
+    if (mixed) {
+      if (int rc = launch_bin_sums_mixed(p, w2, item.N, s)) return rc;
+    } else {
+      launch_bin_sums_fp64(g, w2, s);
+      w2.partial_f32 = 0;
+    }
+    prof_mark(p, DSHT_STAGE_FOLD, s);
+    in.map[nfold] = fold_slot(g, ws, nfold, item.alm, ws.alm_pol + nlm2 * slot);
+    launch_fold(g, w2, in.map[nfold], s);
+    ++nfold;
+    pend.push_back(i);
+    const bool rotate = pend.size() >= (size_t)kMaxRot || li + 1 == list.size();
+    if (nfold == ws.fp64_maps || rotate) {
+      prof_mark(p, DSHT_STAGE_CONTRACT, s);
+      launch_contract_fp64(g, p->tmY64, p->tmY8, in, nfold, ws.tc_next, w2.flags, s);
+      nfold = 0;
+    }
+    if (!rotate) continue;
+    RotMaps rm{};
+    StatusOut so{};
+    for (size_t k = 0; k < pend.size(); ++k) {
+      rm.rot[k] = ws.alm_pol + nlm2 * k;
+      rm.io[k] = items[pend[k]].alm;
+      rm.flags[k] = ws.slot_flags + k;
+      so.slot[k] = ws.slot_flags + k;
+      so.status[k] = items[pend[k]].status;
+    }
+    prof_mark(p, DSHT_STAGE_ROTATE, s);
+    if (mode == DSHT_MODE_CALL) launch_rotate_back_maps(g, rm, (int)pend.size(), s);
+    launch_publish_flags(so, (int)pend.size(), ws.all_flags, s);
+    pend.clear();
+  }
+  return DSHT_OK;
+}
+
 // Several transforms in one call: multi-map transforms (one point set, the later maps marked
 // same_points) and batches of independent transforms on one plan.  Each point set is
 // classified and sorted once; a same_points item only gathers its weights into the sorted
@@ -401,8 +464,6 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
 // them back.  Items with N < DSHT_MIXED_MIN_POINTS on a mixed plan run the FP64 bin sums,
 // in their own class.
 int run_items(dsht_plan_s* p, const Item* items, int n, int mode, const Workspace& ws, cudaStream_t s) {
-  const Geometry& g = p->g;
-  const int64_t nlm2 = 2 * g.Nlm;
   p->ev_n = 0;
   DSHT_CUDA_OK(cudaMemsetAsync(ws.all_flags, 0, sizeof(unsigned), s));
   // Items in two classes by the precision their size selects; same_points chains stay whole
@@ -419,68 +480,7 @@ int run_items(dsht_plan_s* p, const Item* items, int n, int mode, const Workspac
       if (rc) return rc;
       continue;
     }
-    // FP64 tables: one contraction per item, rotations batched up to kMaxRot items.
-    const bool mixed = rt.tc;
-    std::vector<int> pend;                // items awaiting rotation; item pend[k] in slot k
-    auto flush_rotation = [&]() -> int {  // rotate and publish every pending item
-      if (pend.empty()) return DSHT_OK;
-      RotMaps rm{};
-      StatusOut so{};
-      for (size_t k = 0; k < pend.size(); ++k) {
-        rm.rot[k] = ws.alm_pol + nlm2 * k;
-        rm.io[k] = items[pend[k]].alm;
-        rm.flags[k] = ws.slot_flags + k;
-        so.slot[k] = ws.slot_flags + k;
-        so.status[k] = items[pend[k]].status;
-      }
-      prof_mark(p, DSHT_STAGE_ROTATE, s);
-      if (mode == DSHT_MODE_CALL) launch_rotate_back_maps(g, rm, (int)pend.size(), s);
-      launch_publish_flags(so, (int)pend.size(), ws.all_flags, s);
-      pend.clear();
-      return DSHT_OK;
-    };
-    for (size_t li = 0; li < list.size(); ++li) {
-      const int i = list[li];
-      const Item& item = items[i];
-      const int slot = (int)pend.size();
-      Workspace w2 = ws;
-      w2.flags = ws.slot_flags + slot;
-      if (item.same_points && sorted_item >= 0) {
-        prof_mark(p, DSHT_STAGE_BIN_SUMS, s);  // the weight gather counts with the bin sums
-        launch_gather(g, item.w, item.w_f32, item.N, ws, s);
-      } else {
-        prof_mark(p, DSHT_STAGE_POINTS, s);
-        // The sort keeps the input index of every slot when later items share it.
-        Workspace wp = ws;
-        wp.piece_max = plan_piece_max(p, item.N);
-        if (!(li + 1 < list.size() && items[list[li + 1]].same_points)) wp.sidx = nullptr;
-        launch_points(g, item.theta, item.phi, item.w, item.w_f32, item.N, mode, wp, s, plan_uses_nufft(p, item.N));
-        sorted_item = i;
-      }
-      prof_mark(p, DSHT_STAGE_BIN_SUMS, s);
-      DSHT_CUDA_OK(cudaMemcpyAsync(w2.flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
-      if (mixed) {
-        if (int rc = launch_bin_sums_mixed(p, w2, item.N, s)) return rc;
-      } else {
-        launch_bin_sums_fp64(g, w2, s);
-        w2.partial_f32 = 0;
-      }
-      prof_mark(p, DSHT_STAGE_FOLD, s);
-      w2.alm_pol = ws.alm_pol + nlm2 * slot;
-      w2.alm_equ = item.alm;
-      launch_fold(g, w2, s);
-      prof_mark(p, DSHT_STAGE_CONTRACT, s);
-      if (rt.streamed)
-        launch_contract_stream(g, p->tmYv, p->tmYd, ws.fold, ws.tile_live2, w2.alm_equ, w2.alm_pol, w2.flags, s);
-      else
-        launch_contract_fp64(g, p->Yv, p->Yd, w2, s);
-      pend.push_back(i);
-      if (pend.size() >= (size_t)kMaxRot) {
-        int rc = flush_rotation();
-        if (rc) return rc;
-      }
-    }
-    int rc = flush_rotation();
+    int rc = run_class_fp64(p, items, list, mode, ws, s, &sorted_item);
     if (rc) return rc;
   }
   prof_mark(p, -1, s);
@@ -593,7 +593,7 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
     *plan = p;
     return DSHT_OK;
   } else {
-    const size_t tb = sizeof(double) * (size_t)p->g.Nlm * Nx;
+    const size_t tb = sizeof(double) * (size_t)p->g.Nlm * p->g.pitch;
     if (e == cudaSuccess) e = cudaMalloc(&p->Yv, tb);
     if (e == cudaSuccess) e = cudaMalloc(&p->Yd, tb);
     if (e != cudaSuccess) return fail(e, "plan allocation");
@@ -602,9 +602,9 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
   e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(e, "table build");
-  if (contract_stream_ok(p->g) && make_table_tmap(&p->tmYv, p->Yv, Nx, p->g.Nlm) == DSHT_OK &&
-      make_table_tmap(&p->tmYd, p->Yd, Nx, p->g.Nlm) == DSHT_OK) {
-    p->tm64 = true;
+  if (int rc = make_table_tmaps(&p->tmY64, &p->tmY8, p->Yv, p->g)) {
+    dsht_plan_destroy(p);
+    return rc;
   }
   *plan = p;
   return DSHT_OK;
@@ -740,7 +740,7 @@ static size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uin
   // maps per tensor-core contraction pass (digit tables): up to kTcMaxMaps unless tuned
   const int tc = multi ? std::min(std::max(ntrans, 1), p->tune_maps_per_pass > 0 ? p->tune_maps_per_pass
                                                                                   : kTcMaxMaps) : 1;
-  return workspace_layout(p->g, N, plan_piece_max(p, N), base, ws, multi, tc);
+  return workspace_layout(p->g, N, plan_piece_max(p, N), base, ws, multi, tc, std::min(tc, kFp64Maps));
 }
 
 // Resolves the workspace (caller's or the plan's, grown on demand) for a call.
@@ -1012,13 +1012,21 @@ static int decode_rows_to_host(dsht_plan_s* p, int which, int64_t r0, int64_t n,
   return rc;
 }
 
+// The same rows of a plan that holds the FP64 tables.
+static int table_rows_to_host(dsht_plan_s* p, int which, int64_t r0, int64_t n, double* out) {
+  const size_t width = sizeof(double) * p->g.Nx, pitch = sizeof(double) * p->g.pitch;
+  const double* t = (which == 0 ? p->Yv : p->Yd) + (size_t)r0 * p->g.pitch;
+  DSHT_CUDA_OK(cudaMemcpy2D(out, width, t, pitch, width, (size_t)n, cudaMemcpyDeviceToHost));
+  return DSHT_OK;
+}
+
 int dsht_get_row(dsht_plan_t p, int which, int ell, int m, double* out) {
   if (!p || !out || which < 0 || which > 1 || m < 0 || ell < m || ell >= p->g.Nl)
     return set_error(DSHT_ERR_INVALID, "invalid row (which=%d, l=%d, m=%d)", which, ell, m);
   const int64_t row = hp_index(ell, m, p->g.Nl);
   if (p->Yv) {
     const double* t = which == 0 ? p->Yv : p->Yd;
-    DSHT_CUDA_OK(cudaMemcpy(out, t + row * p->g.Nx, sizeof(double) * p->g.Nx, cudaMemcpyDeviceToHost));
+    DSHT_CUDA_OK(cudaMemcpy(out, t + row * p->g.pitch, sizeof(double) * p->g.Nx, cudaMemcpyDeviceToHost));
     return DSHT_OK;
   }
   return decode_rows_to_host(p, which, row, 1, out);
@@ -1026,12 +1034,7 @@ int dsht_get_row(dsht_plan_t p, int which, int ell, int m, double* out) {
 
 int dsht_get_table(dsht_plan_t p, int which, double* out) {
   if (!p || !out || which < 0 || which > 1) return set_error(DSHT_ERR_INVALID, "invalid arguments");
-  const size_t n = (size_t)p->g.Nlm * p->g.Nx;
-  if (p->Yv) {
-    const double* t = which == 0 ? p->Yv : p->Yd;
-    DSHT_CUDA_OK(cudaMemcpy(out, t, sizeof(double) * n, cudaMemcpyDeviceToHost));
-    return DSHT_OK;
-  }
+  if (p->Yv) return table_rows_to_host(p, which, 0, p->g.Nlm, out);
   return decode_rows_to_host(p, which, 0, p->g.Nlm, out);
 }
 
@@ -1055,12 +1058,9 @@ int dsht_get_table_mlayout(dsht_plan_t p, int which, double* out, int out_on_dev
     const int64_t row0 = hp_index(m, m, Nl);
     const size_t n = (size_t)(Nl - m) * Nx;
     double* dst = out + (size_t)m * plane;
-    if (p->Yv) {
-      const double* t = (which == 0 ? p->Yv : p->Yd) + (size_t)row0 * Nx;
-      DSHT_CUDA_OK(cudaMemcpy(dst, t, sizeof(double) * n, cudaMemcpyDeviceToHost));
-    } else if (int rc = decode_rows_to_host(p, which, row0, Nl - m, dst)) {
+    if (int rc = p->Yv ? table_rows_to_host(p, which, row0, Nl - m, dst)
+                       : decode_rows_to_host(p, which, row0, Nl - m, dst))
       return rc;
-    }
     std::memset(dst + n, 0, sizeof(double) * (plane - n));  // k >= Nl - m: l >= Nl (unphysical)
   }
   return DSHT_OK;

@@ -19,6 +19,7 @@
 //
 // Quantisation error of an entry: <= 2^-32 of its row's (column's) scale; a contraction sum
 // errs by at most about 2^-30 (max|T| sum|F| + max|F| sum|T|), far less for spread sets.
+#include "node_sums.cuh"
 #include "recurrence.cuh"
 
 namespace dsht {
@@ -59,14 +60,14 @@ __device__ __forceinline__ int64_t grouped_row(int l, int m, int Nl) {
 }
 
 // Row exponents of the FP64 tables rows [row0, row0 + nrows) (Healpy order, row r at
-// Y + (r - row0) * Nx): one warp per row.
-__global__ void table_rowexp_kernel(int Nl, int Nx, double dx, int64_t row0, int64_t nrows, const double* __restrict__ Yv,
+// Y + (r - row0) * pitch): one warp per row.
+__global__ void table_rowexp_kernel(int Nl, int Nx, int pitch, double dx, int64_t row0, int64_t nrows, const double* __restrict__ Yv,
                                     const double* __restrict__ Yd, int16_t* __restrict__ rexp) {
   const int lane = threadIdx.x & 31;
   const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < nrows; i += wstride) {
-    const double* v = Yv + i * Nx;
-    const double* d = Yd + i * Nx;
+    const double* v = Yv + i * pitch;
+    const double* d = Yd + i * pitch;
     double mx = 0.0;
     for (int j = lane; j < Nx; j += 32) mx = fmax(mx, fmax(fabs(v[j]), fabs(dx * d[j])));
 #pragma unroll
@@ -85,7 +86,7 @@ __global__ void table_rowexp_kernel(int Nl, int Nx, double dx, int64_t row0, int
 }
 
 // Digits of rows [row0, row0 + nrows): one thread per (row, 4 consecutive k).
-__global__ void table_digits_kernel(int Nl, int Nx, int Kp, double dx, int64_t row0, int64_t nrows,
+__global__ void table_digits_kernel(int Nl, int Nx, int pitch, int Kp, double dx, int64_t row0, int64_t nrows,
                                     const double* __restrict__ Yv, const double* __restrict__ Yd,
                                     const int16_t* __restrict__ rexp, int64_t plane, uint8_t* __restrict__ dig) {
   const int words = Kp / 4;
@@ -106,8 +107,8 @@ __global__ void table_digits_kernel(int Nl, int Nx, int Kp, double dx, int64_t r
     for (int e = 0; e < 4; ++e) {
       const int k = k0 + e;
       double v = 0.0;
-      if (k < Nx) v = Yv[i * Nx + k];
-      else if (k < 2 * Nx) v = dx * Yd[i * Nx + (k - Nx)];
+      if (k < Nx) v = Yv[i * pitch + k];
+      else if (k < 2 * Nx) v = dx * Yd[i * pitch + (k - Nx)];
       const uint32_t w = digit_word(v, sh);
 #pragma unroll
       for (int d = 0; d < 4; ++d) b[d] |= ((w >> (8 * (3 - d))) & 0xffu) << (8 * e);
@@ -181,10 +182,9 @@ fold_scale_kernel(int nbins, int Nx, const int* __restrict__ piece_first, const 
 // m fastest, so the 32 lanes of a warp store into 32 different banks.
 // Sums as fold_kernel forms them (set s: A = V0(bin j) + V2(bin j-1), B = dx (V1(bin j) +
 // V3(bin j-1)), V = vr - i vi; even rows A+ + A-, odd rows A+ - A-), stored as B/dx.
-template <typename PT>
+template <typename Src>
 __global__ void __launch_bounds__(32 * kFoldNodes, 2)
-fold_digits_kernel(int Nl, int Nx, int nbins, int Kp, const int* __restrict__ piece_first,
-                   const PT* __restrict__ partial, const unsigned long long* __restrict__ cmax,
+fold_digits_kernel(int Nl, int Nx, int Kp, const Src src, const unsigned long long* __restrict__ cmax,
                    int16_t* __restrict__ cexp, int map, int ncols, uint8_t* __restrict__ fdig) {
   // stage[row][kStageRow], row = (((par * 4 + d) * 4 + c) * 2 + kh) * 32 + m, byte j of the
   // row = node j0 + j (dynamic: 2048 rows)
@@ -200,48 +200,10 @@ fold_digits_kernel(int Nl, int Nx, int nbins, int Kp, const int* __restrict__ pi
   }
   // 2^(31 - e): the fixed-point factor of each half (exact products)
   const double f0 = ldexp(1.0, 31 - e0), f1 = ldexp(1.0, 31 - e1);
-  // Per half h (sets 2h, 2h+1): the piece ranges of the four keys feeding node j -- bin j
-  // (rows 0-3 of its pieces) and bin j - 1 (rows 4-7) of each set.  The first piece of
-  // every key is read before any further ones, so 16 loads are in flight together (most
-  // bins are one piece).  acc[set][A re, A im, B re, B im] with V = vr - i vi.
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    int pa[2][2], pb[2][2];
-#pragma unroll
-    for (int si = 0; si < 2; ++si)
-#pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        const bool ok = m < Nl && j < Nx && (b ? j >= 1 : j < nbins);
-        const int key = (2 * h + si) * nbins + j - b;
-        pa[si][b] = ok ? piece_first[key] : 0;
-        pb[si][b] = ok ? piece_first[key + 1] : 0;
-      }
     double acc[2][4];
-#pragma unroll
-    for (int si = 0; si < 2; ++si) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[si][q] = 0.0;
-#pragma unroll
-      for (int b = 0; b < 2; ++b)
-        if (pa[si][b] < pb[si][b]) {
-          const PT* v = partial + (size_t)pa[si][b] * 8 * Nl + (size_t)(4 * b) * Nl + m;
-          acc[si][0] += v[0];
-          acc[si][1] -= v[(size_t)Nl];
-          acc[si][2] += v[(size_t)2 * Nl];
-          acc[si][3] -= v[(size_t)3 * Nl];
-        }
-    }
-#pragma unroll
-    for (int si = 0; si < 2; ++si)
-#pragma unroll
-      for (int b = 0; b < 2; ++b)
-        for (int p = pa[si][b] + 1; p < pb[si][b]; ++p) {
-          const PT* v = partial + (size_t)p * 8 * Nl + (size_t)(4 * b) * Nl + m;
-          acc[si][0] += v[0];
-          acc[si][1] -= v[(size_t)Nl];
-          acc[si][2] += v[(size_t)2 * Nl];
-          acc[si][3] -= v[(size_t)3 * Nl];
-        }
+    node_sums(src, Nl, Nx, h, j, m, acc);
     const double fh = h ? f1 : f0;
     // entries (par, ri, kh): kh = 0 the A entry, 1 the B/dx entry; even rows A+ + A-, odd A+ - A-
 #pragma unroll
@@ -293,7 +255,7 @@ void launch_table_rowexp(const Geometry& g, int64_t row0, int64_t nrows, const d
   int64_t blocks = (nrows + 7) / 8;
   if (blocks > 148 * 32) blocks = 148 * 32;
   if (blocks < 1) blocks = 1;
-  table_rowexp_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.Nl, g.Nx, g.dx, row0, nrows, Yv, Yd, rexp);
+  table_rowexp_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.Nl, g.Nx, g.pitch, g.dx, row0, nrows, Yv, Yd, rexp);
   count_launches(1);
 }
 
@@ -304,7 +266,7 @@ void launch_table_digits(const Geometry& g, int64_t row0, int64_t nrows, const d
   int64_t blocks = (total + 255) / 256;
   if (blocks > 148 * 64) blocks = 148 * 64;
   if (blocks < 1) blocks = 1;
-  table_digits_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.Nl, g.Nx, Kp, g.dx, row0, nrows, Yv, Yd, rexp,
+  table_digits_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.Nl, g.Nx, g.pitch, Kp, g.dx, row0, nrows, Yv, Yd, rexp,
                                                        (int64_t)g.Nlm * Kp, dig);
   count_launches(1);
 }
@@ -332,15 +294,11 @@ void launch_fold_digits(const Geometry& g, const Workspace& ws, const unsigned l
   const int Kp = digit_kp(g.Nx);
   dim3 grid((g.Nx + kFoldNodes - 1) / kFoldNodes, (g.Nl + 31) / 32);
   constexpr int kStageBytes = 32 * 2 * 4 * 4 * 2 * kStageRow;
-  cudaFuncSetAttribute(fold_digits_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
-  cudaFuncSetAttribute(fold_digits_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
-  if (ws.partial_f32)
-    fold_digits_kernel<float><<<grid, 32 * kFoldNodes, kStageBytes, s>>>(g.Nl, g.Nx, g.nbins, Kp, ws.piece_first,
-                                                              reinterpret_cast<const float*>(ws.partial), cmax,
-                                                              cexp, map, ncols, fdig);
-  else
-    fold_digits_kernel<double><<<grid, 32 * kFoldNodes, kStageBytes, s>>>(g.Nl, g.Nx, g.nbins, Kp, ws.piece_first,
-                                                               ws.partial, cmax, cexp, map, ncols, fdig);
+  with_node_source(g, ws, [&](auto src) {
+    auto kern = fold_digits_kernel<decltype(src)>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
+    kern<<<grid, 32 * kFoldNodes, kStageBytes, s>>>(g.Nl, g.Nx, Kp, src, cmax, cexp, map, ncols, fdig);
+  });
   count_launches(1);
 }
 

@@ -6,8 +6,7 @@
 //            sorted      double [N][4]             (cos phi, sin phi, w, t) by key
 //   pieces   <= 1 bin each, <= piece_max points    (key, start, len)
 //   partial  double [piece][8][Nl]                 (k, re/im) bin sums for every m
-//   fold     double [Nl][4 q][Nx][4]               q = {equ even, equ odd, pol even, pol odd}
-//                                                  entries (A re, A im, B re, B im)
+//   fold     double [Nl][Nx/8][2 parity][8][8]     columns A, B' of eight nodes (fold.cu)
 //   alm      double2 [Nlm]                         complex128, Healpy order
 #pragma once
 
@@ -34,6 +33,8 @@ constexpr unsigned kFlagTimeout = 8u;      // a bounded wait in a tensor-core ke
 
 struct Geometry {
   int Nl, Nx;
+  int pitch;          // doubles from one FP64 table row to the next: Nx rounded up to even (TMA rows
+                      // start on 16 bytes)
   double xmax;
   double dx;          // xmax / (Nx-1), the numpy grid step  (sht/sht.py:48)
   double acos_xmax;   // numpy arccos(xmax), arccos(-xmax) (sht/sht.py:171)
@@ -51,6 +52,22 @@ struct TcOut {
   double* pol[kTcMaxMaps];
 };
 
+
+// One pass of the FP64 contraction: each map's fold, its equatorial and rotated polar alm.
+constexpr int kFp64Maps = 4;
+constexpr int kContractRows = 128;  // rows of one work item
+struct FoldOut {
+  double* fold;   // fold.cu's layout
+  uint8_t* live;  // [ceil(Nx/16)] any point feeds a node of the block of 16
+  double* equ;    // equatorial alm, rotated polar alm
+  double* pol;
+  unsigned* next_item;  // the contraction's work counter (cleared by the fold)
+};
+struct FoldIn {
+  FoldOut map[kFp64Maps];
+};
+// Doubles of one m of an FP64 fold: 16 per node, nodes in groups of eight.
+__host__ __device__ inline size_t fold_stride(int Nx) { return (size_t)((Nx + 7) / 8) * 128; }
 
 // Maps of one batched rotation: io[k] += R(rot[k]) when *flags[k] has polar points.
 constexpr int kMaxRot = 8;
@@ -83,15 +100,14 @@ struct Workspace {
   int* npieces;         // [1]
   unsigned* flags;      // [1]
   double* partial;      // [pmax][8][Nl]
-  double* fold;         // [Nl][4][Nx][4] FP64 fold; the tensor-core route's fold digits
-                        // [Nl][2][4][4 tc_maps][Kp] (int8) share this region
+  double* fold;         // FP64 folds of up to kFp64Maps maps (fold.cu); the tensor-core route's fold
+                        // digits [Nl][2][4][4 tc_maps][Kp] (int8) share this region
+  uint8_t* live;        // [fp64_maps][ceil(Nx/16)] blocks of nodes with points (FP64 folds)
+  int fp64_maps;        // maps one FP64 contraction pass can hold
   int16_t* cexp;        // [tc_maps][2] fold column scale exponents (tensor-core route)
   unsigned long long* cmax;  // [tc_maps][2] largest node |w| sum per half (bits of a double)
-  unsigned* tc_next;    // [1] work counter of the tensor-core contraction
+  unsigned* tc_next;    // [1] work counter of the contractions
   int tc_maps;          // maps one tensor-core contraction pass can hold
-  uint8_t* tile_live;   // [2][ceil(Nx/128)] tiles of the fallback contraction
-  uint8_t* tile_live2;  // [2][ceil(Nx/256)] tiles of the streaming contraction
-  double* alm_equ;      // [Nlm][2]
   double* alm_pol;      // [Nlm][2] (x nmaps for multi-map transforms)
   int64_t npts;         // N, the stride of pay
   int partial_f32;      // partial sums stored as float (tensor-core path) instead of double
@@ -103,16 +119,18 @@ struct Workspace {
 };
 
 // multi: add the records of multi-transform calls (gather indices, rotation and flag slots);
-// tc_maps: maps one tensor-core contraction pass holds (fold digit columns).
+// tc_maps: maps one tensor-core contraction pass holds (fold digit columns), fp64_maps: maps one
+// FP64 contraction pass holds.
 size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws,
-                        bool multi = false, int tc_maps = 1);
+                        bool multi = false, int tc_maps = 1, int fp64_maps = 1);
+// The fold of map k of an FP64 contraction pass and where its alm go.
+FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol);
 int default_piece_max(const Geometry& g, int64_t N);
 int plan_piece_max(const dsht_plan_s* p, int64_t N);
 // How a transform of N points runs on a plan: tensor-core bin sums (tc), tensor-core
-// contraction of the digit tables (digits), else the FP64 tables streamed by TMA (streamed)
-// or, for Nx whose rows are not 16-byte multiples, the FP64 fallback kernel.
+// contraction of the digit tables (digits), else the FP64 table streamed by TMA.
 struct Route {
-  bool tc, digits, streamed;
+  bool tc, digits;
 };
 Route plan_route(const dsht_plan_s* p, int64_t N);
 
@@ -136,8 +154,8 @@ constexpr int kNufftPiece = 8192;  // default points per piece of the NUFFT sums
 constexpr int kNufftMinPerKey = 512;  // AUTO bin sums: NUFFT from this many points per key on average
 constexpr int kFp64MaxPerKey = 28;    // AUTO bin sums: FP64 direct sums below this many per key
 int tc_inner_factor(int Nl);
-// FP64 fold of the current map into ws.fold, and the live-tile flags of the contractions.
-void launch_fold(const Geometry& g, const Workspace& ws, cudaStream_t s);
+// FP64 fold of the current map (fold.cu); clears the alm rows that two items of the contraction add to.
+void launch_fold(const Geometry& g, const Workspace& ws, const FoldOut& out, cudaStream_t s);
 // Digit tables and folds (digits.cu) and the tensor-core contraction (contract_tc.cu).
 int digit_kp(int Nx);                   // bytes per digit row: 2 Nx rounded up to 64
 constexpr int kTcMaxNx = 8192;          // S32 class sums stay below 2^31 for 2 Nx <= 16384
@@ -158,14 +176,11 @@ int launch_contract_tc(const Geometry& g, const CUtensorMap& tmA, const uint32_t
                        const int16_t* rexp, const uint8_t* fdig, int fdig_cols, const int16_t* cexp, int nmaps,
                        const TcOut& out, unsigned* flags, unsigned* next_item, cudaStream_t s);
 
-void launch_contract_fp64(const Geometry& g, const double* Yv, const double* Yd,
-                          const Workspace& ws, cudaStream_t s);
-bool contract_stream_ok(const Geometry& g);
-// FP64 tables through TMA (contract_stream.cu): alm of the fold to alm_equ / alm_pol.
-void launch_contract_stream(const Geometry& g, const CUtensorMap& tmv, const CUtensorMap& tmd, const double* fold,
-                            const uint8_t* live, double* alm_equ, double* alm_pol, unsigned* flags, cudaStream_t s);
-// 2D tensor map of an FP64 table (node x row), boxes of 256 nodes x 16 rows.
-int make_table_tmap(CUtensorMap* tm, const void* base, int Nx, int64_t Nlm);
+// FP64 contraction of the Y table (contract_fp64.cu) for nmaps <= kFp64Maps folds.
+void launch_contract_fp64(const Geometry& g, const CUtensorMap& tm64, const CUtensorMap& tm8, const FoldIn& in,
+                          int nmaps, unsigned* next_item, unsigned* flags, cudaStream_t s);
+// 2D tensor maps of an FP64 table (node x row), boxes of 16 nodes x 64 and 8 rows.
+int make_table_tmaps(CUtensorMap* tm64, CUtensorMap* tm8, const void* base, const Geometry& g);
 // An FP64 table in the JAX path's layout out[m][l - m][j] (Nl x Nl x Nx doubles, zeros
 // where l >= Nl) on the device.
 void launch_table_mlayout(const Geometry& g, const double* t64, double* out, cudaStream_t s);
@@ -218,8 +233,7 @@ struct dsht_plan_s {
   int device = 0;
   double* Yv = nullptr;  // FP64 tables (null in a compact plan)
   double* Yd = nullptr;
-  alignas(64) CUtensorMap tmYv, tmYd;
-  bool tm64 = false;
+  alignas(64) CUtensorMap tmY64, tmY8;  // boxes of 64 and 8 rows of Yv
   // Digit tables of the tensor-core contraction (digits.cu): 4 planes [Nlm][Kp] int8 in
   // rows grouped by parity, row exponents, the work items and the TMA map of the planes.
   uint8_t* dig = nullptr;

@@ -14,10 +14,10 @@ namespace {
 constexpr int kTableThreads = 256;
 
 // TO = double: the FP64 tables (the template keeps the store type explicit).
-// Columns m = m0 + blockIdx.y; row r of the tables lands at (r - row_base) * Nx.
+// Columns m = m0 + blockIdx.y; row r of the tables lands at (r - row_base) * pitch.
 template <typename TO>
 __global__ void __launch_bounds__(kTableThreads)
-table_kernel(int Nl, int Nx, double step, TO* __restrict__ Yv, TO* __restrict__ Yd, int m0, int64_t row_base) {
+table_kernel(int Nl, int Nx, int pitch, double step, TO* __restrict__ Yv, TO* __restrict__ Yd, int m0, int64_t row_base) {
   extern __shared__ double smem_raw[];
   const int m = m0 + blockIdx.y;
   Coef* cf = reinterpret_cast<Coef*>(smem_raw);       // [Nl]
@@ -33,8 +33,8 @@ table_kernel(int Nl, int Nx, double step, TO* __restrict__ Yv, TO* __restrict__ 
   const double ymm = diag_value(m, sx, smm);     // Y_mm (sht/legendre_py.py:28-30)
 
   const int64_t row0 = hp_index(m, m, Nl) - row_base;
-  TO* yv = Yv + row0 * Nx + j;
-  TO* yd = Yd + row0 * Nx + j;
+  TO* yv = Yv + row0 * pitch + j;
+  TO* yd = Yd + row0 * pitch + j;
   ColumnState st;
   double y, d;
   column_first(m, x, omx2, ymm, &st, &y, &d);
@@ -42,12 +42,12 @@ table_kernel(int Nl, int Nx, double step, TO* __restrict__ Yv, TO* __restrict__ 
   yd[0] = (TO)__dmul_rn(d, cf[m].nrm);
   if (m + 1 >= Nl) return;
   column_second(m, cf[m + 1], &st, &y, &d);
-  yv[(size_t)Nx] = (TO)__dmul_rn(y, cf[m + 1].nrm);
-  yd[(size_t)Nx] = (TO)__dmul_rn(d, cf[m + 1].nrm);
+  yv[(size_t)pitch] = (TO)__dmul_rn(y, cf[m + 1].nrm);
+  yd[(size_t)pitch] = (TO)__dmul_rn(d, cf[m + 1].nrm);
   for (int l = m + 2; l < Nl; ++l) {
     const Coef c = cf[l];
     column_step(m, l, c, &st, &y, &d);
-    const size_t off = (size_t)(l - m) * Nx;
+    const size_t off = (size_t)(l - m) * pitch;
     yv[off] = (TO)__dmul_rn(y, c.nrm);
     yd[off] = (TO)__dmul_rn(d, c.nrm);
   }
@@ -57,10 +57,10 @@ table_kernel(int Nl, int Nx, double step, TO* __restrict__ Yv, TO* __restrict__ 
 // Yv[m, l-m, :] layout with its unphysical entries nulled, sht/legendre_jax.py:14-25).
 // Grid: x over node chunks, y = k, z = m; consecutive threads take consecutive nodes.
 template <typename TI>
-__global__ void table_mlayout_kernel(int Nl, int Nx, const TI* __restrict__ t, double* __restrict__ out) {
+__global__ void table_mlayout_kernel(int Nl, int Nx, int pitch, const TI* __restrict__ t, double* __restrict__ out) {
   const int m = blockIdx.z, k = blockIdx.y;
   double* o = out + ((size_t)m * Nl + k) * Nx;
-  const TI* src = k < Nl - m ? t + (size_t)hp_index(m + k, m, Nl) * Nx : nullptr;
+  const TI* src = k < Nl - m ? t + (size_t)hp_index(m + k, m, Nl) * pitch : nullptr;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < Nx; j += gridDim.x * blockDim.x)
     o[j] = src ? (double)src[j] : 0.0;
 }
@@ -69,7 +69,7 @@ __global__ void table_mlayout_kernel(int Nl, int Nx, const TI* __restrict__ t, d
 
 void launch_table_mlayout(const Geometry& g, const double* t64, double* out, cudaStream_t s) {
   dim3 grid((g.Nx + 255) / 256 < 8 ? (g.Nx + 255) / 256 : 8, g.Nl, g.Nl);
-  table_mlayout_kernel<double><<<grid, 256, 0, s>>>(g.Nl, g.Nx, t64, out);
+  table_mlayout_kernel<double><<<grid, 256, 0, s>>>(g.Nl, g.Nx, g.pitch, t64, out);
   count_launches(1);
 }
 
@@ -78,7 +78,7 @@ static void tables_launch(const Geometry& g, TO* Yv, TO* Yd, int m0, int m1, cud
   const size_t smem = (size_t)g.Nl * sizeof(Coef) + (size_t)(g.Nl + 1) * sizeof(double);
   cudaFuncSetAttribute(table_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   dim3 grid((g.Nx + kTableThreads - 1) / kTableThreads, m1 - m0);
-  table_kernel<TO><<<grid, kTableThreads, smem, s>>>(g.Nl, g.Nx, g.dx, Yv, Yd, m0, hp_index(m0, m0, g.Nl));
+  table_kernel<TO><<<grid, kTableThreads, smem, s>>>(g.Nl, g.Nx, g.pitch, g.dx, Yv, Yd, m0, hp_index(m0, m0, g.Nl));
   count_launches(1);
 }
 

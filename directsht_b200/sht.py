@@ -42,7 +42,7 @@ class DirectSHT:
         :param precision: "fp64" (agrees with the reference to ~1e-15), "mixed" (tensor-core
             per-bin sums and a tensor-core contraction of 4-byte fixed-point copies of the
             tables: fastest, <= 1e-7 x max|alm|) or "mixed_f64_tables" (tensor-core sums, FP64
-            tables through the CUDA-core contraction).
+            tables through the FP64 contraction).
         :param compact_tables: keep only the 4-byte fixed-point tables (half the memory of the
             FP64 pair; the plan then runs at precision "mixed" only, and get_Ylm/get_dYlm return
             the stored values, within 2^-31 of each row's largest entry).

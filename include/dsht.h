@@ -91,8 +91,7 @@ enum {
  *                     normal weights: ~3e-7); the NUFFT sums have neither limit.
  *                     Plans with Nx > 8192 (or without room for the digit tables beside the
  *                     FP64 pair) contract the FP64 tables instead.
- *   DSHT_PREC_MIXED_F64_TABLES : the same bin sums with the FP64 tables streamed by the
- *                     CUDA-core contraction.
+ *   DSHT_PREC_MIXED_F64_TABLES : the same bin sums with the FP64 contraction of the FP64 table.
  * Mixed levels need Nl <= 2048; transforms of fewer than DSHT_MIXED_MIN_POINTS points run
  * the FP64 stages (they cost little, and the quantisation error of a handful of points
  * does not average down).  The rotation stays FP64 in all levels. */
@@ -111,8 +110,7 @@ int dsht_get_precision(dsht_plan_t plan, int* precision);
  * multiple of 32 in [256, 65536], 0 = chosen from N and the method (the direct sums, FP64 and
  * tensor-core, cap it at 2048; the NUFFT sums default to 8192).  DSHT_TUNE_MAPS_PER_PASS:
  * maps or point sets that share one read of the tables in a multi-transform call, 1..8,
- * 0 = the most (8; the tensor-core contraction only: the FP64 one reads the tables once per
- * map).  DSHT_TUNE_BIN_SUMS: the bin sums of the mixed levels, DSHT_BIN_SUMS_NUFFT,
+ * 0 = the most (8 with the tensor-core contraction, 4 with the FP64 one).  DSHT_TUNE_BIN_SUMS: the bin sums of the mixed levels, DSHT_BIN_SUMS_NUFFT,
  * DSHT_BIN_SUMS_TC (the direct int8-slice tensor-core sums) or DSHT_BIN_SUMS_FP64 (the direct
  * FP64 CUDA-core sums of the fp64 level); AUTO (the default) chooses per transform (so the
  * transforms of one batch call may differ) from its points per bin key on average: the
@@ -184,7 +182,7 @@ int dsht_status(unsigned flags, int mode);
  * DEVICE pointers theta[i], phi[i], w[i] (float64), alm to the DEVICE pointer alm[i]
  * (2*Nlm doubles); the pointer arrays themselves are HOST arrays read during the call.
  * Each point set is sorted on its own; the contraction serves up to 8 transforms per read
- * of the digit tables (DSHT_TUNE_MAPS_PER_PASS; one per read of FP64 tables) and the
+ * of the digit tables (up to 4 per read of the FP64 table; DSHT_TUNE_MAPS_PER_PASS) and the
  * rotation up to 8.  Results equal those of one dsht_execute per transform.  The workspace (dsht_workspace_size_batch with the
  * largest N of the batch) is used in turn by every transform.  dsht_execute_batch
  * synchronises and returns the first error of any transform; dsht_enqueue_batch does not
