@@ -63,7 +63,7 @@ int default_piece_max(const Geometry& g, int64_t N) {
 }
 
 size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws, bool multi,
-                        int tc_maps, int fp64_maps) {
+                        int tc_maps, int fp64_maps, int nu_grid) {
   size_t off = 0;
   auto take = [&](size_t bytes) -> uint8_t* {
     uint8_t* p = base ? base + off : nullptr;
@@ -76,7 +76,7 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
   // their pieces of default_piece_max(N) or at most 2048 points number at most
   // max(2048, N / 2048) beyond one per key, with N below the NUFFT threshold.
   int64_t extra = (n + piece_max - 1) / piece_max;
-  if (piece_max > 2048) {
+  if (nu_grid) {
     const int64_t direct_n = std::min<int64_t>(n, (int64_t)kNufftMinPerKey * g.nkeys);
     extra = std::max<int64_t>(extra, std::max<int64_t>(2048, (direct_n + 2047) / 2048));
   }
@@ -103,7 +103,16 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
     w.slot_flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * kMaxRot));
     w.all_flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
   }
-  w.partial = reinterpret_cast<double*>(take(sizeof(double) * 8 * (size_t)g.Nl * pmax));
+  size_t sums = 8 * (size_t)pmax;
+  if (nu_grid) {
+    w.piece_cta = reinterpret_cast<int*>(take(sizeof(int) * pmax));
+    w.cta_first = reinterpret_cast<int*>(take(sizeof(int) * (nu_grid + 1)));
+    w.node_first = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
+    // a slot per node with points, two more per CTA
+    const int64_t nodes = std::min<int64_t>(2 * std::min<int64_t>(g.nkeys, n), g.nkeys + kSets);
+    sums = std::max<size_t>(sums, 4 * (size_t)(nodes + 2 * nu_grid));
+  }
+  w.partial = reinterpret_cast<double*>(take(sizeof(double) * (size_t)g.Nl * sums));
   // The FP64 folds of a contraction pass, or the tensor-core route's fold digits ([Nl][2][4][4 tc_maps]
   // [Kp] int8), whichever is larger: a call's route uses one of them.
   w.tc_maps = std::max(1, std::min(tc_maps, kTcMaxMaps));
@@ -126,48 +135,80 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
 
 // The mixed levels' bin-sum method for one transform of N points (chosen per transform, so
 // the transforms of one batch call may differ).  AUTO compares the average points per bin
-// key with two measured crossovers: a NUFFT piece pays a fixed FFT (about 15 us of one SM at
-// Nl = 1024) and little per point, so it wins from kNufftMinPerKey points per key; the
-// tensor-core sums pay a GEMM tile and its epilogue per piece and 0.2-0.3 ns per point
-// (device-wide), the FP64 direct sums little per piece and 1-2 ns per point, so below
-// kFp64MaxPerKey points per key (pieces of a few points) the FP64 sums are the fastest.
+// key with two measured crossovers: a NUFFT node pays a fixed FFT and little per point, so it wins
+// from kNufftMinPerKey points per key; the tensor-core sums pay a GEMM tile and its epilogue per
+// piece and 0.2-0.3 ns per point (device-wide), the FP64 direct sums little per piece and 1-2 ns
+// per point, so below kFp64MaxPerKey points per key (pieces of a few points) the FP64 sums are the
+// fastest.  (The tensor-core sums quantise, so the NUFFT threshold also decides the accuracy.)
 int plan_bin_method(const dsht_plan_s* p, int64_t N) {
   const int t = p->tune_bin_sums;
   if (t == DSHT_BIN_SUMS_FP64 || t == DSHT_BIN_SUMS_TC) return t;
-  if (p->nu_dinv && (t == DSHT_BIN_SUMS_NUFFT || N >= (int64_t)kNufftMinPerKey * p->g.nkeys))
+  if (p->nu_tab[kNuMixed] && (t == DSHT_BIN_SUMS_NUFFT || N >= (int64_t)kNufftMinPerKey * p->g.nkeys))
     return DSHT_BIN_SUMS_NUFFT;
   if (t == DSHT_BIN_SUMS_AUTO && N < (int64_t)kFp64MaxPerKey * p->g.nkeys) return DSHT_BIN_SUMS_FP64;
   return DSHT_BIN_SUMS_TC;
 }
 
-bool plan_uses_nufft(const dsht_plan_s* p, int64_t N) {
-  return plan_route(p, N).tc && plan_bin_method(p, N) == DSHT_BIN_SUMS_NUFFT;
+// Accuracy class of a transform's NUFFT sums, -1 for the direct sums.
+int plan_nufft_class(const dsht_plan_s* p, int64_t N) {
+  if (plan_route(p, N).tc) return plan_bin_method(p, N) == DSHT_BIN_SUMS_NUFFT ? kNuMixed : -1;
+  if (p->precision != DSHT_PREC_FP64 || !p->nu_tab[kNuFp64] || p->tune_bin_sums == DSHT_BIN_SUMS_FP64) return -1;
+  if (p->tune_bin_sums == DSHT_BIN_SUMS_NUFFT) return kNuFp64;
+  // The direct sums cost Nl per point, a node's transform n log n: measured (full sky) equal at 45
+  // points per key for n = 4 Nl, 60-73 for n = 7 Nl, 65-110 for n = 8 Nl.
+  const int64_t n = (int64_t)1 << nufft_logn(p->g.Nl, kNuFp64);
+  return (double)N * p->g.Nl >= 11.0 * (double)n * p->g.nkeys ? kNuFp64 : -1;
 }
 
 // Pieces of the direct sums stay at or below 2048 points (the tensor path's S32 sums stay
-// exact); the NUFFT sums pay one FFT per piece, so theirs are larger.
+// exact); the NUFFT sums' at or below what their sort holds.
 int plan_piece_max(const dsht_plan_s* p, int64_t N) {
-  const bool nufft = plan_uses_nufft(p, N);
-  int pm = p->tune_piece_max > 0 ? p->tune_piece_max : nufft ? kNufftPiece : default_piece_max(p->g, N);
-  if (!nufft && pm > 2048) pm = 2048;
-  return pm;
+  const int cls = plan_nufft_class(p, N);
+  if (cls >= 0) {
+    const int most = nufft_piece(p->g.Nl, cls);
+    return p->tune_piece_max > 0 ? std::min(p->tune_piece_max, most) : most;
+  }
+  const int pm = p->tune_piece_max > 0 ? p->tune_piece_max : default_piece_max(p->g, N);
+  return std::min(pm, 2048);
 }
 
-// Bin sums of one transform of N points on the mixed route (sorted records in w2.pay).
-int launch_bin_sums_mixed(const dsht_plan_s* p, Workspace& w2, int64_t N, cudaStream_t s) {
-  switch (plan_bin_method(p, N)) {
-    case DSHT_BIN_SUMS_NUFFT:
-      w2.partial_f32 = 0;
-      return launch_bin_sums_nufft(p->g, w2, p->nu_logn, p->nu_dinv, p->nu_tw, s);
-    case DSHT_BIN_SUMS_FP64:
-      w2.partial_f32 = 0;
-      launch_piece_maxima(w2, s);  // the |w| sums (fold digit scales)
-      launch_bin_sums_fp64(p->g, w2, s);
-      return DSHT_OK;
-    default:
-      w2.partial_f32 = 1;
-      return launch_bin_sums_tc(p->g, w2, s);  // piece maxima and |w| sums first
+// Sets the workspace for a transform of N points: its piece size and its NUFFT run, if any.
+void route_workspace(const dsht_plan_s* p, int64_t N, Workspace& w) {
+  const int cls = plan_nufft_class(p, N);
+  w.piece_max = plan_piece_max(p, N);
+  w.nu_grid = cls >= 0 ? nufft_grid(p->g.Nl, cls) : 0;
+  w.nu_piece_cost = cls >= 0 ? nufft_piece_cost(p->g.Nl, cls) : 0;
+}
+
+// Bin sums of one transform of N points (sorted records in w.pay); sets w.partial_f32 to the
+// layout written.
+int launch_bin_sums(const dsht_plan_s* p, Workspace& w, int64_t N, cudaStream_t s) {
+  const Route rt = plan_route(p, N);
+  w.partial_f32 = 0;
+  if (w.nu_grid) {
+    const int cls = plan_nufft_class(p, N);
+    const NufftTables t{cls, p->nu_tab[cls], p->nu_tab[cls] + p->g.Nl + (p->g.Nl & 1)};
+    return launch_bin_sums_nufft(p->g, w, t, s);
   }
+  if (rt.tc && plan_bin_method(p, N) == DSHT_BIN_SUMS_TC) {
+    w.partial_f32 = 1;
+    return launch_bin_sums_tc(p->g, w, s);  // piece maxima and |w| sums first
+  }
+  if (rt.tc || rt.digits) launch_piece_maxima(w, s);  // the |w| sums (fold digit scales)
+  launch_bin_sums_fp64(p->g, w, s);
+  return DSHT_OK;
+}
+
+// The NUFFT tables of one class (Nl <= 2048), built once per plan.
+static int build_nufft(dsht_plan_s* p, int cls) {
+  if (p->nu_tab[cls] || p->g.Nl > 2048) return DSHT_OK;
+  std::vector<double> t, tw;
+  nufft_host_tables(p->g.Nl, cls, t, tw);
+  if (p->g.Nl & 1) t.push_back(0.0);  // the twiddles start on 16 bytes
+  t.insert(t.end(), tw.begin(), tw.end());
+  DSHT_CUDA_OK(cudaMalloc(&p->nu_tab[cls], sizeof(double) * t.size()));
+  DSHT_CUDA_OK(cudaMemcpy(p->nu_tab[cls], t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
+  return DSHT_OK;
 }
 
 Route plan_route(const dsht_plan_s* p, int64_t N) {
@@ -276,13 +317,7 @@ int run_after_sort(dsht_plan_s* p, int64_t N, int mode, double* alm, const Works
   Workspace w2 = ws;
   // Small transforms run the FP64 stages even on a mixed-precision plan.
   const Route rt = plan_route(p, N);
-  if (rt.tc) {
-    if (int rc = launch_bin_sums_mixed(p, w2, N, s)) return rc;
-  } else {
-    if (rt.digits) launch_piece_maxima(ws, s);  // the |w| sums (fold digit scales)
-    launch_bin_sums_fp64(g, ws, s);
-    w2.partial_f32 = 0;
-  }
+  if (int rc = launch_bin_sums(p, w2, N, s)) return rc;
   if (rt.digits) {
     mark(DSHT_STAGE_FOLD);
     uint8_t* fdig = reinterpret_cast<uint8_t*>(ws.fold);
@@ -316,9 +351,33 @@ int run_pipeline(dsht_plan_s* p, const double* theta, const double* phi, const d
                         int mode, double* alm, const Workspace& ws, cudaStream_t s) {
   p->ev_n = 0;
   prof_mark(p, DSHT_STAGE_POINTS, s);
-  launch_points(p->g, theta, phi, w, 0, N, mode, ws, s, plan_uses_nufft(p, N));
+  Workspace w1 = ws;
+  route_workspace(p, N, w1);
+  launch_points(p->g, theta, phi, w, 0, N, mode, w1, s);
   prof_mark(p, DSHT_STAGE_BIN_SUMS, s);
-  return run_after_sort(p, N, mode, alm, ws, s, true);
+  return run_after_sort(p, N, mode, alm, w1, s, true);
+}
+
+// The sort (or, for a further map of the sorted points, the weight gather) and the bin sums of one
+// item; w2 is the workspace its fold reads, with the item's flags in `flags`.  more: the next
+// item shares the points, so the sort keeps the input index of every slot.
+static int sort_and_sum(dsht_plan_s* p, const Item& item, bool sorted, bool more, int mode, const Workspace& ws,
+                        unsigned* flags, Workspace& w2, cudaStream_t s) {
+  w2 = ws;
+  route_workspace(p, item.N, w2);
+  if (item.same_points && sorted) {
+    prof_mark(p, DSHT_STAGE_BIN_SUMS, s);  // the weight gather counts with the bin sums
+    launch_gather(p->g, item.w, item.w_f32, item.N, ws, s);
+  } else {
+    prof_mark(p, DSHT_STAGE_POINTS, s);
+    Workspace wp = w2;
+    if (!more) wp.sidx = nullptr;
+    launch_points(p->g, item.theta, item.phi, item.w, item.w_f32, item.N, mode, wp, s);
+  }
+  prof_mark(p, DSHT_STAGE_BIN_SUMS, s);
+  DSHT_CUDA_OK(cudaMemcpyAsync(flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
+  w2.flags = flags;
+  return launch_bin_sums(p, w2, item.N, s);
 }
 
 // Items of one class on the tensor-core route: passes of up to ws.tc_maps items (at most
@@ -328,7 +387,6 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
                             const Workspace& ws, cudaStream_t s, int* sorted_item) {
   const Geometry& g = p->g;
   const int64_t nlm2 = 2 * g.Nlm;
-  const Route rt = plan_route(p, items[list[0]].N);
   const int G = std::min(ws.tc_maps, kMaxRot);
   const int fcols = 4 * ws.tc_maps;
   uint8_t* fdig = reinterpret_cast<uint8_t*>(ws.fold);
@@ -338,27 +396,9 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
     const Item& item = items[i];
     const int slot = (int)pass.size();
     Workspace w2 = ws;
-    w2.flags = ws.slot_flags + slot;
-    if (item.same_points && *sorted_item >= 0) {
-      prof_mark(p, DSHT_STAGE_BIN_SUMS, s);  // the weight gather counts with the bin sums
-      launch_gather(g, item.w, item.w_f32, item.N, ws, s);
-    } else {
-      prof_mark(p, DSHT_STAGE_POINTS, s);
-      Workspace wp = ws;
-      wp.piece_max = plan_piece_max(p, item.N);
-      if (!(li + 1 < list.size() && items[list[li + 1]].same_points)) wp.sidx = nullptr;
-      launch_points(g, item.theta, item.phi, item.w, item.w_f32, item.N, mode, wp, s, plan_uses_nufft(p, item.N));
-      *sorted_item = i;
-    }
-    prof_mark(p, DSHT_STAGE_BIN_SUMS, s);
-    DSHT_CUDA_OK(cudaMemcpyAsync(w2.flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
-    if (rt.tc) {
-      if (int rc = launch_bin_sums_mixed(p, w2, item.N, s)) return rc;
-    } else {
-      launch_piece_maxima(w2, s);
-      launch_bin_sums_fp64(g, w2, s);
-      w2.partial_f32 = 0;
-    }
+    const bool more = li + 1 < list.size() && items[list[li + 1]].same_points;
+    if (int rc = sort_and_sum(p, item, *sorted_item >= 0, more, mode, ws, ws.slot_flags + slot, w2, s)) return rc;
+    *sorted_item = i;
     prof_mark(p, DSHT_STAGE_FOLD, s);
     launch_fold_scale(g, w2, ws.cmax + 2 * slot, s);
     launch_fold_digits(g, w2, ws.cmax + 2 * slot, ws.cexp + 2 * slot, slot, fcols, fdig, s);
@@ -394,7 +434,6 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
                           const Workspace& ws, cudaStream_t s, int* sorted_item) {
   const Geometry& g = p->g;
   const int64_t nlm2 = 2 * g.Nlm;
-  const bool mixed = plan_route(p, items[list[0]].N).tc;
   std::vector<int> pend;  // items awaiting rotation; item pend[k] in slot k
   FoldIn in{};
   int nfold = 0;  // folds awaiting contraction
@@ -404,27 +443,8 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
     const int slot = (int)pend.size();
     const bool more = li + 1 < list.size() && items[list[li + 1]].same_points;
     Workspace w2 = ws;
-    w2.flags = ws.slot_flags + slot;
-    if (item.same_points && *sorted_item >= 0) {
-      prof_mark(p, DSHT_STAGE_BIN_SUMS, s);  // the weight gather counts with the bin sums
-      launch_gather(g, item.w, item.w_f32, item.N, ws, s);
-    } else {
-      prof_mark(p, DSHT_STAGE_POINTS, s);
-      // The sort keeps the input index of every slot when later items share it.
-      Workspace wp = ws;
-      wp.piece_max = plan_piece_max(p, item.N);
-      if (!more) wp.sidx = nullptr;
-      launch_points(g, item.theta, item.phi, item.w, item.w_f32, item.N, mode, wp, s, plan_uses_nufft(p, item.N));
-      *sorted_item = i;
-    }
-    prof_mark(p, DSHT_STAGE_BIN_SUMS, s);
-    DSHT_CUDA_OK(cudaMemcpyAsync(w2.flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
-    if (mixed) {
-      if (int rc = launch_bin_sums_mixed(p, w2, item.N, s)) return rc;
-    } else {
-      launch_bin_sums_fp64(g, w2, s);
-      w2.partial_f32 = 0;
-    }
+    if (int rc = sort_and_sum(p, item, *sorted_item >= 0, more, mode, ws, ws.slot_flags + slot, w2, s)) return rc;
+    *sorted_item = i;
     prof_mark(p, DSHT_STAGE_FOLD, s);
     in.map[nfold] = fold_slot(g, ws, nfold, item.alm, ws.alm_pol + nlm2 * slot);
     launch_fold(g, w2, in.map[nfold], s);
@@ -533,13 +553,23 @@ static int ensure_plan_workspace(dsht_plan_s* p, size_t bytes) {
   return DSHT_OK;
 }
 
+// Workspace of a call: single transforms use the lean layout; multi-transform calls add
+// the gather records, fold digit columns of a contraction pass, rotation and flag slots.
+size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws) {
+  // maps per tensor-core contraction pass (digit tables): up to kTcMaxMaps unless tuned
+  const int tc = multi ? std::min(std::max(ntrans, 1), p->tune_maps_per_pass > 0 ? p->tune_maps_per_pass
+                                                                                  : kTcMaxMaps) : 1;
+  const int cls = plan_nufft_class(p, N);
+  return workspace_layout(p->g, N, plan_piece_max(p, N), base, ws, multi, tc, std::min(tc, kFp64Maps),
+                          cls >= 0 ? nufft_grid(p->g.Nl, cls) : 0);
+}
+
 }  // namespace dsht
 
 using namespace dsht;
 
 
 extern "C" {
-static size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws);
 
 const char* dsht_last_error(void) { return g_last_error.c_str(); }
 
@@ -564,8 +594,6 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
   auto fail = [&](cudaError_t e, const char* what) {
     cudaFree(p->Yv);
     cudaFree(p->Yd);
-    cudaFree(p->nu_dinv);
-    cudaFree(p->nu_tw);
     cudaFreeHost(p->h_flags);
     delete p;
     cudaGetLastError();
@@ -573,19 +601,11 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
   };
   cudaError_t e = cudaMallocHost(&p->h_flags, sizeof(unsigned));
   if (e != cudaSuccess) return fail(e, "plan allocation");
-  if (Nl <= 2048) {  // the NUFFT bin sums of the mixed levels: 1/Psi(m) and the twiddles
-    std::vector<double> dinv, tw;
-    p->nu_logn = nufft_logn(Nl);
-    nufft_host_tables(Nl, p->nu_logn, dinv, tw);
-    e = cudaMalloc(&p->nu_dinv, sizeof(double) * dinv.size());
-    if (e == cudaSuccess) e = cudaMalloc(&p->nu_tw, sizeof(double) * tw.size());
-    if (e == cudaSuccess) e = cudaMemcpy(p->nu_dinv, dinv.data(), sizeof(double) * dinv.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(p->nu_tw, tw.data(), sizeof(double) * tw.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return fail(e, "plan allocation");
-  }
   if (f32_only) {
     // compact plan: the digit tables alone, built from FP64 columns a few m at a time
-    if (int rc = build_digits(p)) {
+    int rc = build_digits(p);
+    if (!rc) rc = build_nufft(p, kNuMixed);
+    if (rc) {
       dsht_plan_destroy(p);
       return rc;
     }
@@ -602,7 +622,9 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
   e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(e, "table build");
-  if (int rc = make_table_tmaps(&p->tmY64, &p->tmY8, p->Yv, p->g)) {
+  int rc = make_table_tmaps(&p->tmY64, &p->tmY8, p->Yv, p->g);
+  if (!rc) rc = build_nufft(p, kNuFp64);
+  if (rc) {
     dsht_plan_destroy(p);
     return rc;
   }
@@ -622,8 +644,8 @@ int dsht_plan_destroy(dsht_plan_t p) {
   cudaFree(p->dig);
   cudaFree(p->rexp);
   cudaFree(p->tc_items);
-  cudaFree(p->nu_dinv);
-  cudaFree(p->nu_tw);
+  cudaFree(p->nu_tab[0]);
+  cudaFree(p->nu_tab[1]);
   cudaFree(p->ws);
   cudaFree(p->in);
   cudaFree(p->alm);
@@ -641,6 +663,7 @@ int dsht_set_precision(dsht_plan_t p, int precision) {
   if (!p->Yv && precision != DSHT_PREC_MIXED)
     return set_error(DSHT_ERR_INVALID, "this plan holds compact tables only (DSHT_PLAN_F32_TABLES): precision MIXED");
   std::lock_guard<std::mutex> lock(p->mu);
+  if (int rc = build_nufft(p, precision == DSHT_PREC_FP64 ? kNuFp64 : kNuMixed)) return rc;
   // MIXED streams the digit tables through the tensor-core contraction (built on first use);
   // where they cannot be built (Nx > kTcMaxNx, or no room beside the FP64 tables) its
   // transforms contract the FP64 tables instead, as DSHT_PREC_MIXED_F64_TABLES does.
@@ -732,15 +755,6 @@ int dsht_workspace_size(dsht_plan_t p, int64_t N, size_t* bytes) {
   if (!p || !bytes || N < 0) return set_error(DSHT_ERR_INVALID, "invalid arguments");
   *bytes = call_layout(p, N, 1, false, nullptr, nullptr);
   return DSHT_OK;
-}
-
-// Workspace of a call: single transforms use the lean layout; multi-transform calls add
-// the gather records, fold digit columns of a contraction pass, rotation and flag slots.
-static size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws) {
-  // maps per tensor-core contraction pass (digit tables): up to kTcMaxMaps unless tuned
-  const int tc = multi ? std::min(std::max(ntrans, 1), p->tune_maps_per_pass > 0 ? p->tune_maps_per_pass
-                                                                                  : kTcMaxMaps) : 1;
-  return workspace_layout(p->g, N, plan_piece_max(p, N), base, ws, multi, tc, std::min(tc, kFp64Maps));
 }
 
 // Resolves the workspace (caller's or the plan's, grown on demand) for a call.
@@ -881,6 +895,7 @@ int dsht_test_point_keys(dsht_plan_t p, const double* theta, const double* phi, 
   Workspace ws;
   call_layout(p, N, 1, false, base, &ws);
   // the sort also moves weights; the keys do not depend on them, so theta stands in
+  route_workspace(p, N, ws);
   launch_points(p->g, theta, phi, theta, 0, N, mode, ws, s);
   DSHT_CUDA_OK(cudaMemcpyAsync(keys, ws.key, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, s));
   DSHT_CUDA_OK(cudaMemcpyAsync(flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
@@ -944,8 +959,7 @@ int dsht_execute_host(dsht_plan_t p, const double* theta, const double* phi, con
     return set_error(DSHT_ERR_INVALID, "invalid arguments");
   if (N == 0 && mode == DSHT_MODE_BASIC) return set_error(DSHT_ERR_EMPTY, "The theta array seems to be empty!");
   std::lock_guard<std::mutex> lock(p->mu);
-  const int piece_max = plan_piece_max(p, N);
-  const size_t need = workspace_layout(p->g, N, piece_max, nullptr, nullptr);
+  const size_t need = call_layout(p, N, 1, false, nullptr, nullptr);
   int rc = ensure_plan_workspace(p, need);
   if (rc) return rc;
   if (p->in_n < N) {
@@ -967,7 +981,7 @@ int dsht_execute_host(dsht_plan_t p, const double* theta, const double* phi, con
     DSHT_CUDA_OK(cudaMemsetAsync(p->alm, 0, sizeof(double) * 2 * p->g.Nlm, s));
   } else {
     Workspace ws;
-    workspace_layout(p->g, N, piece_max, reinterpret_cast<uint8_t*>(p->ws), &ws);
+    call_layout(p, N, 1, false, reinterpret_cast<uint8_t*>(p->ws), &ws);
     rc = run_pipeline(p, p->in, p->in + N, p->in + 2 * N, N, mode, p->alm, ws, s);
     if (rc) return rc;
     DSHT_CUDA_OK(cudaMemcpyAsync(p->h_flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToHost, s));

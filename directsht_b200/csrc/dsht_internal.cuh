@@ -98,8 +98,13 @@ struct Workspace {
   int64_t* piece_start; // [pmax]
   int* piece_len;       // [pmax]
   int* npieces;         // [1]
+  int* piece_cta;       // [pmax] NUFFT sums: the CTA that takes each piece
+  int* cta_first;       // [nu_grid + 1] first piece of every CTA
+  uint32_t* node_first; // [nkeys + 1] nodes with points before each key (those of its left node included)
+  int nu_grid;          // CTAs of the NUFFT sums (0: the direct sums of this call leave sums per piece)
+  int nu_piece_cost;    // cost of a piece in points, for their balance
   unsigned* flags;      // [1]
-  double* partial;      // [pmax][8][Nl]
+  double* partial;      // sums per piece [pmax][8][Nl], or per node slot [slot][4][Nl] (NUFFT)
   double* fold;         // FP64 folds of up to kFp64Maps maps (fold.cu); the tensor-core route's fold
                         // digits [Nl][2][4][4 tc_maps][Kp] (int8) share this region
   uint8_t* live;        // [fp64_maps][ceil(Nx/16)] blocks of nodes with points (FP64 folds)
@@ -120,9 +125,11 @@ struct Workspace {
 
 // multi: add the records of multi-transform calls (gather indices, rotation and flag slots);
 // tc_maps: maps one tensor-core contraction pass holds (fold digit columns), fp64_maps: maps one
-// FP64 contraction pass holds.
+// FP64 contraction pass holds; nu_grid: CTAs of the NUFFT sums (0: none).
 size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws,
-                        bool multi = false, int tc_maps = 1, int fp64_maps = 1);
+                        bool multi = false, int tc_maps = 1, int fp64_maps = 1, int nu_grid = 0);
+// Workspace of a call of ntrans transforms of up to N points on a plan.
+size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws);
 // The fold of map k of an FP64 contraction pass and where its alm go.
 FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol);
 int default_piece_max(const Geometry& g, int64_t N);
@@ -137,20 +144,27 @@ Route plan_route(const dsht_plan_s* p, int64_t N);
 // Kernels launched by api.cu (each file owns its launch helpers).
 void launch_tables(const Geometry& g, double* Yv, double* Yd, cudaStream_t s);
 void launch_points(const Geometry& g, const double* theta, const double* phi, const void* w, int w_f32,
-                   int64_t N, int mode, const Workspace& ws, cudaStream_t s,
-                   bool phi_record = false);
+                   int64_t N, int mode, const Workspace& ws, cudaStream_t s);
 void launch_gather(const Geometry& g, const void* w, int w_f32, int64_t N, const Workspace& ws, cudaStream_t s);
 // Largest |w h_k| of every piece of the sorted records (needed by the tensor-core sums).
 void launch_piece_maxima(const Workspace& ws, cudaStream_t s);
 void launch_publish_flags(const StatusOut& st, int n, unsigned* all, cudaStream_t s);
 void launch_bin_sums_fp64(const Geometry& g, const Workspace& ws, cudaStream_t s);
 int launch_bin_sums_tc(const Geometry& g, const Workspace& ws, cudaStream_t s);
-// NUFFT bin sums (nufft.cu): FP64 partial sums [piece][8][Nl] and the pieces' |w| sums.
-int nufft_logn(int Nl);
-void nufft_host_tables(int Nl, int logn, std::vector<double>& dinv, std::vector<double>& tw);
-int launch_bin_sums_nufft(const Geometry& g, const Workspace& ws, int logn, const double* dinv, const double* tw,
-                          cudaStream_t s);
-constexpr int kNufftPiece = 8192;  // default points per piece of the NUFFT sums
+// NUFFT node sums (nufft.cu) in two accuracy classes: sums of every node with points, and (mixed
+// class) the pieces' |w| sums.
+constexpr int kNuMixed = 0, kNuFp64 = 1;
+struct NufftTables {
+  int cls;
+  const double* dinv;  // [Nl] 1 / Psi(m); null when the plan has none
+  const double* tw;    // twiddles
+};
+int nufft_logn(int Nl, int cls);
+int nufft_grid(int Nl, int cls);
+int nufft_piece(int Nl, int cls);       // most points of a piece
+int nufft_piece_cost(int Nl, int cls);
+void nufft_host_tables(int Nl, int cls, std::vector<double>& dinv, std::vector<double>& tw);
+int launch_bin_sums_nufft(const Geometry& g, const Workspace& ws, const NufftTables& t, cudaStream_t s);
 constexpr int kNufftMinPerKey = 512;  // AUTO bin sums: NUFFT from this many points per key on average
 constexpr int kFp64MaxPerKey = 28;    // AUTO bin sums: FP64 direct sums below this many per key
 int tc_inner_factor(int Nl);
@@ -251,11 +265,9 @@ struct dsht_plan_s {
   double* alm = nullptr;  // [2 Nlm]
   unsigned* h_flags = nullptr;  // pinned
   int precision = DSHT_PREC_FP64;
-  // Type-1 NUFFT bin sums (nufft.cu): grid of 2^nu_logn cells, 1/Psi(m) [Nl] and the
-  // twiddles e^{2 pi i i/n} [n] (complex), built at plan creation for Nl <= 2048.
-  int nu_logn = 0;
-  double* nu_dinv = nullptr;
-  double* nu_tw = nullptr;
+  // NUFFT sums (nufft.cu) of the two accuracy classes: 1/Psi(m) [Nl], then the twiddles (complex),
+  // built for Nl <= 2048 at the first precision level that uses the class.
+  double* nu_tab[2] = {nullptr, nullptr};
   int tune_bin_sums = DSHT_BIN_SUMS_AUTO;
   int tune_piece_max = 0;      // points per bin piece (0: chosen from N and the method)
   int tune_maps_per_pass = 0;  // maps per multi-map contraction pass (0: the most that fit)
@@ -292,11 +304,6 @@ struct Item {
   bool same_points;
   unsigned* status;  // device word that receives the item's flags, or null
 };
-// Bin sums of a tensor-core-route transform: the NUFFT (default) or the tensor-core direct
-// sums; sets w2.partial_f32 to the layout written.
-int launch_bin_sums_mixed(const dsht_plan_s* p, Workspace& w2, int64_t N, cudaStream_t s);
-int plan_bin_method(const dsht_plan_s* p, int64_t N);
-bool plan_uses_nufft(const dsht_plan_s* p, int64_t N);
 // Runs the items in order; every finished item's flags are OR-ed into ws.all_flags.
 int run_items(dsht_plan_s* p, const Item* items, int n, int mode, const Workspace& ws, cudaStream_t s);
 // After the stream has been synchronised: fold the stage events into the plan's totals.

@@ -67,8 +67,7 @@ int dsht_execute_noalloc(dsht_plan_t p, const double* theta, const double* phi, 
   if (mode != DSHT_MODE_CALL && mode != DSHT_MODE_BASIC) return set_error(DSHT_ERR_INVALID, "bad mode %d", mode);
   if (N > (int64_t)0xfffffff0LL) return set_error(DSHT_ERR_INVALID, "too many points (%lld)", (long long)N);
   if (N == 0 && mode == DSHT_MODE_BASIC) return set_error(DSHT_ERR_EMPTY, "The theta array seems to be empty!");
-  const int piece_max = plan_piece_max(p, N);
-  const size_t need = workspace_layout(p->g, N, piece_max, nullptr, nullptr);
+  const size_t need = call_layout(p, N, 1, false, nullptr, nullptr);
   if (need > kNoAllocScratchBytes)
     return set_error(DSHT_ERR_NOMEM,
                      "dsht_execute_noalloc: Nl=%d, Nx=%d, N=%lld needs %zu bytes of scratch, more than the fixed "
@@ -83,7 +82,7 @@ int dsht_execute_noalloc(dsht_plan_t p, const double* theta, const double* phi, 
     return DSHT_OK;
   }
   Workspace ws;
-  workspace_layout(p->g, N, piece_max, reinterpret_cast<uint8_t*>(base), &ws);
+  call_layout(p, N, 1, false, reinterpret_cast<uint8_t*>(base), &ws);
   rc = run_pipeline(p, theta, phi, w, N, mode, alm, ws, s);
   if (rc) return rc;
   unsigned hf = 0;

@@ -11,8 +11,8 @@
 // exclusive scan cuts every key into pieces of at most piece_max points; the scatter pass
 // reserves a contiguous range per key and block with one global add, recomputes each
 // point's 32-byte record (cos phi, sin phi, w, t) -- one DRAM sector -- from its inputs and
-// writes it to its sorted slot; the bin-sum kernels form w h_k(t) themselves (the NUFFT bin
-// sums take the record (phi, 0, w, t) instead).  HBM bytes per point: 16 read + 4 written
+// writes it to its sorted slot; the bin-sum kernels form w h_k(t) themselves (the NUFFT sums
+// take the azimuth in turns instead of its cosine and sine).  HBM bytes per point: 16 read + 4 written
 // (count), 28 read + 32 written (scatter), against the algorithmic 24 read + 32 written.
 #include "dsht_internal.cuh"
 
@@ -224,9 +224,13 @@ count_kernel(Geometry g, int mode, const double* __restrict__ theta, const doubl
     if (hist[k]) atomicAdd(&count[k], hist[k]);
 }
 
-// Single-block exclusive scans: key offsets, pieces per key, and the piece list.
+// Single-block exclusive scans: key offsets, pieces per key, and the piece list.  Every thread
+// takes a run of consecutive keys, so one pass of block scans serves any number of keys.  For the
+// NUFFT sums also the nodes with points before each key, the CTA of every piece (equal shares
+// of points + cost x pieces) and the first piece of every CTA.
 constexpr int kScanThreads = 1024;
 
+// Exclusive scan of one value per thread; *total receives the sum.
 __device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* warp_tot, uint32_t* total) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint32_t x = v;
@@ -249,54 +253,79 @@ __device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* warp_t
     if (lane == 31) *total = s;
   }
   __syncthreads();
-  uint32_t r = x - v + warp_tot[wid];
-  __syncthreads();
-  return r;
+  return x - v + warp_tot[wid];
 }
 
 __global__ void __launch_bounds__(kScanThreads)
 scan_kernel(int nkeys, int nbins, int piece_max, int64_t pmax, const uint32_t* __restrict__ count,
             uint32_t* __restrict__ offset, uint32_t* __restrict__ cursor, int* __restrict__ piece_first,
-            int* __restrict__ piece_key, int64_t* __restrict__ piece_start, int* __restrict__ piece_len,
-            int* __restrict__ npieces) {
-  __shared__ uint32_t warp_tot[32];
-  __shared__ uint32_t total;
-  __shared__ uint32_t carry_off, carry_pc;
-  if (threadIdx.x == 0) { carry_off = 0; carry_pc = 0; }
-  __syncthreads();
-  for (int base = 0; base < nkeys; base += blockDim.x) {
-    const int k = base + threadIdx.x;
-    const uint32_t c = (k < nkeys) ? count[k] : 0u;
+            int* __restrict__ piece_key, int64_t* piece_start, int* __restrict__ piece_len,
+            int* __restrict__ npieces, uint32_t* __restrict__ node_first, int* __restrict__ piece_cta,
+            int* __restrict__ cta_first, int nu_grid, int nu_cost) {
+  __shared__ uint32_t warp_tot[3][32];
+  __shared__ uint32_t total[3];
+  const int per = (nkeys + kScanThreads - 1) / kScanThreads;
+  const int k0 = min(threadIdx.x * per, (unsigned)nkeys), k1 = min(k0 + per, nkeys);
+  // a key's new nodes: its right one, and its left one unless the bin before it has points
+  auto nodes = [&](int k, uint32_t c, uint32_t before) -> uint32_t {
+    return c == 0 ? 0u : (before != 0 && k % nbins != 0) ? 1u : 2u;
+  };
+  uint32_t sum = 0, pcs = 0, nds = 0;
+  uint32_t before = k0 > 0 && k0 < nkeys ? count[k0 - 1] : 0u;
+  for (int k = k0; k < k1; ++k) {
+    const uint32_t c = count[k];
+    sum += c;
+    pcs += (c + piece_max - 1) / piece_max;
+    nds += nodes(k, c, before);
+    before = c;
+  }
+  uint32_t o = block_scan_excl(sum, warp_tot[0], &total[0]);
+  uint32_t p = block_scan_excl(pcs, warp_tot[1], &total[1]);
+  uint32_t nd = nu_grid ? block_scan_excl(nds, warp_tot[2], &total[2]) : 0u;
+  before = k0 > 0 && k0 < nkeys ? count[k0 - 1] : 0u;
+  for (int k = k0; k < k1; ++k) {
+    const uint32_t c = count[k];
     const uint32_t pc = (c + piece_max - 1) / piece_max;
-    uint32_t o = block_scan_excl(c, warp_tot, &total);
-    const uint32_t tot_c = total;
-    uint32_t p = block_scan_excl(pc, warp_tot, &total);
-    const uint32_t tot_p = total;
-    o += carry_off;
-    p += carry_pc;
-    if (k < nkeys) {
-      offset[k] = o;
-      cursor[k] = o;
-      piece_first[k] = (int)p;
-      for (uint32_t q = 0; q < pc; ++q) {
-        const int64_t pi = (int64_t)p + q;
-        if (pi < pmax) {
-          piece_key[pi] = k;
-          piece_start[pi] = (int64_t)o + (int64_t)q * piece_max;
-          const uint32_t rem = c - q * piece_max;
-          piece_len[pi] = (int)(rem < (uint32_t)piece_max ? rem : (uint32_t)piece_max);
-        }
+    offset[k] = o;
+    cursor[k] = o;
+    piece_first[k] = (int)p;
+    if (nu_grid) {
+      node_first[k] = nd;
+      nd += nodes(k, c, before);
+    }
+    before = c;
+    for (uint32_t q = 0; q < pc; ++q) {
+      const int64_t pi = (int64_t)p + q;
+      if (pi < pmax) {
+        piece_key[pi] = k;
+        piece_start[pi] = (int64_t)o + (int64_t)q * piece_max;
+        const uint32_t rem = c - q * piece_max;
+        piece_len[pi] = (int)(rem < (uint32_t)piece_max ? rem : (uint32_t)piece_max);
       }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) { carry_off += tot_c; carry_pc += tot_p; }
-    __syncthreads();
+    o += c;
+    p += pc;
   }
+  const int np = (int)min((int64_t)total[1], pmax);
   if (threadIdx.x == 0) {
-    offset[nkeys] = carry_off;
-    piece_first[nkeys] = (int)carry_pc;
-    *npieces = (int)carry_pc;
+    offset[nkeys] = total[0];
+    piece_first[nkeys] = (int)total[1];
+    *npieces = (int)total[1];
+    if (nu_grid) node_first[nkeys] = total[2];
   }
+  if (!nu_grid) return;
+  // piece i starts at position piece_start[i] + cost i of total[0] + cost np
+  const double scale = (double)nu_grid / ((double)total[0] + (double)nu_cost * np + 1.0);
+  auto cta = [&](int i) {
+    return min(nu_grid - 1, (int)(((double)piece_start[i] + (double)nu_cost * i) * scale));
+  };
+  __syncthreads();  // the piece list is complete
+  for (int i = threadIdx.x; i < np; i += kScanThreads) {
+    const int c = cta(i);
+    piece_cta[i] = c;
+    for (int b = (i ? cta(i - 1) : -1) + 1; b <= c; ++b) cta_first[b] = i;
+  }
+  for (int b = (np ? cta(np - 1) : -1) + 1 + (int)threadIdx.x; b <= nu_grid; b += kScanThreads) cta_first[b] = np;
 }
 
 // Largest |w h_k| of a point as float bits (non-negative floats order like their bits).
@@ -308,10 +337,28 @@ __device__ __forceinline__ uint32_t gmax_bits(const double* h) {
 // to its sorted slot.  The record is recomputed from theta, phi, w and the key of the count
 // pass: for a rotated polar point the azimuth of (c, s sin p, -s cos p), kept as its cosine
 // and sine (c / rho, s sin p / rho), and t = (|x| - x_j) / dx (sht/sht.py:221).
-// PHI: the record holds (phi, 0, w, t) instead -- the azimuth itself (of the rotated point
-// for polar points, in [0, 2 pi)), which is what the NUFFT bin sums spread by; equatorial
-// points then need no sine or cosine of phi at all.
-template <typename WT, bool PHI>
+// TURN: the record holds (turn hi, turn lo, w, t) instead -- the azimuth (of the rotated point for
+// polar points) in turns, in [0, 1), as an unevaluated sum of two doubles, which is what the NUFFT
+// sums spread by: the angle keeps the precision of phi for every m.  Equatorial points then need no
+// sine or cosine of phi at all.
+__device__ __forceinline__ double2 turns(double a) {
+  constexpr double c_hi = 0x1.45f306dc9c883p-3, c_lo = -0x1.6b01ec5417056p-57;  // 1 / (2 pi)
+  if (!(fabs(a) <= 1e5)) {  // far off: the exact reduction of the library's sine and cosine
+    double s, c;
+    sincos(a, &s, &c);
+    a = atan2(s, c);
+  }
+  const double p = a * c_hi;
+  const double e = fma(a, c_hi, -p) + a * c_lo;  // a / (2 pi) = p + e
+  const double f = floor(p);
+  double hi = p - f;
+  const double bb = hi + f, tt = hi - bb;
+  const double err = (-f - tt) + (p - bb);       // the rounding of hi (two-sum)
+  if (hi >= 1.0) hi = 0.0;                       // p just below an integer
+  return make_double2(hi, e + err);
+}
+
+template <typename WT, bool TURN>
 __global__ void __launch_bounds__(kPointThreads)
 scatter_kernel(Geometry g, const double* __restrict__ theta, const double* __restrict__ phi,
                const WT* __restrict__ w, int64_t N, const uint32_t* __restrict__ keys, uint32_t* __restrict__ cursor,
@@ -352,7 +399,6 @@ scatter_kernel(Geometry g, const double* __restrict__ theta, const double* __res
   }
   __syncthreads();
   const int polar_key0 = 2 * g.nbins;
-  const double inv_dx = 1.0 / g.dx;
   for (int64_t b = lo + threadIdx.x; b < hi; b += step) {
     uint32_t k[kUnroll], pos[kUnroll];
     double th[kUnroll], ph[kUnroll], wi[kUnroll];
@@ -377,18 +423,16 @@ scatter_kernel(Geometry g, const double* __restrict__ theta, const double* __res
       double st, c, sp, cp;
       sincos(th[u], &st, &c);
       double cphi, sphi, x = c;
-      if constexpr (PHI) {
-        constexpr double two_pi = 6.28318530717958647693;
-        sphi = 0.0;
+      if constexpr (TURN) {
+        double az = ph[u];
         if ((int)k[u] >= polar_key0) {
           sincos(ph[u], &sp, &cp);
           x = -__dmul_rn(st, cp);
-          cphi = atan2(st * sp, c);  // azimuth of the rotated point (c, s sin p, -s cos p)
-        } else {
-          cphi = ph[u];
-          if (!(cphi >= 0.0 && cphi < two_pi)) cphi -= two_pi * floor(cphi / two_pi);
+          az = atan2(st * sp, c);  // azimuth of the rotated point (c, s sin p, -s cos p)
         }
-        if (cphi < 0.0) cphi += two_pi;
+        const double2 tr = turns(az);
+        cphi = tr.x;
+        sphi = tr.y;
       } else {
         sincos(ph[u], &sp, &cp);
         cphi = cp;
@@ -408,10 +452,8 @@ scatter_kernel(Geometry g, const double* __restrict__ theta, const double* __res
       }
       const int kk = (int)k[u];  // bin j = key - set nbins, without an integer division
       const int j = kk - g.nbins * ((kk >= g.nbins) + (kk >= 2 * g.nbins) + (kk >= 3 * g.nbins));
-      // t = (|x| - x_j) / dx in the reference's rounding (sht/sht.py:221); the NUFFT route
-      // (mixed levels) takes the product with 1/dx, within an ulp of it
-      const double t = PHI ? (fabs(x) - (double)j * g.dx) * inv_dx
-                           : __ddiv_rn(__dadd_rn(fabs(x), -(double)j * g.dx), g.dx);
+      // t = (|x| - x_j) / dx in the reference's rounding (sht/sht.py:221)
+      const double t = __ddiv_rn(__dadd_rn(fabs(x), -(double)j * g.dx), g.dx);
       double2* out = reinterpret_cast<double2*>(pay + (size_t)kRec * pos[u]);  // one 32-byte sector
       out[0] = make_double2(cphi, sphi);
       out[1] = make_double2(wi[u], t);
@@ -491,7 +533,7 @@ __global__ void publish_flags_kernel(const StatusOut st, int n, unsigned* all) {
 }  // namespace
 
 void launch_points(const Geometry& g, const double* theta, const double* phi, const void* w, int w_f32,
-                   int64_t N, int mode, const Workspace& ws, cudaStream_t s, bool phi_record) {
+                   int64_t N, int mode, const Workspace& ws, cudaStream_t s) {
   cudaMemsetAsync(ws.count, 0, sizeof(uint32_t) * (g.nkeys + 1), s);
   cudaMemsetAsync(ws.flags, 0, sizeof(unsigned), s);
   const size_t hsmem = sizeof(uint32_t) * g.nkeys;
@@ -509,7 +551,8 @@ void launch_points(const Geometry& g, const double* theta, const double* phi, co
   }
   scan_kernel<<<1, kScanThreads, 0, s>>>(g.nkeys, g.nbins, ws.piece_max, ws.pmax, ws.count, ws.offset,
                                          ws.cursor, ws.piece_first, ws.piece_key, ws.piece_start,
-                                         ws.piece_len, ws.npieces);
+                                         ws.piece_len, ws.npieces, ws.node_first, ws.piece_cta, ws.cta_first,
+                                         ws.nu_grid, ws.nu_piece_cost);
   count_launches(1);
   if (N > 0) {
     const int64_t blocks = (N + kScatterTile - 1) / kScatterTile;
@@ -518,7 +561,7 @@ void launch_points(const Geometry& g, const double* theta, const double* phi, co
       kern<<<(unsigned)blocks, kPointThreads, hsmem, s>>>(g, theta, phi, wp, N, ws.key, ws.cursor, ws.pay,
                                                           ws.sidx);
     };
-    if (phi_record) {
+    if (ws.nu_grid) {
       if (w_f32) go(scatter_kernel<float, true>, reinterpret_cast<const float*>(w));
       else go(scatter_kernel<double, true>, reinterpret_cast<const double*>(w));
     } else {
