@@ -339,7 +339,13 @@ int run_after_sort(dsht_plan_s* p, int64_t N, int mode, double* alm, const Works
     launch_contract_fp64(g, p->tmY64, p->tmY8, in, 1, ws.tc_next, ws.flags, s);
   }
   mark(DSHT_STAGE_ROTATE);
-  if (mode == DSHT_MODE_CALL) launch_rotate_back(g, ws.alm_pol, alm, alm, ws.flags, s);
+  if (mode == DSHT_MODE_CALL) {
+    RotMaps rm{};
+    rm.rot[0] = ws.alm_pol;
+    rm.io[0] = alm;
+    rm.flags[0] = ws.flags;
+    launch_rotate_back(g, rm, 1, rotation_tables(p->rot_tab, g.Nl), s);
+  }
   mark(-1);
   if (int rc = launch_error("kernel launch")) return rc;
   DSHT_CUDA_OK(cudaGetLastError());
@@ -421,7 +427,7 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
                                     (int)pass.size(), out, ws.slot_flags, ws.tc_next, s))
       return rc;
     prof_mark(p, DSHT_STAGE_ROTATE, s);
-    if (mode == DSHT_MODE_CALL) launch_rotate_back_maps(g, rm, (int)pass.size(), s);
+    if (mode == DSHT_MODE_CALL) launch_rotate_back(g, rm, (int)pass.size(), rotation_tables(p->rot_tab, g.Nl), s);
     launch_publish_flags(so, (int)pass.size(), ws.all_flags, s);
     pass.clear();
   }
@@ -467,7 +473,7 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
       so.status[k] = items[pend[k]].status;
     }
     prof_mark(p, DSHT_STAGE_ROTATE, s);
-    if (mode == DSHT_MODE_CALL) launch_rotate_back_maps(g, rm, (int)pend.size(), s);
+    if (mode == DSHT_MODE_CALL) launch_rotate_back(g, rm, (int)pend.size(), rotation_tables(p->rot_tab, g.Nl), s);
     launch_publish_flags(so, (int)pend.size(), ws.all_flags, s);
     pend.clear();
   }
@@ -592,6 +598,7 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
   p->g = make_geometry(Nl, Nx, xmax);
   cudaGetDevice(&p->device);
   auto fail = [&](cudaError_t e, const char* what) {
+    cudaFree(p->rot_tab);
     cudaFree(p->Yv);
     cudaFree(p->Yd);
     cudaFreeHost(p->h_flags);
@@ -600,7 +607,9 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
     return set_cuda_error(e, what, __FILE__, __LINE__);
   };
   cudaError_t e = cudaMallocHost(&p->h_flags, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc(&p->rot_tab, rotation_table_bytes(Nl));
   if (e != cudaSuccess) return fail(e, "plan allocation");
+  launch_rotation_tables(p->g, rotation_tables(p->rot_tab, Nl), 0);
   if (f32_only) {
     // compact plan: the digit tables alone, built from FP64 columns a few m at a time
     int rc = build_digits(p);
@@ -639,6 +648,7 @@ int dsht_plan_destroy(dsht_plan_t p) {
       if (p->ev[k]) cudaEventDestroy(p->ev[k]);
     delete[] p->ev;
   }
+  cudaFree(p->rot_tab);
   cudaFree(p->Yv);
   cudaFree(p->Yd);
   cudaFree(p->dig);
@@ -999,11 +1009,13 @@ int dsht_rotate_back(dsht_plan_t p, const double* alm_rot, const double* alm_add
                      void* stream) {
   if (!p || !alm_rot || !alm_out) return set_error(DSHT_ERR_INVALID, "invalid arguments");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (!alm_add) {
-    DSHT_CUDA_OK(cudaMemsetAsync(alm_out, 0, sizeof(double) * 2 * p->g.Nlm, s));
-    alm_add = alm_out;
-  }
-  launch_rotate_back(p->g, alm_rot, alm_add, alm_out, nullptr, s);
+  const size_t bytes = sizeof(double) * 2 * p->g.Nlm;
+  if (!alm_add) DSHT_CUDA_OK(cudaMemsetAsync(alm_out, 0, bytes, s));
+  else if (alm_add != alm_out) DSHT_CUDA_OK(cudaMemcpyAsync(alm_out, alm_add, bytes, cudaMemcpyDeviceToDevice, s));
+  RotMaps rm{};
+  rm.rot[0] = alm_rot;
+  rm.io[0] = alm_out;
+  launch_rotate_back(p->g, rm, 1, rotation_tables(p->rot_tab, p->g.Nl), s);
   DSHT_CUDA_OK(cudaGetLastError());
   return DSHT_OK;
 }

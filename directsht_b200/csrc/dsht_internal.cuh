@@ -198,10 +198,20 @@ int make_table_tmaps(CUtensorMap* tm64, CUtensorMap* tm8, const void* base, cons
 // An FP64 table in the JAX path's layout out[m][l - m][j] (Nl x Nl x Nx doubles, zeros
 // where l >= Nl) on the device.
 void launch_table_mlayout(const Geometry& g, const double* t64, double* out, cudaStream_t s);
-void launch_rotate_back(const Geometry& g, const double* alm_rot, const double* alm_add,
-                        double* alm_out, const unsigned* flags, cudaStream_t s);
-// alm io[k] += R(rot[k]) for k < nmaps <= kMaxRot (a map without polar points is left as it is).
-void launch_rotate_back_maps(const Geometry& g, const RotMaps& maps, int nmaps, cudaStream_t s);
+// Tables of the rotation (rotate.cu): recursion coefficients, row scales and start values of every
+// (l, k), Nl (Nl + 1) / 2 entries each.
+struct RotTables {
+  double* al;
+  double* sc;
+  double* start;
+  int* start_e;
+};
+size_t rotation_table_bytes(int Nl);
+RotTables rotation_tables(void* base, int Nl);
+void launch_rotation_tables(const Geometry& g, const RotTables& t, cudaStream_t s);
+// alm io[k] += R(rot[k]) for k < nmaps <= kMaxRot (a map without polar points is left as it is;
+// flags null: rotate anyway).
+void launch_rotate_back(const Geometry& g, const RotMaps& maps, int nmaps, const RotTables& t, cudaStream_t s);
 
 // Hint: bring [p, p + bytes) into L2 (cp.async.bulk.prefetch.L2, 16-byte aligned chunks of at
 // most 32 KB; the unaligned ends are left out).  lane, nlanes: the calling threads share the
@@ -246,6 +256,7 @@ struct dsht_plan_s {
   dsht::Geometry g;
   int device = 0;
   double* Yv = nullptr;  // FP64 tables (null in a compact plan)
+  void* rot_tab = nullptr;  // tables of the rotation (rotate.cu)
   double* Yd = nullptr;
   alignas(64) CUtensorMap tmY64, tmY8;  // boxes of 64 and 8 rows of Yv
   // Digit tables of the tensor-core contraction (digits.cu): 4 planes [Nlm][Kp] int8 in

@@ -8,10 +8,25 @@
 // This stands in for healpy's Rotator(rot=(0,90,0), eulertype='ZYZ', inv=True).rotate_alm
 // called at sht/sht.py:138-139.  d_{k,m}(pi/2) is generated per output m by the downward
 // three-term recursion in k of Trapani & Navaza (Acta Cryst. A62, 262, 2006),
-//   sqrt((l+k)(l-k+1)) d_{k-1,m} = 2m d_{k,m} - sqrt((l-k)(l+k+1)) d_{k+1,m},
+//   b_k d_{k-1,m} = 2m d_{k,m} - b_(k+1) d_{k+1,m},  b_k = sqrt((l+k)(l-k+1)),
 // from d_{l,m} = (-1)^(l-m) 2^-l sqrt(C(2l, l+m)); values below the double range are
-// carried with a binary exponent.  One CTA per l; each thread runs two interleaved output
-// columns m.  FP64 compute bound: about 5 DFMA per (l, m, m').
+// carried with a binary exponent.
+//
+// Scaling the rows by d_k = s_k e_k with b_k s_(k-1) = b_(k+1) s_(k+1) turns the recursion into
+//   e_(k-1) = 2m al_k e_k - e_(k+1),  al_k = s_k / (b_k s_(k-1)),
+// one product and one FMA per step instead of two products and an FMA, and one FMA instead of
+// three operations in its dependent chain; s_k goes into the coefficients a'.  al, s and the start
+// values depend on (l, k) alone: they are tables of the plan (28 bytes per entry, 15 MB at
+// Nl = 1024), built once with compensated products, so a call has no square roots, divisions or
+// products over k to form.
+//
+// One CTA per l (the largest first); each thread runs up to four output columns m of one parity,
+// which share every shared-memory read; one to eight maps share the recursion.  FP64 pipe bound: 3
+// operations per (l, m, m') for one map, (2 + maps) for several; at Nl = 1024 1.1e9 operations,
+// 60 us at the measured 62 per clock and SM.  Measured: one map 129 us (square roots and the start
+// column in every call, four operations: 232), eight maps 522 (827).
+#include <type_traits>
+
 #include "dsht_internal.cuh"
 
 namespace dsht {
@@ -19,336 +34,270 @@ namespace {
 
 constexpr int kRotThreads = 256;
 
-__global__ void __launch_bounds__(kRotThreads)
-rotate_back_kernel(int Nl, const double* __restrict__ alm_rot, const double* __restrict__ alm_add,
-                   double* __restrict__ alm_out, const unsigned* __restrict__ flags) {
-  extern __shared__ double sm[];
-  const int l = Nl - 1 - blockIdx.x;  // largest l first
-  const bool has_polar = (flags == nullptr) || ((*flags & kFlagHasPolar) != 0);
-  if (!has_polar) {
-    for (int m = threadIdx.x; m <= l; m += blockDim.x) {
-      const int64_t i = hp_index(l, m, Nl);
-      alm_out[2 * i] = alm_add[2 * i];
-      alm_out[2 * i + 1] = alm_add[2 * i + 1];
+// Row l of a table starts at l (l + 1) / 2; entry i stands for k = l - i.
+__host__ __device__ __forceinline__ int64_t tri(int l) { return (int64_t)l * (l + 1) / 2; }
+
+// A product of quotients num / den with its relative rounding error: (1 + err) p 2^e.
+struct Product {
+  double p = 1.0, err = 0.0;
+  int e = 0;
+  __device__ void times(const Product& o) {
+    const double n = __dmul_rn(p, o.p);
+    err += o.err + fma(p, o.p, -n) / n;
+    p = n;
+    e += o.e;
+    if (p > 0x1p64) {
+      p *= 0x1p-64;
+      e += 64;
     }
-    return;
   }
-  double* a_re = sm;                 // [l+1]
-  double* a_im = a_re + (l + 1);     // [l+1]
-  double* c1 = a_im + (l + 1);       // [l+1] sqrt((l-k)(l+k+1))
-  double* c2 = c1 + (l + 1);         // [l+1] 1/sqrt((l+k)(l-k+1))
-  double* rat = c2 + (l + 1);        // [l+1] r[k]: d_{l,k-1} = r[k] d_{l,k}
-  double* st_m = rat + (l + 1);      // [l+1] start mantissa d_{l,m}
-  int* st_e = reinterpret_cast<int*>(st_m + (l + 1));  // [l+1] start exponent
-  for (int k = threadIdx.x; k <= l; k += blockDim.x) {
-    const int64_t i = hp_index(l, k, Nl);
-    a_re[k] = alm_rot[2 * i];
-    a_im[k] = alm_rot[2 * i + 1];
-    c1[k] = sqrt((double)(l - k) * (double)(l + k + 1));
-    c2[k] = (k >= 1) ? 1.0 / sqrt((double)(l + k) * (double)(l - k + 1)) : 0.0;
-    rat[k] = (k >= 1) ? -sqrt((double)(l + k) / (double)(l - k + 1)) : 1.0;
+  __device__ void times(double num, double den) {
+    Product o;
+    o.p = __ddiv_rn(num, den);
+    o.err = fma(-o.p, den, num) / num;
+    times(o);
   }
-  __syncthreads();
-  // Start column d_{l,m} = 2^-l P(m), P(m) = prod_{k=m+1..l} r[k] (P(l) = 1).  Warp 0
-  // splits m into 32 chunks [lo, hi): T = prod_{k=lo+1..hi} r[k] links P(hi) to P(lo); an
-  // exclusive suffix product over lanes gives P(hi), and each lane walks its chunk down.
-  // Values are carried as (mantissa, binary exponent) so nothing under- or overflows.
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    auto rr = [&](int k) { return (k >= 1 && k <= l) ? rat[k] : 1.0; };
-    const int per = (l + 1 + 31) / 32;
-    const int lo = min(lane * per, l + 1), hi = min(lo + per, l + 1);
-    double tm = 1.0;
-    int te = 0;
-    for (int k = lo + 1; k <= hi; ++k) {
-      int de;
-      tm = frexp(tm * rr(k), &de);
-      te += de;
-    }
-    double pm = tm;  // inclusive suffix product over lanes >= lane
-    int pe = te;
+  // square root of 2^(2x) times the product, as a number and a binary exponent (e is a multiple of 64)
+  __device__ double root(int x, int* exponent) const {
+    *exponent = x + e / 2;
+    return sqrt(p) * (1.0 + 0.5 * err);
+  }
+};
+
+constexpr int kTabThreads = 128;
+
+// s_k and the start values of row l = blockIdx.x as running products.  Chain 0: start values
+// d_{l,m} = (-1)^(l-m) 2^-l sqrt(prod_{k=m+1..l} (l+k)/(l-k+1)); chains 1, 2: s_k for k = l, l-2, ...
+// and k = l-1, l-3, ... from s_l = s_(l-1) = 1.  Each thread multiplies a run of factors, a block
+// scan links the runs.
+__global__ void __launch_bounds__(kTabThreads)
+rotation_table_kernel(double* __restrict__ sc, double* __restrict__ start, int* __restrict__ start_e) {
+  __shared__ Product total[kTabThreads / 32];
+  const int l = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t row = tri(l);
+  for (int chain = 0; chain < 3; ++chain) {
+    // entry j of the chain stands for k; `step` multiplies by the factor between it and the next
+    const int n = chain == 0 ? l + 1 : chain == 1 ? l / 2 + 1 : (l + 1) / 2;
+    auto k_of = [&](int j) { return chain == 0 ? l - j : l - (chain - 1) - 2 * j; };
+    auto step = [&](Product& p, int j) {
+      const int k = k_of(j);
+      if (j + 1 >= n) return;
+      if (chain == 0) p.times((double)(l + k), (double)(l - k + 1));
+      // s_(k-2)^2 = s_k^2 b_k^2 / b_(k-1)^2
+      else p.times((double)(l + k) * (double)(l - k + 1), (double)(l + k - 1) * (double)(l - k + 2));
+    };
+    const int per = (n + kTabThreads - 1) / kTabThreads;
+    const int j0 = min((int)threadIdx.x * per, n), j1 = min(j0 + per, n);
+    Product p;
+    for (int j = j0; j < j1; ++j) step(p, j);
+    Product x = p;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const double om = __shfl_down_sync(0xffffffffu, pm, o);
-      const int oe = __shfl_down_sync(0xffffffffu, pe, o);
-      if (lane + o < 32) {
-        int de;
-        pm = frexp(pm * om, &de);
-        pe += oe + de;
+      Product y;
+      y.p = __shfl_up_sync(0xffffffffu, x.p, o);
+      y.err = __shfl_up_sync(0xffffffffu, x.err, o);
+      y.e = __shfl_up_sync(0xffffffffu, x.e, o);
+      if (lane >= o) x.times(y);
+    }
+    __syncthreads();
+    if (lane == 31) total[warp] = x;
+    Product run;
+    run.p = __shfl_up_sync(0xffffffffu, x.p, 1);
+    run.err = __shfl_up_sync(0xffffffffu, x.err, 1);
+    run.e = __shfl_up_sync(0xffffffffu, x.e, 1);
+    if (lane == 0) run = Product{};
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) run.times(total[w]);
+    for (int j = j0; j < j1; ++j) {
+      int e;
+      if (chain == 0) {
+        const double v = run.root(-l, &e);
+        start[row + j] = (j & 1) ? -v : v;
+        start_e[row + j] = e;
+      } else {
+        sc[row + l - k_of(j)] = run.root(0, &e);
       }
-    }
-    double vm = __shfl_down_sync(0xffffffffu, pm, 1);
-    int ve = __shfl_down_sync(0xffffffffu, pe, 1);
-    if (lane == 31) {
-      vm = 1.0;
-      ve = 0;
-    }
-    for (int m = hi - 1; m >= lo; --m) {
-      int de;
-      vm = frexp(vm * rr(m + 1), &de);
-      ve += de;
-      st_m[m] = vm;
-      st_e[m] = ve - l;
-    }
-  }
-  __syncthreads();
-  // a'_{l,k} pre-scaled by 2 (the k = 0 term has weight 1 on the real part).
-  for (int k = threadIdx.x; k <= l; k += blockDim.x) {
-    a_re[k] *= (k >= 1) ? 2.0 : 1.0;
-    a_im[k] *= 2.0;
-  }
-  __syncthreads();
-  // Output column m: d_{k,m} for k = l .. 0 by the downward recurrence.  With pi = m & 1,
-  // the terms with k = l, l-2, ... go to Re if pi == 0 and to Im if pi == 1 (l+m+k even
-  // <-> real), so each column adds alternately into acc0 (rows k = l, l-2, ...) and acc1.
-  // acc0/acc1 are kept in the recurrence's scaled units (x 2^-E) and rescaled with it.
-  const double big = 0x1p256, small = 0x1p-256;
-  const int step = 2 * blockDim.x;
-  for (int ma = threadIdx.x; ma <= l; ma += step) {
-    const int mb = ma + blockDim.x;
-    const bool hb = mb <= l;
-    const double* A0a = (ma & 1) ? a_im : a_re;  // k = l, l-2, ...
-    const double* A1a = (ma & 1) ? a_re : a_im;  // k = l-1, l-3, ...
-    const double* A0b = (mb & 1) ? a_im : a_re;
-    const double* A1b = (mb & 1) ? a_re : a_im;
-    double ca = st_m[ma], na = 0.0, cb = hb ? st_m[mb] : 0.0, nb = 0.0;
-    int Ea = st_e[ma], Eb = hb ? st_e[mb] : 0;
-    double s0a = 0.0, s1a = 0.0, s0b = 0.0, s1b = 0.0;
-    const double twoa = 2.0 * ma, twob = 2.0 * mb;
-    int k = l;
-    // Pairs (k, k-1) while k >= 1; the single k = 0 term is handled after the loop.
-    for (int it = 0; k >= 2; ++it) {
-      // row k (acc0)
-      s0a = fma(ca, A0a[k], s0a);
-      s0b = fma(cb, A0b[k], s0b);
-      double pa = (twoa * ca - c1[k] * na) * c2[k];
-      double pb = (twob * cb - c1[k] * nb) * c2[k];
-      na = ca;
-      ca = pa;
-      nb = cb;
-      cb = pb;
-      // row k-1 (acc1)
-      s1a = fma(ca, A1a[k - 1], s1a);
-      s1b = fma(cb, A1b[k - 1], s1b);
-      pa = (twoa * ca - c1[k - 1] * na) * c2[k - 1];
-      pb = (twob * cb - c1[k - 1] * nb) * c2[k - 1];
-      na = ca;
-      ca = pa;
-      nb = cb;
-      cb = pb;
-      k -= 2;
-      if ((it & 1) == 1) {  // growth per step is bounded, so checking every 4 steps is safe
-        if (fabs(ca) > big) {
-          ca *= small; na *= small; s0a *= small; s1a *= small; Ea += 256;
-        }
-        if (fabs(cb) > big) {
-          cb *= small; nb *= small; s0b *= small; s1b *= small; Eb += 256;
-        }
-      }
-    }
-    // Remaining rows: k == 1 (then 0) or k == 0.
-    if (k == 1) {
-      s0a = fma(ca, A0a[1], s0a);
-      s0b = fma(cb, A0b[1], s0b);
-      const double pa = (twoa * ca - c1[1] * na) * c2[1];
-      const double pb = (twob * cb - c1[1] * nb) * c2[1];
-      na = ca; ca = pa; nb = cb; cb = pb;
-      // k = 0 follows k = 1 in acc1's sequence (l odd): the weight-1 real term counts
-      // when l + m is even, i.e. m odd, and acc1 is then the real part.
-      s1a = fma(ca, ((ma & 1) ? a_re[0] : 0.0), s1a);
-      s1b = fma(cb, ((mb & 1) ? a_re[0] : 0.0), s1b);
-    } else {  // k == 0 in acc0's sequence (l even): counts when m is even (acc0 real)
-      s0a = fma(ca, ((ma & 1) ? 0.0 : a_re[0]), s0a);
-      s0b = fma(cb, ((mb & 1) ? 0.0 : a_re[0]), s0b);
-    }
-    const double fa = (Ea > -1074) ? ldexp(1.0, Ea) : 0.0;
-    const double fb = (Eb > -1074) ? ldexp(1.0, Eb) : 0.0;
-    // acc0 holds Re when m even, Im when m odd (and acc1 the other).
-    const double rea = ((ma & 1) ? s1a : s0a) * fa, ima = ((ma & 1) ? s0a : s1a) * fa;
-    {
-      const int64_t i = hp_index(l, ma, Nl);
-      alm_out[2 * i] = alm_add[2 * i] + rea;
-      alm_out[2 * i + 1] = alm_add[2 * i + 1] + ima;
-    }
-    if (hb) {
-      const double reb = ((mb & 1) ? s1b : s0b) * fb, imb = ((mb & 1) ? s0b : s1b) * fb;
-      const int64_t i = hp_index(l, mb, Nl);
-      alm_out[2 * i] = alm_add[2 * i] + reb;
-      alm_out[2 * i + 1] = alm_add[2 * i + 1] + imb;
+      step(run, j);
     }
   }
 }
 
-// Several maps per CTA (kMaps of them, map index blockIdx.y * kMaps + g): the d_{k,m}
-// recurrence of a column is shared by all maps, each map adds its own two sums, so the
-// cost per map falls from about 5 to about 2 DFMA per (l, m, m').  One column per thread;
-// io[map] += R(rot[map]) in place; a map whose flags show no polar point is skipped (its
-// rotated alm are zero).
-template <int kMaps>
-__global__ void __launch_bounds__(kRotThreads)
-rotate_back_maps_kernel(int Nl, int nmaps, const RotMaps maps) {
-  extern __shared__ double sm[];
-  const int l = Nl - 1 - blockIdx.x;
-  const int map0 = blockIdx.y * kMaps;
-  const int nm = min(kMaps, nmaps - map0);
-  double* a_re = sm;                         // [kMaps][l+1]
-  double* a_im = a_re + kMaps * (l + 1);     // [kMaps][l+1]
-  double* c1 = a_im + kMaps * (l + 1);
-  double* c2 = c1 + (l + 1);
-  double* rat = c2 + (l + 1);
-  double* st_m = rat + (l + 1);
-  int* st_e = reinterpret_cast<int*>(st_m + (l + 1));
-  for (int k = threadIdx.x; k <= l; k += blockDim.x) {
-    const int64_t i = hp_index(l, k, Nl);
+__global__ void rotation_alpha_kernel(int Nl, const double* __restrict__ sc, double* __restrict__ al) {
+  const int l = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x, k = l - i;
+  if (i > l) return;
+  const int64_t at = tri(l) + i;
+  al[at] = k >= 1 ? sc[at] / (sqrt((double)(l + k) * (double)(l - k + 1)) * sc[at + 1]) : 0.0;
+}
+
+// Columns m = m0, m0 + blockDim, ... (C of them, one parity) of degree l: io[map] += R(rot[map]).
+// al: [i], S: [map][i] the coefficients of this parity's alternating real and imaginary rows, both
+// padded with zeros.
+template <int kMaps, int C>
+__device__ __forceinline__ void rotate_columns(int Nl, int l, int m0, int map0, int nm, const RotMaps& maps,
+                                               const double* al, const double* S, int stride,
+                                               const double* __restrict__ start, const int* __restrict__ start_e) {
+  double c[C], n[C], m2[C], s[C][kMaps][2];
+  int E[C];
 #pragma unroll
-    for (int g = 0; g < kMaps; ++g) {
-      const bool ok = g < nm && (!maps.flags[map0 + g] || (*maps.flags[map0 + g] & kFlagHasPolar));
-      const double* src = maps.rot[ok ? map0 + g : 0];
-      a_re[g * (l + 1) + k] = ok ? src[2 * i] * ((k >= 1) ? 2.0 : 1.0) : 0.0;
-      a_im[g * (l + 1) + k] = ok ? src[2 * i + 1] * 2.0 : 0.0;
-    }
-    c1[k] = sqrt((double)(l - k) * (double)(l + k + 1));
-    c2[k] = (k >= 1) ? 1.0 / sqrt((double)(l + k) * (double)(l - k + 1)) : 0.0;
-    rat[k] = (k >= 1) ? -sqrt((double)(l + k) / (double)(l - k + 1)) : 1.0;
+  for (int j = 0; j < C; ++j) {
+    const int m = m0 + j * kRotThreads;
+    const bool in = m <= l;
+    c[j] = in ? start[tri(l) + l - m] : 0.0;
+    E[j] = in ? start_e[tri(l) + l - m] : 0;
+    n[j] = 0.0;
+    m2[j] = 2.0 * m;
+#pragma unroll
+    for (int g = 0; g < kMaps; ++g) s[j][g][0] = s[j][g][1] = 0.0;
   }
-  __syncthreads();
-  if (threadIdx.x < 32) {  // start column, as in rotate_back_kernel
-    const int lane = threadIdx.x;
-    auto rr = [&](int k) { return (k >= 1 && k <= l) ? rat[k] : 1.0; };
-    const int per = (l + 1 + 31) / 32;
-    const int lo = min(lane * per, l + 1), hi = min(lo + per, l + 1);
-    double tm = 1.0;
-    int te = 0;
-    for (int k = lo + 1; k <= hi; ++k) {
-      int de;
-      tm = frexp(tm * rr(k), &de);
-      te += de;
-    }
-    double pm = tm;
-    int pe = te;
+  // two steps at a time, the next two's values loaded meanwhile (the arrays end in a spare group)
+  double2 an = *reinterpret_cast<const double2*>(al), vn[kMaps];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double om = __shfl_down_sync(0xffffffffu, pm, o);
-      const int oe = __shfl_down_sync(0xffffffffu, pe, o);
-      if (lane + o < 32) {
-        int de;
-        pm = frexp(pm * om, &de);
-        pe += oe + de;
+  for (int g = 0; g < kMaps; ++g) vn[g] = *reinterpret_cast<const double2*>(S + g * stride);
+  for (int i = 0; i <= l; i += 4) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double2 a = an;
+      double2 v[kMaps];
+      an = *reinterpret_cast<const double2*>(al + i + 2 * h + 2);
+#pragma unroll
+      for (int g = 0; g < kMaps; ++g) {
+        v[g] = vn[g];
+        vn[g] = *reinterpret_cast<const double2*>(S + g * stride + i + 2 * h + 2);
+      }
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+#pragma unroll
+        for (int g = 0; g < kMaps; ++g) s[j][g][0] = fma(c[j], v[g].x, s[j][g][0]);
+        const double p = fma(m2[j] * a.x, c[j], -n[j]);
+#pragma unroll
+        for (int g = 0; g < kMaps; ++g) s[j][g][1] = fma(p, v[g].y, s[j][g][1]);
+        n[j] = p;
+        c[j] = fma(m2[j] * a.y, p, -c[j]);
       }
     }
-    double vm = __shfl_down_sync(0xffffffffu, pm, 1);
-    int ve = __shfl_down_sync(0xffffffffu, pe, 1);
-    if (lane == 31) {
-      vm = 1.0;
-      ve = 0;
-    }
-    for (int m = hi - 1; m >= lo; --m) {
-      int de;
-      vm = frexp(vm * rr(m + 1), &de);
-      ve += de;
-      st_m[m] = vm;
-      st_e[m] = ve - l;
-    }
-  }
-  __syncthreads();
-  const double big = 0x1p256, small = 0x1p-256;
-  const int L1 = l + 1;
-  for (int m = threadIdx.x; m <= l; m += blockDim.x) {
-    // rows k = l, l-2, ... read A0 (Re when m even), rows l-1, l-3, ... read A1.
-    const double* A0 = (m & 1) ? a_im : a_re;
-    const double* A1 = (m & 1) ? a_re : a_im;
-    double c = st_m[m], n = 0.0;
-    int E = st_e[m];
-    double s0[kMaps], s1[kMaps];
+    // the growth of four steps is bounded, so a check every four is safe (on the exponent bits)
 #pragma unroll
-    for (int g = 0; g < kMaps; ++g) s0[g] = s1[g] = 0.0;
-    const double two_m = 2.0 * m;
-    int k = l;
-    for (int it = 0; k >= 2; ++it) {
-#pragma unroll
-      for (int g = 0; g < kMaps; ++g) s0[g] = fma(c, A0[g * L1 + k], s0[g]);
-      double p = (two_m * c - c1[k] * n) * c2[k];
-      n = c;
-      c = p;
-#pragma unroll
-      for (int g = 0; g < kMaps; ++g) s1[g] = fma(c, A1[g * L1 + k - 1], s1[g]);
-      p = (two_m * c - c1[k - 1] * n) * c2[k - 1];
-      n = c;
-      c = p;
-      k -= 2;
-      if ((it & 1) == 1 && fabs(c) > big) {
-        c *= small;
-        n *= small;
+    for (int j = 0; j < C; ++j)
+      if ((__double2hiint(c[j]) & 0x7fffffff) > 0x4ff00000) {  // |c| >= 2^256
+        c[j] *= 0x1p-256;
+        n[j] *= 0x1p-256;
 #pragma unroll
         for (int g = 0; g < kMaps; ++g) {
-          s0[g] *= small;
-          s1[g] *= small;
+          s[j][g][0] *= 0x1p-256;
+          s[j][g][1] *= 0x1p-256;
         }
-        E += 256;
+        E[j] += 256;
       }
-    }
-    if (k == 1) {
+  }
 #pragma unroll
-      for (int g = 0; g < kMaps; ++g) s0[g] = fma(c, A0[g * L1 + 1], s0[g]);
-      const double p = (two_m * c - c1[1] * n) * c2[1];
-      n = c;
-      c = p;
-      if (m & 1) {
-#pragma unroll
-        for (int g = 0; g < kMaps; ++g) s1[g] = fma(c, a_re[g * L1], s1[g]);
-      }
-    } else if (!(m & 1)) {
-#pragma unroll
-      for (int g = 0; g < kMaps; ++g) s0[g] = fma(c, a_re[g * L1], s0[g]);
-    }
-    const double f = (E > -1074) ? ldexp(1.0, E) : 0.0;
-    const int64_t i = hp_index(l, m, Nl);
+  for (int j = 0; j < C; ++j) {
+    const int m = m0 + j * kRotThreads;
+    if (m > l) continue;
+    const double f = (E[j] > -1074) ? ldexp(1.0, E[j]) : 0.0;
+    const int64_t at = 2 * hp_index(l, m, Nl);
 #pragma unroll
     for (int g = 0; g < kMaps; ++g) {
       if (g < nm && (!maps.flags[map0 + g] || (*maps.flags[map0 + g] & kFlagHasPolar))) {
         double* out = maps.io[map0 + g];
-        const double re = ((m & 1) ? s1[g] : s0[g]) * f, im = ((m & 1) ? s0[g] : s1[g]) * f;
-        out[2 * i] += re;
-        out[2 * i + 1] += im;
+        out[at] += ((m & 1) ? s[j][g][1] : s[j][g][0]) * f;
+        out[at + 1] += ((m & 1) ? s[j][g][0] : s[j][g][1]) * f;
       }
     }
   }
 }
 
+// Maps blockIdx.y kMaps + g of degree l = Nl - 1 - blockIdx.x; a map without polar points is skipped
+// (its rotated alm are zero).  C: most columns per thread at a time.
+template <int kMaps, int C>
+__global__ void __launch_bounds__(kRotThreads)
+rotate_back_kernel(int Nl, int nmaps, const RotMaps maps, const double* __restrict__ al_t,
+                   const double* __restrict__ sc_t, const double* __restrict__ start,
+                   const int* __restrict__ start_e) {
+  extern __shared__ __align__(16) double sm[];
+  const int l = Nl - 1 - blockIdx.x;
+  const int map0 = blockIdx.y * kMaps;
+  const int nm = min(kMaps, nmaps - map0);
+  bool any = false;
+#pragma unroll
+  for (int g = 0; g < kMaps; ++g)
+    any |= g < nm && (!maps.flags[map0 + g] || (*maps.flags[map0 + g] & kFlagHasPolar));
+  if (!any) return;
+  const int pad = ((l + 4) & ~3) + 2;  // l + 1 entries up to a multiple of four, and a spare pair
+  double* al = sm;
+  double* S = sm + pad;  // [parity of m][map][pad]
+  for (int i = threadIdx.x; i < pad; i += blockDim.x) {
+    const int k = l - i;
+    al[i] = k >= 0 ? al_t[tri(l) + i] : 0.0;
+    const double sc = k >= 0 ? sc_t[tri(l) + i] : 0.0;
+    const int64_t at = k >= 0 ? 2 * hp_index(l, k, Nl) : 0;
+#pragma unroll
+    for (int g = 0; g < kMaps; ++g) {
+      const bool ok = k >= 0 && g < nm && (!maps.flags[map0 + g] || (*maps.flags[map0 + g] & kFlagHasPolar));
+      double re = 0.0, im = 0.0;
+      if (ok) {
+        re = maps.rot[map0 + g][at] * (k >= 1 ? 2.0 * sc : sc);
+        im = k >= 1 ? maps.rot[map0 + g][at + 1] * (2.0 * sc) : 0.0;
+      }
+      // l + m + k even goes to the real part: i even for even m
+      S[g * pad + i] = (i & 1) ? im : re;
+      S[(kMaps + g) * pad + i] = (i & 1) ? re : im;
+    }
+  }
+  __syncthreads();
+  // a warp takes every second column: one parity, so that its shared-memory reads are broadcasts
+  const int lane = threadIdx.x & 31, par = (threadIdx.x >> 5) & 1;
+  const double* Sp = S + par * kMaps * pad;
+  for (int first = (threadIdx.x >> 6) * 64 + par; first <= l; first += C * kRotThreads) {
+    const int m0 = first + 2 * lane;
+    const int left = (l - first) / kRotThreads + 1;  // columns of the warp's first lane from here on
+    auto run = [&](auto columns) {
+      constexpr int n = decltype(columns)::value < C ? decltype(columns)::value : C;
+      rotate_columns<kMaps, n>(Nl, l, m0, map0, nm, maps, al, Sp, pad, start, start_e);
+    };
+    switch (min(left, C)) {
+      case 1: run(std::integral_constant<int, 1>{}); break;
+      case 2: run(std::integral_constant<int, 2>{}); break;
+      case 3: run(std::integral_constant<int, 3>{}); break;
+      default: run(std::integral_constant<int, C>{}); break;
+    }
+  }
+}
+
+template <int kMaps, int C>
+void rotate_launch(const Geometry& g, const RotMaps& maps, int nmaps, const RotTables& t, cudaStream_t s) {
+  const size_t smem = sizeof(double) * (size_t)(((g.Nl + 3) & ~3) + 2) * (1 + 2 * kMaps);
+  cudaFuncSetAttribute(rotate_back_kernel<kMaps, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  dim3 grid(g.Nl, (nmaps + kMaps - 1) / kMaps);
+  rotate_back_kernel<kMaps, C><<<grid, kRotThreads, smem, s>>>(g.Nl, nmaps, maps, t.al, t.sc, t.start, t.start_e);
+  count_launches(1);
+}
+
 }  // namespace
 
-void launch_rotate_back(const Geometry& g, const double* alm_rot, const double* alm_add, double* alm_out,
-                        const unsigned* flags, cudaStream_t s) {
-  const size_t smem = (size_t)g.Nl * (6 * sizeof(double) + sizeof(int)) + 64;
-  cudaFuncSetAttribute(rotate_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  rotate_back_kernel<<<g.Nl, kRotThreads, smem, s>>>(g.Nl, alm_rot, alm_add, alm_out, flags);
-  count_launches(1);
+size_t rotation_table_bytes(int Nl) { return (size_t)tri(Nl) * (3 * sizeof(double) + sizeof(int)); }
+
+RotTables rotation_tables(void* base, int Nl) {
+  double* d = static_cast<double*>(base);
+  const size_t n = (size_t)tri(Nl);
+  return RotTables{d, d + n, d + 2 * n, reinterpret_cast<int*>(d + 3 * n)};
 }
 
-template <int kMaps>
-static void rotate_maps_launch(const Geometry& g, const RotMaps& maps, int nmaps, size_t smem, cudaStream_t s) {
-  cudaFuncSetAttribute(rotate_back_maps_kernel<kMaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid(g.Nl, (nmaps + kMaps - 1) / kMaps);
-  rotate_back_maps_kernel<kMaps><<<grid, kRotThreads, smem, s>>>(g.Nl, nmaps, maps);
-  count_launches(1);
+void launch_rotation_tables(const Geometry& g, const RotTables& t, cudaStream_t s) {
+  rotation_table_kernel<<<g.Nl, kTabThreads, 0, s>>>(t.sc, t.start, t.start_e);
+  rotation_alpha_kernel<<<dim3((g.Nl + 255) / 256, g.Nl), 256, 0, s>>>(g.Nl, t.sc, t.al);
+  count_launches(2);
 }
 
-void launch_rotate_back_maps(const Geometry& g, const RotMaps& maps, int nmaps, cudaStream_t s) {
+void launch_rotate_back(const Geometry& g, const RotMaps& maps, int nmaps, const RotTables& t, cudaStream_t s) {
   if (nmaps <= 0) return;
-  // As many maps per CTA (8, 4, 2, 1) as the shared-memory limit allows for this Nl; eight
-  // only while two such CTAs still fit an SM (at Nl=1024 one 8-map CTA per SM took 0.131 ms
-  // per map, two 4-map CTAs per SM 0.107: the recurrence is latency-bound, so residency wins
-  // over sharing it between more maps).
-  auto bytes = [&](int k) { return (size_t)g.Nl * ((5 + 2 * k) * sizeof(double) + sizeof(int)) + 64; };
+  // As many maps per CTA (4, 2, 1) as shared memory holds.  For eight maps at
+  // Nl = 1024 four maps and three columns take 522 us, two columns 541, four columns 765 and eight
+  // maps with two columns 694 (registers: fewer CTAs per SM).
+  auto bytes = [&](int k) { return sizeof(double) * (size_t)(((g.Nl + 3) & ~3) + 2) * (1 + 2 * k); };
   const size_t lim = 227 * 1024;
-  if (nmaps > 4 && 2 * (bytes(8) + 1024) <= 228 * 1024)
-    rotate_maps_launch<8>(g, maps, nmaps, bytes(8), s);
-  else if (nmaps > 2 && bytes(4) <= lim)
-    rotate_maps_launch<4>(g, maps, nmaps, bytes(4), s);
-  else if (nmaps == 2 && bytes(2) <= lim)
-    rotate_maps_launch<2>(g, maps, nmaps, bytes(2), s);
-  else
-    rotate_maps_launch<1>(g, maps, nmaps, bytes(1), s);
+  if (nmaps > 2 && bytes(4) <= lim) rotate_launch<4, 3>(g, maps, nmaps, t, s);
+  else if (nmaps == 2 && bytes(2) <= lim) rotate_launch<2, 2>(g, maps, nmaps, t, s);
+  else rotate_launch<1, 4>(g, maps, nmaps, t, s);
 }
 
 }  // namespace dsht
