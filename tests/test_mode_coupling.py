@@ -64,3 +64,18 @@ def test_gpu_mode_coupling_large_vs_closed_form():
     rows = [0, 1, 57, 200, 399]
     ref = O.mode_coupling_closed_form(Nl, W)
     assert np.abs(M[rows] - ref[rows]).max() <= 1e-11 * np.abs(ref).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Nl,nW", [(1, 1), (1, 0), (2, 3), (17, 5), (31, 61), (64, 200), (129, 257), (300, 40)])
+def test_gpu_mode_coupling_edges(Nl, nW):
+    """Sizes around the thread runs, windows shorter and longer than 2 Nl - 1.  The products of at most
+    2 Nl rounded ratios err by at most 2 Nl 2^-53 of a sum of non-negative terms: below 1e-13."""
+    from directsht_b200.mask import mode_coupling_matrix
+    rng = np.random.default_rng(Nl)
+    W = rng.uniform(0.1, 1.0, nW)
+    full = np.zeros(2 * Nl - 1)
+    full[:min(nW, 2 * Nl - 1)] = W[:2 * Nl - 1]
+    M = mode_coupling_matrix(Nl, W)
+    ref = O.mode_coupling_closed_form(Nl, full)
+    assert np.abs(M - ref).max() <= 1e-12 * max(np.abs(ref).max(), 1e-300)
