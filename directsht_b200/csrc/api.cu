@@ -89,6 +89,7 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
     w.sidx = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * n));
   }
   w.count = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
+  w.flags = base ? w.count + g.nkeys : nullptr;  // cleared with the counts
   w.offset = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
   w.cursor = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
   w.piece_first = reinterpret_cast<int*>(take(sizeof(int) * (g.nkeys + 1)));
@@ -98,7 +99,6 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
   w.piecemax = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * pmax));
   w.wsum = reinterpret_cast<double*>(take(sizeof(double) * pmax));
   w.npieces = reinterpret_cast<int*>(take(sizeof(int)));
-  w.flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
   if (maps) {
     w.slot_flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * kMaxRot));
     w.all_flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));

@@ -20,8 +20,13 @@ namespace dsht {
 namespace {
 
 constexpr int kPointThreads = 256;
-constexpr int kScatterTile = 8192;  // points per block in the scatter pass: 1221 blocks at N = 1e7,
-                                    // several waves of 3 resident blocks per SM
+// Points per block in the scatter pass: 8192 for large N (1221 blocks at N = 1e7, several waves of 3
+// resident blocks per SM, few reservations per point), else such that two blocks per SM have work,
+// down to 512 (N = 1e5 in blocks of 8192 took 33 us, with 13 blocks; now 10).
+int scatter_tile(int64_t N) {
+  const int64_t t = (N + 2 * 148 - 1) / (2 * 148);
+  return t >= 8192 ? 8192 : t <= 512 ? 512 : (int)((t + 255) / 256 * 256);
+}
 
 // The binning of one point: key = set * nbins + bin (DSHT_KEY_DROP when it is in no set)
 // and its flag bits.  x = cos(theta) for equatorial points; a polar point (|cos theta| >=
@@ -262,8 +267,11 @@ scan_kernel(int nkeys, int nbins, int piece_max, int64_t pmax, const uint32_t* _
             int* __restrict__ piece_key, int64_t* piece_start, int* __restrict__ piece_len,
             int* __restrict__ npieces, uint32_t* __restrict__ node_first, int* __restrict__ piece_cta,
             int* __restrict__ cta_first, int nu_grid, int nu_cost) {
+  extern __shared__ uint32_t cnt[];  // [nkeys] the counts, read once
   __shared__ uint32_t warp_tot[3][32];
   __shared__ uint32_t total[3];
+  for (int k = threadIdx.x; k < nkeys; k += kScanThreads) cnt[k] = count[k];
+  __syncthreads();
   const int per = (nkeys + kScanThreads - 1) / kScanThreads;
   const int k0 = min(threadIdx.x * per, (unsigned)nkeys), k1 = min(k0 + per, nkeys);
   // a key's new nodes: its right one, and its left one unless the bin before it has points
@@ -271,9 +279,9 @@ scan_kernel(int nkeys, int nbins, int piece_max, int64_t pmax, const uint32_t* _
     return c == 0 ? 0u : (before != 0 && k % nbins != 0) ? 1u : 2u;
   };
   uint32_t sum = 0, pcs = 0, nds = 0;
-  uint32_t before = k0 > 0 && k0 < nkeys ? count[k0 - 1] : 0u;
+  uint32_t before = k0 > 0 && k0 < nkeys ? cnt[k0 - 1] : 0u;
   for (int k = k0; k < k1; ++k) {
-    const uint32_t c = count[k];
+    const uint32_t c = cnt[k];
     sum += c;
     pcs += (c + piece_max - 1) / piece_max;
     nds += nodes(k, c, before);
@@ -282,9 +290,9 @@ scan_kernel(int nkeys, int nbins, int piece_max, int64_t pmax, const uint32_t* _
   uint32_t o = block_scan_excl(sum, warp_tot[0], &total[0]);
   uint32_t p = block_scan_excl(pcs, warp_tot[1], &total[1]);
   uint32_t nd = nu_grid ? block_scan_excl(nds, warp_tot[2], &total[2]) : 0u;
-  before = k0 > 0 && k0 < nkeys ? count[k0 - 1] : 0u;
+  before = k0 > 0 && k0 < nkeys ? cnt[k0 - 1] : 0u;
   for (int k = k0; k < k1; ++k) {
-    const uint32_t c = count[k];
+    const uint32_t c = cnt[k];
     const uint32_t pc = (c + piece_max - 1) / piece_max;
     offset[k] = o;
     cursor[k] = o;
@@ -360,12 +368,12 @@ __device__ __forceinline__ double2 turns(double a) {
 
 template <typename WT, bool TURN>
 __global__ void __launch_bounds__(kPointThreads)
-scatter_kernel(Geometry g, const double* __restrict__ theta, const double* __restrict__ phi,
+scatter_kernel(Geometry g, int tile, const double* __restrict__ theta, const double* __restrict__ phi,
                const WT* __restrict__ w, int64_t N, const uint32_t* __restrict__ keys, uint32_t* __restrict__ cursor,
                double* __restrict__ pay, uint32_t* __restrict__ sidx) {
   extern __shared__ uint32_t loc[];  // [nkeys] local counts, then local bases
-  const int64_t lo = (int64_t)blockIdx.x * kScatterTile;
-  const int64_t hi = min(lo + (int64_t)kScatterTile, N);
+  const int64_t lo = (int64_t)blockIdx.x * tile;
+  const int64_t hi = min(lo + (int64_t)tile, N);
   for (int k = threadIdx.x; k < g.nkeys; k += blockDim.x) loc[k] = 0;
   __syncthreads();
   constexpr int kUnroll = 4;
@@ -534,8 +542,7 @@ __global__ void publish_flags_kernel(const StatusOut st, int n, unsigned* all) {
 
 void launch_points(const Geometry& g, const double* theta, const double* phi, const void* w, int w_f32,
                    int64_t N, int mode, const Workspace& ws, cudaStream_t s) {
-  cudaMemsetAsync(ws.count, 0, sizeof(uint32_t) * (g.nkeys + 1), s);
-  cudaMemsetAsync(ws.flags, 0, sizeof(unsigned), s);
+  cudaMemsetAsync(ws.count, 0, sizeof(uint32_t) * (g.nkeys + 1), s);  // the flags follow the counts
   const size_t hsmem = sizeof(uint32_t) * g.nkeys;
   const size_t csmem = hsmem + sizeof(uint32_t) * kQueueRounds * kCountUnroll * kPointThreads;
   cudaFuncSetAttribute(count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
@@ -549,16 +556,18 @@ void launch_points(const Geometry& g, const double* theta, const double* phi, co
                                                                 ws.flags, guard);
     count_launches(1);
   }
-  scan_kernel<<<1, kScanThreads, 0, s>>>(g.nkeys, g.nbins, ws.piece_max, ws.pmax, ws.count, ws.offset,
+  cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem);
+  scan_kernel<<<1, kScanThreads, hsmem, s>>>(g.nkeys, g.nbins, ws.piece_max, ws.pmax, ws.count, ws.offset,
                                          ws.cursor, ws.piece_first, ws.piece_key, ws.piece_start,
                                          ws.piece_len, ws.npieces, ws.node_first, ws.piece_cta, ws.cta_first,
                                          ws.nu_grid, ws.nu_piece_cost);
   count_launches(1);
   if (N > 0) {
-    const int64_t blocks = (N + kScatterTile - 1) / kScatterTile;
+    const int tile = scatter_tile(N);
+    const int64_t blocks = (N + tile - 1) / tile;
     auto go = [&](auto kern, const auto* wp) {
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem);
-      kern<<<(unsigned)blocks, kPointThreads, hsmem, s>>>(g, theta, phi, wp, N, ws.key, ws.cursor, ws.pay,
+      kern<<<(unsigned)blocks, kPointThreads, hsmem, s>>>(g, tile, theta, phi, wp, N, ws.key, ws.cursor, ws.pay,
                                                           ws.sidx);
     };
     if (ws.nu_grid) {
