@@ -25,9 +25,9 @@
 namespace dsht {
 namespace {
 
-constexpr int kFoldNodes = 16;  // nodes per fold_digits block (32 m x 16 nodes, 512 threads)
-constexpr int kStageRow = kFoldNodes + 4;  // bytes per staging row (a 4-byte pad: lanes store to
-                                           // rows 20 bytes apart, i.e. 32 different banks)
+constexpr int kFoldNodes = 32;  // fold_digits block: 16 m x 32 nodes, 512 threads
+constexpr int kFoldM = 16;
+constexpr int kStageRow = kFoldNodes + 4;  // bytes per staging row (a 4-byte pad: 36 bytes apart)
 constexpr double kScaleMargin = 1.01;  // scale > 1.01 x bound: |X| < 2^31 / 1.01 < 2^31 - 2^24
 
 // Smallest e with kScaleMargin * v <= 2^e (v >= 0; 0 for v = 0).
@@ -174,24 +174,28 @@ fold_scale_kernel(int nbins, int Nx, const int* __restrict__ piece_first, const 
   if (threadIdx.x < 2 && red[threadIdx.x]) atomicMax(&cmax[threadIdx.x], red[threadIdx.x]);
 }
 
-// Fold of one map straight into digits.  A block covers 32 m x 16 nodes (512 threads, two
-// blocks per SM, so one block's loads overlap the other's stores): warp = node, lane = m
-// while the per-piece sums are read (consecutive m: coalesced), then the digit bytes go
+// Fold of one map straight into digits.  A block covers 16 m x 32 nodes (512 threads, two
+// blocks per SM, so one block's loads overlap the other's stores): half a warp per node, lane = m
+// while the per-piece sums are read (consecutive m: whole sectors), then the digit bytes go
 // through shared memory so that consecutive threads store consecutive nodes.  Staging rows
-// (one per (parity, digit, column, K half, m), 16 node bytes each) are 20 bytes apart with
-// m fastest, so the 32 lanes of a warp store into 32 different banks.
+// (one per (parity, digit, column, K half, m), 32 node bytes each, so every store to memory
+// fills its sectors: 32 m x 16 nodes took 176 us per map at Nl = 1024, Nx = 2048 with tensor-core
+// sums, now 162) are 36 bytes apart with m fastest: lanes store into different banks.  A
+// version whose lanes each took 32 bytes of every row at four nodes, without staging, took 347, one
+// with four nodes per warp and three blocks per SM 257: fewer loads in flight.
 // Sums as fold_kernel forms them (set s: A = V0(bin j) + V2(bin j-1), B = dx (V1(bin j) +
 // V3(bin j-1)), V = vr - i vi; even rows A+ + A-, odd rows A+ - A-), stored as B/dx.
 template <typename Src>
-__global__ void __launch_bounds__(32 * kFoldNodes, 2)
+__global__ void __launch_bounds__(kFoldM * kFoldNodes, 2)
 fold_digits_kernel(int Nl, int Nx, int Kp, const Src src, const unsigned long long* __restrict__ cmax,
                    int16_t* __restrict__ cexp, int map, int ncols, uint8_t* __restrict__ fdig) {
-  // stage[row][kStageRow], row = (((par * 4 + d) * 4 + c) * 2 + kh) * 32 + m, byte j of the
-  // row = node j0 + j (dynamic: 2048 rows)
+  // stage[row][kStageRow], row = (((par * 4 + d) * 4 + c) * 2 + kh) * 16 + m, byte j of the
+  // row = node j0 + j (dynamic: 1024 rows)
   extern __shared__ __align__(16) uint8_t stage[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int m0 = blockIdx.y * 32, j0 = blockIdx.x * kFoldNodes;
-  const int m = m0 + lane, j = j0 + warp;
+  const int m0 = blockIdx.y * kFoldM, j0 = blockIdx.x * kFoldNodes;
+  const int ml0 = lane & (kFoldM - 1), nl = 2 * warp + (lane >> 4);  // half a warp per node
+  const int m = m0 + ml0, j = j0 + nl;
   const int e0 = scale_exp(__longlong_as_double((long long)cmax[0]));
   const int e1 = scale_exp(__longlong_as_double((long long)cmax[1]));
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {  // the column scales of the contraction
@@ -217,22 +221,22 @@ fold_digits_kernel(int Nl, int Nx, int Kp, const Src src, const unsigned long lo
           const int c = 2 * h + ri;
 #pragma unroll
           for (int d = 0; d < 4; ++d)
-            stage[(((((par * 4 + d) * 4 + c) * 2 + kh) * 32) + lane) * kStageRow + warp] =
+            stage[(((((par * 4 + d) * 4 + c) * 2 + kh) * kFoldM) + ml0) * kStageRow + nl] =
                 (uint8_t)(w >> (8 * (3 - d)));
         }
   }
   __syncthreads();
-  // 2048 rows x kFoldNodes/4 words; word w covers 4 nodes of one (par, d, c, kh, m) row.
+  // 1024 rows x kFoldNodes/4 words; word w covers 4 nodes of one (par, d, c, kh, m) row.
   constexpr int kWords = kFoldNodes / 4;
   const int nj = min(kFoldNodes, Nx - j0);
-  for (int w = threadIdx.x; w < 32 * 2 * 4 * 4 * 2 * kWords; w += blockDim.x) {
+  for (int w = threadIdx.x; w < kFoldM * 2 * 4 * 4 * 2 * kWords; w += blockDim.x) {
     const int q = w % kWords;      // 4-node group
-    const int row = w / kWords;    // (((par * 4 + d) * 4 + c) * 2 + kh) * 32 + ml
-    const int ml = row & 31;
-    const int kh = (row >> 5) & 1;
-    const int c = (row >> 6) & 3;
-    const int d = (row >> 8) & 3;
-    const int par = (row >> 10) & 1;
+    const int row = w / kWords;    // (((par * 4 + d) * 4 + c) * 2 + kh) * 16 + ml
+    const int ml = row & 15;
+    const int kh = (row >> 4) & 1;
+    const int c = (row >> 5) & 3;
+    const int d = (row >> 7) & 3;
+    const int par = (row >> 9) & 1;
     const int mm = m0 + ml;
     if (mm >= Nl || 4 * q >= nj) continue;
     const uint32_t word = *reinterpret_cast<const uint32_t*>(stage + row * kStageRow + 4 * q);
@@ -292,12 +296,12 @@ void launch_fold_scale(const Geometry& g, const Workspace& ws, unsigned long lon
 void launch_fold_digits(const Geometry& g, const Workspace& ws, const unsigned long long* cmax, int16_t* cexp,
                         int map, int ncols, uint8_t* fdig, cudaStream_t s) {
   const int Kp = digit_kp(g.Nx);
-  dim3 grid((g.Nx + kFoldNodes - 1) / kFoldNodes, (g.Nl + 31) / 32);
-  constexpr int kStageBytes = 32 * 2 * 4 * 4 * 2 * kStageRow;
+  dim3 grid((g.Nx + kFoldNodes - 1) / kFoldNodes, (g.Nl + kFoldM - 1) / kFoldM);
+  constexpr int kStageBytes = kFoldM * 2 * 4 * 4 * 2 * kStageRow;
   with_node_source(g, ws, [&](auto src) {
     auto kern = fold_digits_kernel<decltype(src)>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
-    kern<<<grid, 32 * kFoldNodes, kStageBytes, s>>>(g.Nl, g.Nx, Kp, src, cmax, cexp, map, ncols, fdig);
+    kern<<<grid, kFoldM * kFoldNodes, kStageBytes, s>>>(g.Nl, g.Nx, Kp, src, cmax, cexp, map, ncols, fdig);
   });
   count_launches(1);
 }
