@@ -17,6 +17,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
+from .hostcopy import to_host
 
 
 def mode_coupling_matrix(Nl: int, W_l, device=None) -> np.ndarray:
@@ -29,7 +30,7 @@ def mode_coupling_matrix(Nl: int, W_l, device=None) -> np.ndarray:
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
         L.check(lib.dsht_mode_coupling(int(Nl), L.ptr(W), int(W.numel()), L.ptr(M), ct.c_void_p(stream)))
-    return M.cpu().numpy()
+        return to_host(M)
 
 
 class MaskDeconvolution:

@@ -16,13 +16,14 @@ import numpy as np
 import torch
 
 from . import _lib as L
+from .hostcopy import to_device, to_host
 
 
 def _as_device_f64(a, device) -> torch.Tensor:
     if isinstance(a, torch.Tensor):
         return a.to(device=device, dtype=torch.float64).contiguous()
     arr = np.ascontiguousarray(np.asarray(a, dtype=np.float64))
-    return torch.from_numpy(arr).to(device=device, non_blocking=False)
+    return to_device(arr, device)
 
 
 class DirectSHT:
@@ -221,7 +222,7 @@ class DirectSHT:
             stream = torch.cuda.current_stream(self.device).cuda_stream
             rc = self._lib.dsht_execute(self._plan, L.ptr(td), L.ptr(pd), L.ptr(wd), n, mode, L.ptr(alm),
                                         L.ptr(ws), ws.numel(), ct.c_void_p(stream))
-        return rc, (alm if on_device else alm.cpu().numpy())
+            return rc, (alm if on_device else to_host(alm))
 
     def __call__(self, t, p, w):
         """alm of weighted points at (theta, phi) (``sht/sht.py:112-150``).
@@ -260,7 +261,12 @@ class DirectSHT:
         if isinstance(wts, torch.Tensor):
             wd = wts.to(device=self.device)
         else:
-            wd = torch.from_numpy(np.ascontiguousarray(np.asarray(wts)))
+            wd = np.ascontiguousarray(np.asarray(wts))
+            if wd.dtype in (np.float32, np.float64):
+                with torch.cuda.device(self.device):
+                    wd = to_device(wd, self.device)
+            else:
+                wd = torch.from_numpy(wd)
         if wd.dim() == 1:
             wd = wd[None, :]
         if wd.dtype not in (torch.float32, torch.float64):
@@ -291,7 +297,10 @@ class DirectSHT:
             raise ValueError("The theta array seems to be empty!")
         else:
             L.check(rc)
-        return alm if on_device else alm.cpu().numpy()
+        if on_device:
+            return alm
+        with torch.cuda.device(self.device):
+            return to_host(alm)
 
     def call_batch(self, point_sets, mode="call"):
         """alm of several independent point sets, each ``(theta, phi, w)``: item i is
@@ -338,7 +347,10 @@ class DirectSHT:
                 raise AssertionError("theta must be in [ACos[xmax],ACos[-xmax]).")
             else:
                 L.check(rc)
-        return alms if on_device else [a.cpu().numpy() for a in alms]
+        if on_device:
+            return alms
+        with torch.cuda.device(self.device):
+            return [to_host(a) for a in alms]
 
     def basic_sht(self, theta, phi, wt, reg_factor=1.0, verbose=True):
         """alm of points with |cos theta| < xmax, no rotation (``sht/sht.py:153-283``).

@@ -1,0 +1,52 @@
+"""Host <-> device copies through pinned chunks: sizes around the direct-copy limit and the chunk
+boundaries come back byte for byte, from several threads and streams at once."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _sizes():
+    from directsht_b200 import hostcopy as H
+    c, m = H._CHUNK // 8, H._MIN_BYTES // 8
+    return [0, 1, m - 1, m, m + 1, c - 1, c, c + 1, 3 * c, 3 * c + 5, 7 * c - 3]
+
+
+def test_round_trip():
+    from directsht_b200.hostcopy import to_device, to_host
+    rng = np.random.default_rng(0)
+    for n in _sizes():
+        a = rng.normal(size=n)
+        keep = a.copy()
+        d = to_device(a, "cuda")
+        a[:] = 0.0  # the source may change at once
+        np.testing.assert_array_equal(to_host(d), keep)
+    for a in (rng.normal(size=(3, 250001)).astype(np.float32), rng.normal(size=400001) + 1j * rng.normal(size=400001)):
+        d = to_device(a, "cuda")
+        assert tuple(d.shape) == a.shape
+        np.testing.assert_array_equal(to_host(d), a)
+    d = to_device(rng.normal(size=(1000, 600)), "cuda")
+    np.testing.assert_array_equal(to_host(d.t()), d.t().cpu().numpy())  # not contiguous
+
+
+def test_threads_and_streams():
+    import torch
+    from directsht_b200.hostcopy import to_device, to_host
+    bad = []
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(5):
+                a = rng.normal(size=900000)
+                if not np.array_equal(to_host(to_device(a, "cuda") * 2.0), a * 2.0):
+                    bad.append(seed)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
