@@ -14,18 +14,22 @@
 // writes it to its sorted slot; the bin-sum kernels form w h_k(t) themselves (the NUFFT sums
 // take the azimuth in turns instead of its cosine and sine).  HBM bytes per point: 16 read + 4 written
 // (count), 28 read + 32 written (scatter), against the algorithmic 24 read + 32 written.
+#include <algorithm>
+
 #include "dsht_internal.cuh"
 
 namespace dsht {
 namespace {
 
 constexpr int kPointThreads = 256;
-// Points per block in the scatter pass: 8192 for large N (1221 blocks at N = 1e7, several waves of 3
-// resident blocks per SM, few reservations per point), else such that two blocks per SM have work,
-// down to 512 (N = 1e5 in blocks of 8192 took 33 us, with 13 blocks; now 10).
-int scatter_tile(int64_t N) {
-  const int64_t t = (N + 2 * 148 - 1) / (2 * 148);
-  return t >= 8192 ? 8192 : t <= 512 ? 512 : (int)((t + 255) / 256 * 256);
+// Points per block in the scatter pass: at most 4096, in whole waves of the blocks that fit the chip
+// (resident per SM; a last wave of a few blocks costs a whole one: N = 2e6 took 140 us of points stage
+// in 489 blocks, 123 in 444), at least 512.  Larger tiles reserve less often but wrote 10 % slower
+// (N = 1e7: 340 us of points stage at 8192, 310 at 3840), smaller ones pay for the reservations.
+int scatter_tile(int64_t N, int resident) {
+  const int64_t wave = 148 * (int64_t)resident, waves = (N + wave * 4096 - 1) / (wave * 4096);
+  const int64_t t = (N + wave * waves - 1) / (wave * waves);
+  return t <= 512 ? 512 : (int)((t + 63) / 64 * 64);
 }
 
 // The binning of one point: key = set * nbins + bin (DSHT_KEY_DROP when it is in no set)
@@ -157,7 +161,8 @@ __device__ __forceinline__ bool screen_key(const Geometry& g, float inv_dx_f, fl
 // shared memory and decided by the FP64 path a few rounds later by whole warps, so the FP64
 // sines and cosines run for those points only.
 constexpr int kCountUnroll = 4;
-constexpr int kQueueRounds = 2;  // rounds of kCountUnroll * blockDim points between queue flushes
+constexpr int kQueueRounds = 4;  // rounds of kCountUnroll * blockDim points between queue flushes
+                                 // (2: 3 us more at N = 1e7, in the barriers)
 
 __global__ void __launch_bounds__(kPointThreads)
 count_kernel(Geometry g, int mode, const double* __restrict__ theta, const double* __restrict__ phi,
@@ -229,111 +234,128 @@ count_kernel(Geometry g, int mode, const double* __restrict__ theta, const doubl
     if (hist[k]) atomicAdd(&count[k], hist[k]);
 }
 
-// Single-block exclusive scans: key offsets, pieces per key, and the piece list.  Every thread
-// takes a run of consecutive keys, so one pass of block scans serves any number of keys.  For the
-// NUFFT sums also the nodes with points before each key, the CTA of every piece (equal shares
-// of points + cost x pieces) and the first piece of every CTA.
+// Single-block exclusive scans: key offsets, pieces per key, and the piece list.  Every warp takes a
+// run of consecutive keys, 32 at a time, so that the lists are written in whole sectors (a run per
+// thread wrote seven lists at strides of nkeys/1024 entries: 43 us at nkeys = 8188, bound by those
+// sectors; now 22 us).  For the NUFFT sums also the nodes with points before each key, the CTA of every
+// piece (equal shares of points + cost x pieces) and the first piece of every CTA.
 constexpr int kScanThreads = 1024;
 
-// Exclusive scan of one value per thread; *total receives the sum.
-__device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* warp_tot, uint32_t* total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t x = v;
+// Inclusive warp scans of three values together (their shuffles overlap).
+struct Scan3 {
+  uint32_t pts, pcs, nds;
+};
+__device__ __forceinline__ Scan3 warp_scan(Scan3 v) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warp_tot[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    uint32_t t = (lane < (int)(blockDim.x >> 5)) ? warp_tot[lane] : 0u;
-    uint32_t s = t;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += y;
+    const uint32_t a = __shfl_up_sync(0xffffffffu, v.pts, o);
+    const uint32_t b = __shfl_up_sync(0xffffffffu, v.pcs, o);
+    const uint32_t c = __shfl_up_sync(0xffffffffu, v.nds, o);
+    if (lane >= o) {
+      v.pts += a;
+      v.pcs += b;
+      v.nds += c;
     }
-    warp_tot[lane] = s - t;
-    if (lane == 31) *total = s;
   }
-  __syncthreads();
-  return x - v + warp_tot[wid];
+  return v;
+}
+__device__ __forceinline__ Scan3 from_lane(const Scan3& v, int lane) {
+  Scan3 r;
+  r.pts = __shfl_sync(0xffffffffu, v.pts, lane);
+  r.pcs = __shfl_sync(0xffffffffu, v.pcs, lane);
+  r.nds = __shfl_sync(0xffffffffu, v.nds, lane);
+  return r;
 }
 
 __global__ void __launch_bounds__(kScanThreads)
 scan_kernel(int nkeys, int nbins, int piece_max, int64_t pmax, const uint32_t* __restrict__ count,
             uint32_t* __restrict__ offset, uint32_t* __restrict__ cursor, int* __restrict__ piece_first,
-            int* __restrict__ piece_key, int64_t* piece_start, int* __restrict__ piece_len,
-            int* __restrict__ npieces, uint32_t* __restrict__ node_first, int* __restrict__ piece_cta,
+            int* __restrict__ piece_key, int64_t* __restrict__ piece_start, int* __restrict__ piece_len,
+            int* __restrict__ npieces, uint32_t* __restrict__ node_first, int* piece_cta,
             int* __restrict__ cta_first, int nu_grid, int nu_cost) {
   extern __shared__ uint32_t cnt[];  // [nkeys] the counts, read once
-  __shared__ uint32_t warp_tot[3][32];
-  __shared__ uint32_t total[3];
+  __shared__ Scan3 wtot[32];
   for (int k = threadIdx.x; k < nkeys; k += kScanThreads) cnt[k] = count[k];
   __syncthreads();
-  const int per = (nkeys + kScanThreads - 1) / kScanThreads;
-  const int k0 = min(threadIdx.x * per, (unsigned)nkeys), k1 = min(k0 + per, nkeys);
-  // a key's new nodes: its right one, and its left one unless the bin before it has points
-  auto nodes = [&](int k, uint32_t c, uint32_t before) -> uint32_t {
-    return c == 0 ? 0u : (before != 0 && k % nbins != 0) ? 1u : 2u;
-  };
-  uint32_t sum = 0, pcs = 0, nds = 0;
-  uint32_t before = k0 > 0 && k0 < nkeys ? cnt[k0 - 1] : 0u;
-  for (int k = k0; k < k1; ++k) {
-    const uint32_t c = cnt[k];
-    sum += c;
-    pcs += (c + piece_max - 1) / piece_max;
-    nds += nodes(k, c, before);
-    before = c;
-  }
-  uint32_t o = block_scan_excl(sum, warp_tot[0], &total[0]);
-  uint32_t p = block_scan_excl(pcs, warp_tot[1], &total[1]);
-  uint32_t nd = nu_grid ? block_scan_excl(nds, warp_tot[2], &total[2]) : 0u;
-  before = k0 > 0 && k0 < nkeys ? cnt[k0 - 1] : 0u;
-  for (int k = k0; k < k1; ++k) {
-    const uint32_t c = cnt[k];
-    const uint32_t pc = (c + piece_max - 1) / piece_max;
-    offset[k] = o;
-    cursor[k] = o;
-    piece_first[k] = (int)p;
-    if (nu_grid) {
-      node_first[k] = nd;
-      nd += nodes(k, c, before);
-    }
-    before = c;
-    for (uint32_t q = 0; q < pc; ++q) {
-      const int64_t pi = (int64_t)p + q;
-      if (pi < pmax) {
-        piece_key[pi] = k;
-        piece_start[pi] = (int64_t)o + (int64_t)q * piece_max;
-        const uint32_t rem = c - q * piece_max;
-        piece_len[pi] = (int)(rem < (uint32_t)piece_max ? rem : (uint32_t)piece_max);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int run = (nkeys + kScanThreads - 1) / kScanThreads * 32;  // keys per warp
+  const int k0 = min(wid * run, nkeys), k1 = min(k0 + run, nkeys);
+  // one key: its points, its pieces, and its new nodes -- its right one, and its left one unless
+  // the bin before it has points
+  auto key_counts = [&](int k) {
+    Scan3 v{0u, 0u, 0u};
+    if (k < k1) {
+      v.pts = cnt[k];
+      const bool first = k == 0 || k == nbins || k == 2 * nbins || k == 3 * nbins;  // of its set
+      if (v.pts) {
+        v.pcs = v.pts <= (uint32_t)piece_max ? 1u : (v.pts + piece_max - 1) / piece_max;
+        v.nds = (!first && cnt[k - 1] != 0) ? 1u : 2u;
       }
     }
-    o += c;
-    p += pc;
+    return v;
+  };
+  Scan3 sum{0u, 0u, 0u};
+  for (int k = k0 + lane; k < k1; k += 32) {
+    const Scan3 v = key_counts(k);
+    sum.pts += v.pts;
+    sum.pcs += v.pcs;
+    sum.nds += v.nds;
   }
-  const int np = (int)min((int64_t)total[1], pmax);
+  sum = from_lane(warp_scan(sum), 31);
+  if (lane == 0) wtot[wid] = sum;
+  __syncthreads();
+  const Scan3 mine = wtot[lane];
+  const Scan3 incl = warp_scan(mine);
+  const Scan3 total = from_lane(incl, 31);
+  Scan3 at = from_lane(incl, wid);  // what lies before this warp's keys
+  at.pts -= sum.pts;
+  at.pcs -= sum.pcs;
+  at.nds -= sum.nds;
+  const int np = (int)min((int64_t)total.pcs, pmax);
+  // piece i starts at position start + cost i of total.pts + cost np
+  const double scale = (double)nu_grid / ((double)total.pts + (double)nu_cost * np + 1.0);
+  for (int kb = k0; kb < k1; kb += 32) {
+    const int k = kb + lane;
+    const Scan3 v = key_counts(k);
+    const Scan3 s = warp_scan(v);
+    const uint32_t o = at.pts + s.pts - v.pts, p = at.pcs + s.pcs - v.pcs;
+    if (k < k1) {
+      offset[k] = o;
+      cursor[k] = o;
+      piece_first[k] = (int)p;
+      if (nu_grid) node_first[k] = at.nds + s.nds - v.nds;
+    }
+    for (uint32_t q = 0; q < v.pcs; ++q) {
+      const int64_t pi = (int64_t)p + q;
+      if (pi < pmax) {
+        const int64_t start = (int64_t)o + (int64_t)q * piece_max;
+        const uint32_t rem = v.pts - q * piece_max;
+        piece_key[pi] = k;
+        piece_start[pi] = start;
+        piece_len[pi] = (int)(rem < (uint32_t)piece_max ? rem : (uint32_t)piece_max);
+        if (nu_grid)
+          piece_cta[pi] = min(nu_grid - 1, (int)(((double)start + (double)nu_cost * (int)pi) * scale));
+      }
+    }
+    const Scan3 last = from_lane(s, 31);
+    at.pts += last.pts;
+    at.pcs += last.pcs;
+    at.nds += last.nds;
+  }
   if (threadIdx.x == 0) {
-    offset[nkeys] = total[0];
-    piece_first[nkeys] = (int)total[1];
-    *npieces = (int)total[1];
-    if (nu_grid) node_first[nkeys] = total[2];
+    offset[nkeys] = total.pts;
+    piece_first[nkeys] = (int)total.pcs;
+    *npieces = (int)total.pcs;
+    if (nu_grid) node_first[nkeys] = total.nds;
   }
   if (!nu_grid) return;
-  // piece i starts at position piece_start[i] + cost i of total[0] + cost np
-  const double scale = (double)nu_grid / ((double)total[0] + (double)nu_cost * np + 1.0);
-  auto cta = [&](int i) {
-    return min(nu_grid - 1, (int)(((double)piece_start[i] + (double)nu_cost * i) * scale));
-  };
   __syncthreads();  // the piece list is complete
   for (int i = threadIdx.x; i < np; i += kScanThreads) {
-    const int c = cta(i);
-    piece_cta[i] = c;
-    for (int b = (i ? cta(i - 1) : -1) + 1; b <= c; ++b) cta_first[b] = i;
+    const int c = piece_cta[i];
+    for (int b = (i ? piece_cta[i - 1] : -1) + 1; b <= c; ++b) cta_first[b] = i;
   }
-  for (int b = (np ? cta(np - 1) : -1) + 1 + (int)threadIdx.x; b <= nu_grid; b += kScanThreads) cta_first[b] = np;
+  for (int b = (np ? piece_cta[np - 1] : -1) + 1 + (int)threadIdx.x; b <= nu_grid; b += kScanThreads) cta_first[b] = np;
 }
 
 // Largest |w h_k| of a point as float bits (non-negative floats order like their bits).
@@ -366,27 +388,38 @@ __device__ __forceinline__ double2 turns(double a) {
   return make_double2(hi, e + err);
 }
 
+// Rotated polar points take two sines and cosines and an arc tangent more than the others.  With
+// points in any order nearly every warp holds some, so each warp queues its polar points and does
+// them 32 at a time.  (N = 1e7, a third of them polar, Nx = 2048: 286 us with the polar arithmetic in
+// line, 217 queued and in tiles of 4096; the traffic is 640 MB or 99 us, and the rest is instructions
+// -- 57 % of the issue slots -- and the latency of a round's loads.)
+constexpr int kScatUnroll = 4;
+constexpr int kScatQueue = 31 + 32 * kScatUnroll;  // entries per warp: a partial batch and one round
+
 template <typename WT, bool TURN>
 __global__ void __launch_bounds__(kPointThreads)
 scatter_kernel(Geometry g, int tile, const double* __restrict__ theta, const double* __restrict__ phi,
                const WT* __restrict__ w, int64_t N, const uint32_t* __restrict__ keys, uint32_t* __restrict__ cursor,
                double* __restrict__ pay, uint32_t* __restrict__ sidx) {
-  extern __shared__ uint32_t loc[];  // [nkeys] local counts, then local bases
+  extern __shared__ uint32_t loc[];  // [nkeys] local counts, then local bases; then the queues
+  const int lane = threadIdx.x & 31;
+  uint32_t* q_at = loc + g.nkeys + (threadIdx.x >> 5) * (3 * kScatQueue);  // point, relative to lo
+  uint32_t* q_pos = q_at + kScatQueue;                                     // its slot
+  uint32_t* q_key = q_pos + kScatQueue;
   const int64_t lo = (int64_t)blockIdx.x * tile;
   const int64_t hi = min(lo + (int64_t)tile, N);
   for (int k = threadIdx.x; k < g.nkeys; k += blockDim.x) loc[k] = 0;
   __syncthreads();
-  constexpr int kUnroll = 4;
-  const int64_t step = (int64_t)kUnroll * blockDim.x;
+  const int64_t step = (int64_t)kScatUnroll * blockDim.x;
   for (int64_t b = lo + threadIdx.x; b < hi; b += step) {
-    uint32_t k[kUnroll];
+    uint32_t k[kScatUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kScatUnroll; ++u) {
       const int64_t i = b + (int64_t)u * blockDim.x;
       k[u] = (i < hi) ? keys[i] : DSHT_KEY_DROP;
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u)
+    for (int u = 0; u < kScatUnroll; ++u)
       if (k[u] != DSHT_KEY_DROP) atomicAdd(&loc[k[u]], 1u);
   }
   __syncthreads();
@@ -407,11 +440,42 @@ scatter_kernel(Geometry g, int tile, const double* __restrict__ theta, const dou
   }
   __syncthreads();
   const int polar_key0 = 2 * g.nbins;
-  for (int64_t b = lo + threadIdx.x; b < hi; b += step) {
-    uint32_t k[kUnroll], pos[kUnroll];
-    double th[kUnroll], ph[kUnroll], wi[kUnroll];
+  // t = (|x| - x_j) / dx in the reference's rounding (sht/sht.py:221); one 32-byte sector
+  auto put = [&](int64_t i, uint32_t pos, int kk, double a, double b, double wi, double x) {
+    const int j = kk - g.nbins * ((kk >= g.nbins) + (kk >= 2 * g.nbins) + (kk >= 3 * g.nbins));  // key % nbins
+    const double t = __ddiv_rn(__dadd_rn(fabs(x), -(double)j * g.dx), g.dx);
+    double2* out = reinterpret_cast<double2*>(pay + (size_t)kRec * pos);
+    out[0] = make_double2(a, b);
+    out[1] = make_double2(wi, t);
+    if (sidx) sidx[pos] = (uint32_t)i;
+  };
+  auto polar = [&](int e) {  // queue entry e
+    const int64_t i = lo + q_at[e];
+    double st, c, sp, cp;
+    sincos(theta[i], &st, &c);
+    sincos(phi[i], &sp, &cp);
+    const double x = -__dmul_rn(st, cp), ny = st * sp;
+    double a = 1.0, b = 0.0;
+    if constexpr (TURN) {
+      const double2 tr = turns(atan2(ny, c));  // azimuth of the rotated point (c, s sin p, -s cos p)
+      a = tr.x;
+      b = tr.y;
+    } else {
+      const double rho = sqrt(ny * ny + c * c);
+      if (rho > 0.0) {
+        const double ir = 1.0 / rho;
+        a = c * ir;
+        b = ny * ir;
+      }
+    }
+    put(i, q_pos[e], (int)q_key[e], a, b, (double)w[i], x);
+  };
+  int qn = 0;
+  for (int64_t b = lo + threadIdx.x; b - lane < hi; b += step) {
+    uint32_t k[kScatUnroll], pos[kScatUnroll];
+    double th[kScatUnroll], ph[kScatUnroll], wi[kScatUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kScatUnroll; ++u) {
       const int64_t i = b + (int64_t)u * blockDim.x;
       k[u] = DSHT_KEY_DROP;
       if (i < hi) {
@@ -423,51 +487,34 @@ scatter_kernel(Geometry g, int tile, const double* __restrict__ theta, const dou
     }
     // the slots first: their shared-memory round trips overlap the record arithmetic
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u)
+    for (int u = 0; u < kScatUnroll; ++u)
       if (k[u] != DSHT_KEY_DROP) pos[u] = atomicAdd(&loc[k[u]], 1u);
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      if (k[u] == DSHT_KEY_DROP) continue;
-      double st, c, sp, cp;
-      sincos(th[u], &st, &c);
-      double cphi, sphi, x = c;
-      if constexpr (TURN) {
-        double az = ph[u];
-        if ((int)k[u] >= polar_key0) {
-          sincos(ph[u], &sp, &cp);
-          x = -__dmul_rn(st, cp);
-          az = atan2(st * sp, c);  // azimuth of the rotated point (c, s sin p, -s cos p)
-        }
-        const double2 tr = turns(az);
-        cphi = tr.x;
-        sphi = tr.y;
-      } else {
-        sincos(ph[u], &sp, &cp);
-        cphi = cp;
-        sphi = sp;
-        if ((int)k[u] >= polar_key0) {
-          x = -__dmul_rn(st, cp);
-          const double ny = st * sp;
-          const double rho = sqrt(ny * ny + c * c);
-          cphi = 1.0;
-          sphi = 0.0;
-          if (rho > 0.0) {
-            const double ir = 1.0 / rho;
-            cphi = c * ir;
-            sphi = ny * ir;
-          }
-        }
+    for (int u = 0; u < kScatUnroll; ++u) {
+      const int64_t i = b + (int64_t)u * blockDim.x;
+      const bool live = k[u] != DSHT_KEY_DROP, pol = live && (int)k[u] >= polar_key0;
+      const unsigned m = __ballot_sync(0xffffffffu, pol);
+      if (pol) {
+        const int e = qn + __popc(m & ((1u << lane) - 1u));
+        q_at[e] = (uint32_t)(i - lo);
+        q_pos[e] = pos[u];
+        q_key[e] = k[u];
       }
-      const int kk = (int)k[u];  // bin j = key - set nbins, without an integer division
-      const int j = kk - g.nbins * ((kk >= g.nbins) + (kk >= 2 * g.nbins) + (kk >= 3 * g.nbins));
-      // t = (|x| - x_j) / dx in the reference's rounding (sht/sht.py:221)
-      const double t = __ddiv_rn(__dadd_rn(fabs(x), -(double)j * g.dx), g.dx);
-      double2* out = reinterpret_cast<double2*>(pay + (size_t)kRec * pos[u]);  // one 32-byte sector
-      out[0] = make_double2(cphi, sphi);
-      out[1] = make_double2(wi[u], t);
-      if (sidx) sidx[pos[u]] = (uint32_t)(b + (int64_t)u * blockDim.x);
+      qn += __popc(m);
+      if (live && !pol) {
+        double st, c;
+        sincos(th[u], &st, &c);
+        double2 az;
+        if constexpr (TURN) az = turns(ph[u]);
+        else sincos(ph[u], &az.y, &az.x);
+        put(i, pos[u], (int)k[u], az.x, az.y, wi[u], c);
+      }
     }
+    __syncwarp();
+    for (; qn >= 32; qn -= 32) polar(qn - 32 + lane);
+    __syncwarp();
   }
+  if (lane < qn) polar(lane);
 }
 
 // Another weight map on the same sorted points (multi-map transforms share the sort): the
@@ -563,11 +610,13 @@ void launch_points(const Geometry& g, const double* theta, const double* phi, co
                                          ws.nu_grid, ws.nu_piece_cost);
   count_launches(1);
   if (N > 0) {
-    const int tile = scatter_tile(N);
+    const size_t ssmem = hsmem + sizeof(uint32_t) * 3 * kScatQueue * (kPointThreads / 32);
+    const int resident = (int)std::min<size_t>(3, (size_t)(227 * 1024) / (ssmem + 1024));  // 3 by registers
+    const int tile = scatter_tile(N, std::max(1, resident));
     const int64_t blocks = (N + tile - 1) / tile;
     auto go = [&](auto kern, const auto* wp) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem);
-      kern<<<(unsigned)blocks, kPointThreads, hsmem, s>>>(g, tile, theta, phi, wp, N, ws.key, ws.cursor, ws.pay,
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem);
+      kern<<<(unsigned)blocks, kPointThreads, ssmem, s>>>(g, tile, theta, phi, wp, N, ws.key, ws.cursor, ws.pay,
                                                           ws.sidx);
     };
     if (ws.nu_grid) {
