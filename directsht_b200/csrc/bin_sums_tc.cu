@@ -33,11 +33,19 @@
 // into one of two anchor buffers, one block ahead, two threads per point (warps 6-7 the
 // heavier half, on the sub-partitions without a B slicer warp); warps 0-5
 // quantise and slice them into a ring of 64-byte-swizzled K-major int8 tiles (warps 0-1
-// the B tiles, 2-5 the A tiles); warp 10 issues the MMAs from one thread; warps 0-3 run
-// each piece's epilogue (TMEM lanes 0-127) while warps 4-5 and the anchor warps start the
-// next piece.  Hand-overs are mbarriers (afull/aempty: anchors <-> slicers, full/empty:
+// the B tiles, 2-5 the A tiles); warp 10 issues the MMAs from one thread; warps 11-14 run
+// each piece's epilogue (one TMEM lane quarter each) while the others start the next
+// piece.  Hand-overs are mbarriers (afull/aempty: anchors <-> slicers, full/empty:
 // slicers <-> MMA via tcgen05.commit, done: MMA -> epilogue, tfree: epilogue -> MMA).
 // Every wait is bounded.
+//
+// What bounds it: the accumulators fill TMEM at CH = 64, so a piece's MMAs wait for the epilogue
+// of the piece before.  In the slicer warps that cost 30 % of the kernel (Nl = 1024, Nx = 2048,
+// N = 2e6: 1240 us a map with gather and piece maxima, 870 without any epilogue); warps of its own,
+// the sign of Vr folded into the exchanged value and one 32-byte store per lane and step made it
+// 1117.  The rest is shared evenly by anchors and slicers, one warp per sub-partition each: without
+// either 160 us less, without both 420.  More slicer or epilogue warps cost more in registers (80 to
+// 96 a thread spill: 1290-1430 us) than they hide, and so do uneven halves of the anchors (1153).
 //
 // FP64 is the limiting pipe: while int8 MMAs run, an SM sub-partition issues about one
 // FP64 warp instruction in 16 clocks (one in 2 on an SM that has not used its tensor
@@ -50,11 +58,14 @@ namespace dsht {
 namespace {
 
 constexpr int kBK = 64;                 // points per stage: one 64-byte row of int8
-constexpr int kSlicerWarps = 6;         // warps 0-5: int8 slice tiles (0-3: epilogue too)
+constexpr int kSlicerWarps = 6;         // warps 0-5: int8 slice tiles
 constexpr int kAnchorWarps = 4;         // warps 6-9: FP64 anchors, one block ahead
 constexpr int kBThreads = 64;           // slicer threads 0-63: B tiles, 64-191: A tiles
 constexpr int kSlicers = 32 * kSlicerWarps;
-constexpr int kThreads = 32 * (kSlicerWarps + kAnchorWarps + 1);  // + warp 10: MMA issuer
+constexpr int kMmaWarp = kSlicerWarps + kAnchorWarps;  // warp 10: MMA issuer
+constexpr int kEpiWarps = 4;            // warps 11-: epilogue (4 per set of TMEM lanes 0-127)
+constexpr int kEpiSets = kEpiWarps / 4;
+constexpr int kThreads = 32 * (kMmaWarp + 1 + kEpiWarps);
 constexpr int kM = 128;
 constexpr float kQf = 4193280.0f;       // 2^22 - 2^10: |X| < 2^22, so X >> 16 fits int8
 constexpr double kQ = 4193280.0;
@@ -197,7 +208,7 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
       tc::mbar_init(&afull[b], kAnchorWarps);
       tc::mbar_init(&aempty[b], kSlicerWarps);
     }
-    tc::mbar_init(tfree, 4);
+    tc::mbar_init(tfree, kEpiWarps);
     *abort_flag = 0;
     tc::mbar_fence_init();
   }
@@ -328,9 +339,9 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
       }
     }
   } else if (warp < kSlicerWarps) {
-    // ==== slicer warps: int8 slice tiles; warps 0-3 also run the epilogue ==============
-    uint32_t g = 0, piece_iter = 0;
-    for (int piece = blockIdx.x; piece < npieces; piece += gridDim.x, ++piece_iter) {
+    // ==== slicer warps: int8 slice tiles ================================================
+    uint32_t g = 0;
+    for (int piece = blockIdx.x; piece < npieces; piece += gridDim.x) {
       const int len = piece_len[piece];
       const int nblk = (len + kBK - 1) / kBK;
       for (int b = 0; b < nblk; ++b, ++g) {
@@ -401,72 +412,8 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
           tc::mbar_arrive(&aempty[buf]);
         }
       }
-
-      // ---- epilogue: warps 0-3 own TMEM lanes 0-127 -----------------------------------
-      // Lane r holds row r = 2 (16 k + a) + ri of D.  For every c:
-      //   Vr = D[re, Rr] - D[im, Ri],  Vi = D[re, Ri] + D[im, Rr],
-      // so each lane sends its D[., Ri] to its neighbour (lane r ^ 1) and keeps D[., Rr]:
-      // the re lane writes Vr, the im lane Vi, for m = Cf a + cbase + c.  Warps 4-7 go on
-      // with the next piece meanwhile.
-      if (warp < 4) {
-        bool ok = !*abort_flag;
-        if (ok && !tc::mbar_wait(done, piece_iter & 1, abort_flag)) {
-          fail();
-          ok = false;
-        }
-        tc::tc_fence_after();
-        const int r = tid;  // TMEM lane == GEMM row
-        const int ri = r & 1, j = r >> 1;
-        const int k = j >> 4, a = j & 15;
-        const double f = tc_scale(piecemax[piece]) * kKScale[k] / (kQ * kQ);
-        const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
-        float* out = partial + ((size_t)piece * 8 + 2 * k + ri) * Nl;
-        const int m0 = Cf * a + cbase;
-        // D q^2 / 2^8 = 2^24 W0 + 2^16 W1 + 2^8 W2 + W3 is an exact integer below 2^50, so
-        // the re/im combination is done in int64 too and each output needs one conversion
-        // (through the bit pattern of 1.5 2^52: no conversion-pipe instruction).
-        const double fs = f * 256.0;
-        const bool vec_out = (Nl & 3) == 0;
-        for (int cb = 0; cb < CH; cb += 8) {
-          long long T[2][8];
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            uint32_t w[4][8];
-            if (ok) {
-#pragma unroll
-              for (int q = 0; q < 4; ++q) tc::tmem_ld8_nowait(tmem + lane_off + q * N + (half ? CH : 0) + cb, w[q]);
-              tc::tmem_wait_ld();
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              T[half][i] = ok ? ((long long)(int)w[0][i] << 24) + ((long long)(int)w[1][i] << 16) +
-                                    ((long long)(int)w[2][i] << 8) + (long long)(int)w[3][i]
-                              : 0ll;
-          }
-          float o8[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const long long x = __shfl_xor_sync(0xffffffffu, T[1][i], 1);
-            const long long v = ri ? x + T[0][i] : T[0][i] - x;
-            const double dv = __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
-            o8[i] = (float)(dv * fs);
-          }
-          if (vec_out && m0 + cb + 8 <= Nl) {  // 16-byte aligned: Nl % 4 == 0, m0 + cb % 8 == 0
-            float4* o4 = reinterpret_cast<float4*>(out + m0 + cb);
-            o4[0] = make_float4(o8[0], o8[1], o8[2], o8[3]);
-            o4[1] = make_float4(o8[4], o8[5], o8[6], o8[7]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              if (m0 + cb + i < Nl) out[m0 + cb + i] = o8[i];
-          }
-        }
-        tc::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(tfree);
-      }
     }
-  } else if (warp == kSlicerWarps + kAnchorWarps) {
+  } else if (warp == kMmaWarp) {
     // ==== MMA issuer (one thread) ======================================================
     constexpr uint32_t i1 = idesc_i8(kM, N, true, true), i2 = idesc_i8(kM, 2 * N, true, true);
     static_assert(2 * N <= 256, "B0|B1 must be one MMA operand");
@@ -521,6 +468,75 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
       }
     }
     __syncwarp();
+  } else {
+    // ==== epilogue warps: one warp per TMEM lane quarter and set of columns ==============
+    // Lane r holds row r = 2 (16 k + a) + ri of D.  For every c:
+    //   Vr = D[re, Rr] - D[im, Ri],  Vi = D[re, Ri] + D[im, Rr],
+    // so each lane sends its D[., Ri] to its neighbour (lane r ^ 1) and keeps D[., Rr]:
+    // the re lane writes Vr, the im lane Vi, for m = Cf a + cbase + c.
+    const int quarter = warp & 3, set = (warp - kMmaWarp - 1) >> 2;
+    const int r = 32 * quarter + lane;  // TMEM lane == GEMM row
+    const int ri = r & 1, j = r >> 1;
+    const int k = j >> 4, a = j & 15;
+    const int sign = ri ? -1 : 1;  // an im lane sends its D[im, Ri] negated: the re lane subtracts it
+    const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+    const int m0 = Cf * a + cbase;
+    const int vec_out = (Nl & 7) == 0 ? 8 : (Nl & 3) == 0 ? 4 : 1;  // floats per store (m0, cb: multiples of 8)
+    uint32_t piece_iter = 0;
+    for (int piece = blockIdx.x; piece < npieces; piece += gridDim.x, ++piece_iter) {
+      // D q^2 / 2^8 = 2^24 W0 + 2^16 W1 + 2^8 W2 + W3 is an exact integer below 2^50, so
+      // the re/im combination is done in int64 too and each output needs one conversion
+      // (through the bit pattern of 1.5 2^52: no conversion-pipe instruction).
+      const double fs = tc_scale(piecemax[piece]) * kKScale[k] / (kQ * kQ) * 256.0;
+      float* out = partial + ((size_t)piece * 8 + 2 * k + ri) * Nl;
+      bool ok = !*abort_flag;
+      if (ok && !tc::mbar_wait(done, piece_iter & 1, abort_flag)) {
+        fail();
+        ok = false;
+      }
+      tc::tc_fence_after();
+#pragma unroll 1
+      for (int cb = 8 * set; cb < CH; cb += 8 * kEpiSets) {
+        long long T[2][8];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t w[4][8];
+          if (ok) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tc::tmem_ld8_nowait(tmem + lane_off + q * N + (half ? CH : 0) + cb, w[q]);
+            tc::tmem_wait_ld();
+          }
+          const int sg = half ? sign : 1;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            T[half][i] = ok ? (long long)(int)w[0][i] * (sg << 24) + (long long)(int)w[1][i] * (sg << 16) +
+                                  (long long)(int)w[2][i] * (sg << 8) + (long long)(int)w[3][i] * sg
+                            : 0ll;
+        }
+        float o8[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const long long v = T[0][i] + __shfl_xor_sync(0xffffffffu, T[1][i], 1);
+          o8[i] = (float)((__longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0) * fs);
+        }
+        if (vec_out == 8 && m0 + cb + 8 <= Nl) {  // a whole sector
+          asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + m0 + cb), "f"(o8[0]),
+                       "f"(o8[1]), "f"(o8[2]), "f"(o8[3]), "f"(o8[4]), "f"(o8[5]), "f"(o8[6]), "f"(o8[7])
+                       : "memory");
+        } else if (vec_out == 4 && m0 + cb + 8 <= Nl) {
+          float4* o4 = reinterpret_cast<float4*>(out + m0 + cb);
+          o4[0] = make_float4(o8[0], o8[1], o8[2], o8[3]);
+          o4[1] = make_float4(o8[4], o8[5], o8[6], o8[7]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (m0 + cb + i < Nl) out[m0 + cb + i] = o8[i];
+        }
+      }
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(tfree);
+    }
   }
   __syncthreads();
   if (warp == 0) {
