@@ -336,7 +336,7 @@ int run_after_sort(dsht_plan_s* p, int64_t N, int mode, double* alm, const Works
     in.map[0] = fold_slot(g, ws, 0, alm, ws.alm_pol);
     launch_fold(g, w2, in.map[0], s);
     mark(DSHT_STAGE_CONTRACT);
-    launch_contract_fp64(g, p->tmY64, p->tmY8, in, 1, ws.tc_next, ws.flags, s);
+    launch_contract_fp64(g, p->tmY, in, 1, ws.tc_next, ws.flags, s);
   }
   mark(DSHT_STAGE_ROTATE);
   if (mode == DSHT_MODE_CALL) {
@@ -459,7 +459,7 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
     const bool rotate = pend.size() >= (size_t)kMaxRot || li + 1 == list.size();
     if (nfold == ws.fp64_maps || rotate) {
       prof_mark(p, DSHT_STAGE_CONTRACT, s);
-      launch_contract_fp64(g, p->tmY64, p->tmY8, in, nfold, ws.tc_next, w2.flags, s);
+      launch_contract_fp64(g, p->tmY, in, nfold, ws.tc_next, w2.flags, s);
       nfold = 0;
     }
     if (!rotate) continue;
@@ -631,7 +631,7 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
   e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(e, "table build");
-  int rc = make_table_tmaps(&p->tmY64, &p->tmY8, p->Yv, p->g);
+  int rc = make_table_tmaps(&p->tmY, p->Yv, p->g);
   if (!rc) rc = build_nufft(p, kNuFp64);
   if (rc) {
     dsht_plan_destroy(p);

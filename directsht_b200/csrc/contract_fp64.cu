@@ -21,8 +21,10 @@
 // largest columns first, so that the last items are small, and neighbour CTAs share a column's
 // fold in L2 (a fixed assignment gave some CTAs full and others partial blocks: 248 instead of
 // 220 us at Nl = 500, Nx = 1000).  Warp 0 (one thread) claims and issues, for
-// every stage of 32 nodes that has points, the table boxes (16 nodes x 64 or 8 rows, 128-byte
-// swizzle, only as many rows as the column has left) and one bulk copy per map of the fold.
+// every stage of 32 nodes that has points, the table boxes (16 nodes x 8 to 128 rows, one for each
+// binary digit of the rows that the column has left, 128-byte swizzle) and one bulk copy per map of
+// the fold.  (With boxes of 64 and 8 rows only, up to 16 issues a stage: 222 instead of 216 us at
+// Nl = 500, 1412 instead of 1382 at Nl = 1024, Nx = 2048.)
 // Warps 1-8 consume: parity (w & 1), two row tiles of eight rows of that parity each, so every
 // fold fragment feeds two products.  The fold comes in fragment order (fold.cu): lane 4 n + k
 // reads its column n and its two nodes as one 16-byte word.  Up to four maps share a pass: three
@@ -31,6 +33,13 @@
 // Products for neighbour rows go through shared memory.  Across items (the last of 128 rows and
 // the first of the next) both contributions are added with atomics onto zeros (the fold
 // kernel clears those rows); 0 + a + b does not depend on the order.
+//
+// What bounds it: at Nl = 1024, Nx = 2048 the table (1364 us, 6.30 TB/s of the 6.45 measured); at
+// smaller Nl what an item costs beyond its bytes (208 us at Nl = 500, Nx = 1000, where the bytes
+// take 155; 64-row items: 318).  So the consumers take m and the row group from the claim instead of
+// searching again, and form the square roots of an item before its first stage, while that is
+// loading (216 and 1382 us with both after the last).  Finishing an item inside the next one's stage
+// loop costs more in that loop than it hides (217, 1400); twice the accumulators change nothing.
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -107,8 +116,8 @@ struct StreamLayout {
 
 template <int G>
 __global__ void __launch_bounds__(kThreads, 1)
-contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_constant__ CUtensorMap tm64,
-                     const __grid_constant__ CUtensorMap tm8, const FoldIn in, int nstage,
+contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_constant__ TableMaps tm,
+                     const FoldIn in, int nstage,
                      unsigned* __restrict__ next_item, unsigned* __restrict__ err) {
   using L = StreamLayout<G>;
   extern __shared__ uint8_t smem_raw[];
@@ -153,16 +162,16 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
       uint32_t n = 0;  // stages issued
       for (uint32_t j = 0; !*abort_flag; ++j) {
         int item = (int)atomicAdd(next_item, 1u);
-        if (item >= nitems) item = -1;
-        item_ring[j % kItemRing] = item;
+        int m = 0, g = 0;
+        if (item < nitems) item_of(item, Nl, &m, &g);
+        else item = -1;
+        item_ring[j % kItemRing] = item < 0 ? -1 : m << 8 | g;  // g < 16384 / kRows
         tc::mbar_arrive(&item_full[j % kItemRing]);  // releases the ring entry
         if (item < 0) break;
-        int m, g;
-        item_of(item, Nl, &m, &g);
         const int l0 = m + g * kRows;
         const int row0 = (int)hp_index(l0, m, Nl);
         const int nrows = min(kRows, Nl - l0);
-        const int n64 = nrows / 64, n8 = (nrows % 64 + 7) / 8;
+        const int nr8 = (nrows + 7) / 8 * 8;  // the column's rows left, one box per set bit
         for (int t = 0; t < nstage; ++t) {
           if (!live[t]) continue;
           const int s = n % kStages;
@@ -176,12 +185,16 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
           uint8_t* st = smem + s * L::kStage;
           const uint32_t fold_bytes = (uint32_t)min(kFoldStage, (Nx - j0 + 7) / 8 * 1024);
           // boxes always transfer all their elements (zero fill out of range)
-          tc::mbar_arrive_expect_tx(&full[s], (uint32_t)(n64 * 64 + n8 * 8) * 256u + (uint32_t)G * fold_bytes);
+          tc::mbar_arrive_expect_tx(&full[s], (uint32_t)nr8 * 256u + (uint32_t)G * fold_bytes);
           for (int h = 0; h < 2; ++h) {
             uint8_t* dst = st + h * (kTab / 2);
             int r = 0;
-            for (int b = 0; b < n64; ++b, r += 64) tma_load_2d(dst + r * 128, &tm64, j0 + 16 * h, row0 + r, &full[s]);
-            for (int b = 0; b < n8; ++b, r += 8) tma_load_2d(dst + r * 128, &tm8, j0 + 16 * h, row0 + r, &full[s]);
+#pragma unroll
+            for (int b = kTableMaps - 1; b >= 0; --b)
+              if (nr8 & (8 << b)) {
+                tma_load_2d(dst + r * 128, &tm.box[b], j0 + 16 * h, row0 + r, &full[s]);
+                r += 8 << b;
+              }
           }
 #pragma unroll
           for (int k = 0; k < G; ++k)
@@ -223,14 +236,33 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
       }
       const int item = item_ring[iter % kItemRing];
       if (item < 0) break;
-      int m, g;
-      item_of(item, Nl, &m, &g);
-      const int l0 = m + g * kRows;
+      const int m = item >> 8, l0 = m + (item & 255) * kRows;
       const int nrows = min(kRows, Nl - l0);
       const bool on0 = p + 16 * tq < nrows, on1 = p + 16 * tq + 64 < nrows;
       // the tile (0 or 1) that holds the column's last row, if this warp does: it also forms x B'
       const int rl = Nl - 1 - l0 - p;  // offset of row Nl - 1 from the warp's first row of parity
       const int lt = (l0 + nrows == Nl && (rl & 1) == 0 && ((rl >> 4) & 3) == tq) ? rl >> 6 : -1;
+      // factors of the neighbour rows' products, while the item's first stages are on their way
+      auto a_l = [&](int l) {  // a_l of this column
+        return sqrt((double)(l - m) * (double)(l + m) / ((2.0 * l - 1.0) * (2.0 * l + 1.0)));
+      };
+      auto from_below = [&](int l) {  // factor of Y[l - 1] . B'
+        return (l + 1 < Nl ? (double)(l + 1) : (double)(2 * l + 1)) * a_l(l);
+      };
+      double f1[2], f2[2];
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        const int r = row[a], l = l0 + r;
+        f1[a] = f2[a] = 0.0;
+        if (r >= nrows) continue;
+        if (q < 2) {  // of rows l - 1 and l + 1, added to row l
+          if (l > m) f1[a] = from_below(l);
+          if (l + 1 < Nl) f2[a] = -(double)l * a_l(l + 1);
+        } else {  // of row l, added to a row of the item before or of the next
+          if (r == 0 && l > m) f1[a] = -(double)(l - 1) * a_l(l);
+          if (r == kRows - 1 && l + 1 < Nl) f2[a] = from_below(l + 1);
+        }
+      }
       double acc[2][G][2], accx[G][2];
 #pragma unroll
       for (int k = 0; k < G; ++k) {
@@ -299,12 +331,6 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
       // Results: lane (i, q) holds columns 2q, 2q + 1 of its row: q = 0, 1: A of the equatorial,
       // polar half, q = 2, 3: B' of them (for the neighbour rows); accx: x B' (q = 0, 1).
       double2* ex = exch + (iter & 1) * kRows * G * 2;
-      auto a_l = [&](int l) {  // a_l of this column
-        return sqrt((double)(l - m) * (double)(l + m) / ((2.0 * l - 1.0) * (2.0 * l + 1.0)));
-      };
-      auto from_below = [&](int l) {  // factor of Y[l - 1] . B'
-        return (l + 1 < Nl ? (double)(l + 1) : (double)(2 * l + 1)) * a_l(l);
-      };
       if (q >= 2) {
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
@@ -316,16 +342,14 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
             ex[(r * G + k) * 2 + (q & 1)] = v;
             double* alm = (q & 1) ? in.map[k].pol : in.map[k].equ;
             if (r == 0 && l > m) {  // to the last row of the item before
-              const double f = -(double)(l - 1) * a_l(l);
               double* o = alm + 2 * hp_index(l - 1, m, Nl);
-              atomicAdd(o, f * v.x);
-              atomicAdd(o + 1, f * v.y);
+              atomicAdd(o, f1[a] * v.x);
+              atomicAdd(o + 1, f1[a] * v.y);
             }
             if (r == kRows - 1 && l + 1 < Nl) {  // to the first row of the next item
-              const double f = from_below(l + 1);
               double* o = alm + 2 * hp_index(l + 1, m, Nl);
-              atomicAdd(o, f * v.x);
-              atomicAdd(o + 1, f * v.y);
+              atomicAdd(o, f2[a] * v.x);
+              atomicAdd(o + 1, f2[a] * v.y);
             }
           }
         }
@@ -343,20 +367,19 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
         for (int a = 0; a < 2; ++a) {
           const int r = row[a], l = l0 + r;
           if (r >= nrows) continue;
-          const double fb = l > m ? from_below(l) : 0.0, fa = l + 1 < Nl ? -(double)l * a_l(l + 1) : 0.0;
           const bool shared = (r == 0 && l > m) || (r == kRows - 1 && l + 1 < Nl);  // two items add to the row
 #pragma unroll
           for (int k = 0; k < G; ++k) {
             double vr = acc[a][k][0], vi = acc[a][k][1];
             if (r > 0) {
               const double2 e = ex[((r - 1) * G + k) * 2 + q];
-              vr = fma(fb, e.x, vr);
-              vi = fma(fb, e.y, vi);
+              vr = fma(f1[a], e.x, vr);
+              vi = fma(f1[a], e.y, vi);
             }
             if (r + 1 < nrows) {
               const double2 e = ex[((r + 1) * G + k) * 2 + q];
-              vr = fma(fa, e.x, vr);
-              vi = fma(fa, e.y, vi);
+              vr = fma(f2[a], e.x, vr);
+              vi = fma(f2[a], e.y, vi);
             }
             if (l + 1 == Nl) {
               vr = fma(-(double)l, accx[k][0], vr);
@@ -401,8 +424,8 @@ int encode_table(CUtensorMap* tm, const void* base, const Geometry& g, int box_r
 }
 
 template <int G>
-void launch_g(const Geometry& g, const CUtensorMap& tm64, const CUtensorMap& tm8, const FoldIn& in,
-              unsigned* next_item, unsigned* flags, cudaStream_t s) {
+void launch_g(const Geometry& g, const TableMaps& tm, const FoldIn& in, unsigned* next_item, unsigned* flags,
+              cudaStream_t s) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -412,25 +435,26 @@ void launch_g(const Geometry& g, const CUtensorMap& tm64, const CUtensorMap& tm8
   const int64_t grid = nitems < sms ? nitems : sms;
   const int bytes = StreamLayout<G>::bytes(nstage);
   cudaFuncSetAttribute(contract_fp64_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  contract_fp64_kernel<G><<<(unsigned)grid, kThreads, bytes, s>>>(g.Nl, g.Nx, g.dx, nitems, tm64, tm8, in, nstage,
+  contract_fp64_kernel<G><<<(unsigned)grid, kThreads, bytes, s>>>(g.Nl, g.Nx, g.dx, nitems, tm, in, nstage,
                                                                   next_item, flags);
   count_launches(1);
 }
 
 }  // namespace
 
-int make_table_tmaps(CUtensorMap* tm64, CUtensorMap* tm8, const void* base, const Geometry& g) {
-  if (int rc = encode_table(tm64, base, g, 64)) return rc;
-  return encode_table(tm8, base, g, 8);
+int make_table_tmaps(TableMaps* tm, const void* base, const Geometry& g) {
+  for (int b = 0; b < kTableMaps; ++b)
+    if (int rc = encode_table(&tm->box[b], base, g, 8 << b)) return rc;
+  return DSHT_OK;
 }
 
-void launch_contract_fp64(const Geometry& g, const CUtensorMap& tm64, const CUtensorMap& tm8, const FoldIn& in,
-                          int nmaps, unsigned* next_item, unsigned* flags, cudaStream_t s) {
+void launch_contract_fp64(const Geometry& g, const TableMaps& tm, const FoldIn& in, int nmaps, unsigned* next_item,
+                          unsigned* flags, cudaStream_t s) {
   switch (nmaps) {
-    case 1: launch_g<1>(g, tm64, tm8, in, next_item, flags, s); break;
-    case 2: launch_g<2>(g, tm64, tm8, in, next_item, flags, s); break;
-    case 3: launch_g<3>(g, tm64, tm8, in, next_item, flags, s); break;
-    default: launch_g<4>(g, tm64, tm8, in, next_item, flags, s); break;
+    case 1: launch_g<1>(g, tm, in, next_item, flags, s); break;
+    case 2: launch_g<2>(g, tm, in, next_item, flags, s); break;
+    case 3: launch_g<3>(g, tm, in, next_item, flags, s); break;
+    default: launch_g<4>(g, tm, in, next_item, flags, s); break;
   }
 }
 

@@ -56,6 +56,11 @@ struct TcOut {
 // One pass of the FP64 contraction: each map's fold, its equatorial and rotated polar alm.
 constexpr int kFp64Maps = 4;
 constexpr int kContractRows = 128;  // rows of one work item
+// Tensor maps of the FP64 table Yv with boxes of 8, 16, 32, 64 and 128 rows.
+constexpr int kTableMaps = 5;
+struct alignas(64) TableMaps {
+  CUtensorMap box[kTableMaps];
+};
 struct FoldOut {
   double* fold;   // fold.cu's layout
   uint8_t* live;  // [ceil(Nx/16)] any point feeds a node of the block of 16
@@ -191,10 +196,10 @@ int launch_contract_tc(const Geometry& g, const CUtensorMap& tmA, const uint32_t
                        const TcOut& out, unsigned* flags, unsigned* next_item, cudaStream_t s);
 
 // FP64 contraction of the Y table (contract_fp64.cu) for nmaps <= kFp64Maps folds.
-void launch_contract_fp64(const Geometry& g, const CUtensorMap& tm64, const CUtensorMap& tm8, const FoldIn& in,
-                          int nmaps, unsigned* next_item, unsigned* flags, cudaStream_t s);
-// 2D tensor maps of an FP64 table (node x row), boxes of 16 nodes x 64 and 8 rows.
-int make_table_tmaps(CUtensorMap* tm64, CUtensorMap* tm8, const void* base, const Geometry& g);
+void launch_contract_fp64(const Geometry& g, const TableMaps& tm, const FoldIn& in, int nmaps, unsigned* next_item,
+                          unsigned* flags, cudaStream_t s);
+// 2D tensor maps of an FP64 table (node x row), boxes of 16 nodes x 8 to 128 rows.
+int make_table_tmaps(TableMaps* tm, const void* base, const Geometry& g);
 // An FP64 table in the JAX path's layout out[m][l - m][j] (Nl x Nl x Nx doubles, zeros
 // where l >= Nl) on the device.
 void launch_table_mlayout(const Geometry& g, const double* t64, double* out, cudaStream_t s);
@@ -258,7 +263,7 @@ struct dsht_plan_s {
   double* Yv = nullptr;  // FP64 tables (null in a compact plan)
   void* rot_tab = nullptr;  // tables of the rotation (rotate.cu)
   double* Yd = nullptr;
-  alignas(64) CUtensorMap tmY64, tmY8;  // boxes of 64 and 8 rows of Yv
+  dsht::TableMaps tmY;
   // Digit tables of the tensor-core contraction (digits.cu): 4 planes [Nlm][Kp] int8 in
   // rows grouped by parity, row exponents, the work items and the TMA map of the planes.
   uint8_t* dig = nullptr;
