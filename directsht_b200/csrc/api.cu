@@ -72,13 +72,14 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
   };
   const int64_t n = N > 0 ? N : 1;
   // Pieces of a transform of up to n points.  A workspace laid out for the NUFFT sums' large
-  // pieces also serves the smaller transforms of a batch, which may take the direct sums:
-  // their pieces of default_piece_max(N) or at most 2048 points number at most
-  // max(2048, N / 2048) beyond one per key, with N below the NUFFT threshold.
+  // pieces also serves smaller transforms (of a batch, or of later calls), which may take the direct
+  // sums, with N below the NUFFT threshold: their pieces of default_piece_max(N) number at
+  // most min(2048, N / 256) or N / 2048 beyond one per key.
   int64_t extra = (n + piece_max - 1) / piece_max;
   if (nu_grid) {
     const int64_t direct_n = std::min<int64_t>(n, (int64_t)kNufftMinPerKey * g.nkeys);
-    extra = std::max<int64_t>(extra, std::max<int64_t>(2048, (direct_n + 2047) / 2048));
+    extra = std::max(extra, std::min<int64_t>(2048, (direct_n + 255) / 256));
+    extra = std::max<int64_t>(extra, (direct_n + 2047) / 2048);
   }
   const int64_t pmax = std::min<int64_t>(g.nkeys, n) + extra;
   Workspace w{};
@@ -172,11 +173,20 @@ int plan_piece_max(const dsht_plan_s* p, int64_t N) {
   return std::min(pm, 2048);
 }
 
+// CTAs of the NUFFT sums of N points, 0 for the direct sums: no more than there can be pieces.
+int plan_nufft_grid(const dsht_plan_s* p, int64_t N) {
+  const int cls = plan_nufft_class(p, N);
+  if (cls < 0) return 0;
+  const int64_t pm = plan_piece_max(p, N);
+  const int64_t pieces = std::min<int64_t>(p->g.nkeys, N) + (N + pm - 1) / pm;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(nufft_grid(p->g.Nl, cls), pieces));
+}
+
 // Sets the workspace for a transform of N points: its piece size and its NUFFT run, if any.
 void route_workspace(const dsht_plan_s* p, int64_t N, Workspace& w) {
   const int cls = plan_nufft_class(p, N);
   w.piece_max = plan_piece_max(p, N);
-  w.nu_grid = cls >= 0 ? nufft_grid(p->g.Nl, cls) : 0;
+  w.nu_grid = plan_nufft_grid(p, N);
   w.nu_piece_cost = cls >= 0 ? nufft_piece_cost(p->g.Nl, cls) : 0;
 }
 
@@ -565,9 +575,8 @@ size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* b
   // maps per tensor-core contraction pass (digit tables): up to kTcMaxMaps unless tuned
   const int tc = multi ? std::min(std::max(ntrans, 1), p->tune_maps_per_pass > 0 ? p->tune_maps_per_pass
                                                                                   : kTcMaxMaps) : 1;
-  const int cls = plan_nufft_class(p, N);
   return workspace_layout(p->g, N, plan_piece_max(p, N), base, ws, multi, tc, std::min(tc, kFp64Maps),
-                          cls >= 0 ? nufft_grid(p->g.Nl, cls) : 0);
+                          plan_nufft_grid(p, N));
 }
 
 }  // namespace dsht
