@@ -141,22 +141,23 @@ def dram_traffic(stage, precision, N, Nlm, Nx):
     return e["bytes_per_point"] * N + e.get("bytes_per_table_entry", 0.0) * Nlm * Nx
 
 
-def nufft_logn(Nl):
-    """log2 of the NUFFT grid: 4 x 2^ceil(log2 Nl) cells, at least 128 (nufft.cu)."""
-    lg = max(int(np.ceil(np.log2(max(Nl, 1)))), 0) + 2
+def nufft_logn(Nl, fp64=False):
+    """log2 of the NUFFT grid: 4 x 2^ceil(log2 Nl) cells (8 x at the FP64 level up to Nl = 256), at least 128
+    (nufft.cu)."""
+    lg = max(int(np.ceil(np.log2(max(Nl, 1)))), 0) + (3 if fp64 and Nl <= 256 else 2)
     return max(lg, 7)
 
 
-def nufft_pieces(th, ph, Nx, xmax, piece):
-    """Bin pieces of a point set as the sort forms them: per (set, bin) key ceil(count/piece)."""
+def nufft_nodes(th, ph, Nx, xmax):
+    """Spline nodes next to a bin with points, over the four sets: one FFT of the NUFFT sums each."""
     c = np.cos(th)
     pol = np.abs(c) >= xmax
     x = np.where(pol, -np.sin(th) * np.cos(ph), c)
     nb = Nx - 1
     j = np.minimum((np.abs(x) * (nb / xmax)).astype(np.int64), nb - 1)
-    key = (np.where(pol, 2, 0) + (x < 0)) * nb + j
-    counts = np.bincount(key, minlength=4 * nb)
-    return int(((counts + piece - 1) // piece).sum())
+    live = np.zeros((4, nb), bool)
+    live.reshape(-1)[(np.where(pol, 2, 0) + (x < 0)) * nb + j] = True
+    return int((live[:, 1:] | live[:, :-1]).sum() + live[:, 0].sum() + live[:, -1].sum())
 
 
 def measured_peaks():
@@ -605,6 +606,9 @@ def main(argv=None):
     # FP64 direct sums below 28 and the tensor-core sums in between (DSHT_TUNE_BIN_SUMS)
     bin_method = args.bin_sums if args.bin_sums != "auto" else (
         "nufft" if N >= 512 * 4 * (Nx - 1) else "fp64" if N < 28 * 4 * (Nx - 1) else "tc")
+    if args.precision == "fp64":  # the FP64 level: the NUFFT sums from 11 grids of points per key and Nl, else direct
+        nu = N * Nl >= 11 * (1 << nufft_logn(Nl, True)) * 4 * (Nx - 1) and nufft_logn(Nl, True) <= 13
+        bin_method = "nufft" if args.bin_sums == "nufft" or (nu and args.bin_sums != "fp64") else "fp64"
     # eight point sets per headline step: one contraction pass holds up to eight (32 fold
     # columns), so the table read is shared by all of them
     batch = args.batch if args.batch is not None else (8 if args.workload == "c2" else 1)
@@ -614,8 +618,8 @@ def main(argv=None):
     main = single
     if batch > 1:
         # The headline: `batch` independent point sets of the same distribution per step,
-        # one dsht_enqueue_batch call (the contraction reads the tables once per three
-        # point sets, the rotation shares one recursion); point set 0 is the one above.
+        # one dsht_enqueue_batch call (the contraction reads the tables once for all of
+        # them, the rotation shares one recursion); point set 0 is the one above.
         sets = [(thd, phd, wd)] + [tuple(torch.from_numpy(a).to(dev) for a in make_points(spec, seed=1000 * rank + i))
                                    for i in range(1, batch)]
         balm = torch.empty((batch, d.Nlm), dtype=torch.complex128, device=dev)
@@ -694,8 +698,10 @@ def main(argv=None):
     # Stage times sum every launch of the step: with several maps, bin sums, fold and rotation
     # ran once per map and the contraction once per pass of maps_per_pass maps.
     # maps per contraction pass: the tensor-core contraction serves up to 8 per table read,
-    # the FP64 CUDA-core contraction one
-    per_pass = (d.tune()["maps_per_pass"] or (8 if args.precision == "mixed" else 1)) if maps > 1 else 1
+    # the FP64 contraction up to 4
+    per_pass = (d.tune()["maps_per_pass"] or (8 if args.precision == "mixed" else 4)) if maps > 1 else 1
+    if args.precision != "mixed":
+        per_pass = min(per_pass, 4)
     passes = -(-maps // per_pass)
     # point sets per step: the headline step's stage times cover `batch` sets (points, bin
     # sums, fold and rotation once per set; one contraction pass serves all of them)
@@ -707,14 +713,13 @@ def main(argv=None):
         if ms <= 0:
             return None
         if name == "contract":
-            eb = 4 if f32_tables else 8
-            alg = 2.0 * eb * d.Nlm * Nx * passes
+            alg = 8.0 * d.Nlm * Nx * passes
             a = alg / (ms * 1e-3) / 1e9
             kern = ("contract_tc_kernel (tcgen05 kind::i8 on 4-byte digit tables, TMA 3D boxes)" if f32_tables
-                    else "contract_stream_kernel (FP64 tables, TMA 2D tiles)")
+                    else "contract_fp64_kernel (FP64 table of Y, matrix instructions fed by TMA 2D boxes)")
             return {"kernel": kern, "bound": "hbm", "achieved": a,
                     "peak": hbm_peak, "unit": "GB/s", "frac": a / hbm_peak, "peak_source": peak_src,
-                    "algorithmic": f"{2 * eb} B of {'digit' if f32_tables else 'FP64'} table (Yv, Yd) per "
+                    "algorithmic": f"8 B of {'digit tables (Yv, Yd)' if f32_tables else 'the FP64 table Yv'} per "
                                    f"(l, m, node) per pass ({passes} passes)"}
         if name == "points":
             alg = 56.0 * N * nsets
@@ -722,28 +727,30 @@ def main(argv=None):
             return {"kernel": "count/scan/scatter (counting sort by bin)", "bound": "hbm", "achieved": a,
                     "peak": hbm_peak, "unit": "GB/s", "frac": a / hbm_peak, "peak_source": peak_src,
                     "algorithmic": "24 B of inputs read + 32 B of sorted record written per point"}
-        if name == "bin_sums" and args.precision != "fp64" and bin_method == "nufft":
-            # the NUFFT kernel's own FP64 work: per point 132 DFMA of kernel values, 48
-            # products and fixed-point conversions of the spread, ~50 for atan2 and the
-            # Hermite weights; per piece two complex FFTs of n cells (5 n log2 n each)
-            logn = nufft_logn(Nl)
-            pieces = nufft_pieces(th, ph, Nx, 0.75, 8192)
-            alg = (400.0 * N + pieces * 2 * 5.0 * (1 << logn) * logn * (2 if logn > 12 else 1)) * maps * nsets
+        if name == "bin_sums" and bin_method == "nufft":
+            # the NUFFT kernel's own FP64 work: per point the kernel values (two polynomials in s^2 per
+            # pair of cells), four FMA per cell of its window and ~20 for the weights; per node one
+            # complex FFT of n cells (5 n log2 n)
+            f64 = args.precision == "fp64"
+            W, logn = (16 if f64 else 12), nufft_logn(Nl, f64)
+            nodes = nufft_nodes(th, ph, Nx, 0.75)
+            per_point = 2.0 * (W * (W + 2) / 2 + 4 * W + 20)
+            alg = (per_point * N + nodes * 5.0 * (1 << logn) * logn) * maps * nsets
             a = alg / (ms * 1e-3) / 1e12
-            return {"kernel": "nufft_sums_kernel (FP64 spread, shared-memory FFT)", "bound": "fp64",
-                    "achieved": a, "peak": 40.0, "unit": "TFLOP/s", "frac": a / 40.0,
+            return {"kernel": "nufft_nodes_kernel (sorted spread in registers, shared-memory FFT per node)",
+                    "bound": "fp64", "achieved": a, "peak": 40.0, "unit": "TFLOP/s", "frac": a / 40.0,
                     "peak_source": "nominal (no measured FP64 figure)",
-                    "algorithmic": f"400 flop per point + 10 n log2 n per piece ({pieces} pieces, n = {1 << logn}) "
-                                   f"x {nsets} point sets",
-                    "bound_note": "the kernel's own limit is its shared-memory pipe (96 32-bit reductions per "
-                                  "point for the spread, the in-place FFT): L1/TEX throughput 79 % of peak in the "
-                                  "ncu capture summarised in profiles/nufft_sums_c2prof.md; no FP64 peak is "
-                                  "measured here, so the fp64 fraction uses the nominal 40 TFLOP/s",
+                    "algorithmic": f"{per_point:.0f} flop per point + 5 n log2 n per node ({nodes} nodes, n = "
+                                   f"{1 << logn}) x {nsets} point sets",
+                    "bound_note": "the kernel's own limit is the issue of its spread (11 clocks of an SM per "
+                                  "point, 392 of 766 us at Nl=1024, N=1e7) and the shared-memory round trips of "
+                                  "the FFT (152 us); no FP64 peak is measured here, so the fp64 fraction uses "
+                                  "the nominal 40 TFLOP/s",
                     "equivalent_direct": {"value": 24.0 * N * Nl * maps * nsets / (ms * 1e-3) / 1e12,
                                           "unit": "TFLOP/s",
                                           "what": "24 flop per (point, m, map) of the direct sums over the "
                                                   "stage time: the rate the direct method would need"}}
-        if name == "bin_sums" and args.precision != "fp64" and bin_method == "tc":
+        if name == "bin_sums" and bin_method == "tc":
             alg = 24.0 * N * Nl * maps * nsets
             a = alg / (ms * 1e-3) / 1e12
             ops = 2.0 * 128 * (2 * C) * 8 * N * maps * nsets
@@ -768,7 +775,7 @@ def main(argv=None):
             # map; the recursion that forms d (shared by the maps of a launch) is not counted
             alg = 2.0 * 2 * sum((l + 1) ** 2 for l in range(Nl)) * maps * nsets
             a = alg / (ms * 1e-3) / 1e12
-            return {"kernel": "rotate_back_kernel" if maps * nsets == 1 else "rotate_back_maps_kernel",
+            return {"kernel": "rotate_back_kernel",
                     "bound": "fp64", "achieved": a, "peak": 40.0,
                     "unit": "TFLOP/s", "frac": a / 40.0, "peak_source": "nominal (no measured FP64 figure)",
                     "algorithmic": "2 FMA per (l, m >= 0, m' >= 0, map): real d^l_{mm'}(pi/2) times a complex "

@@ -41,11 +41,11 @@
 //
 // What bounds it: the accumulators fill TMEM at CH = 64, so a piece's MMAs wait for the epilogue
 // of the piece before.  In the slicer warps that cost 30 % of the kernel (Nl = 1024, Nx = 2048,
-// N = 2e6: 1240 us a map with gather and piece maxima, 870 without any epilogue); warps of its own,
-// the sign of Vr folded into the exchanged value and one 32-byte store per lane and step made it
-// 1117.  The rest is shared evenly by anchors and slicers, one warp per sub-partition each: without
-// either 160 us less, without both 420.  More slicer or epilogue warps cost more in registers (80 to
-// 96 a thread spill: 1290-1430 us) than they hide, and so do uneven halves of the anchors (1153).
+// N = 2e6, eight maps: 620 us a map with gather and piece maxima, 434 without any epilogue); warps of
+// its own, the sign of Vr folded into the exchanged value and one 32-byte store per lane and step
+// made it 558.  The rest is shared evenly by anchors and slicers, one warp per sub-partition each:
+// without either 80 us less, without both 210.  More slicer or epilogue warps cost more in registers
+// (80 to 96 a thread spill: 643-714 us) than they hide, and so do uneven halves of the anchors (577).
 //
 // FP64 is the limiting pipe: while int8 MMAs run, an SM sub-partition issues about one
 // FP64 warp instruction in 16 clocks (one in 2 on an SM that has not used its tensor

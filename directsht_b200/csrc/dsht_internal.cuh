@@ -1,9 +1,10 @@
 // Internal declarations shared by the DirectSHT B200 kernels.
 //
 // Data layout in HBM (Nlm = Nl(Nl+1)/2, rows in Healpy order m(2Nl-1-m)/2 + l):
-//   tables   Yv, Yd      double [Nlm][Nx]          (sht/sht.py:50-56 layout, numpy path)
+//   tables   Yv, Yd      double [Nlm][pitch]       (sht/sht.py:50-56 layout, numpy path; Nx even up)
 //   points   key         uint32 [N]                set*(Nx-1) + bin, or DSHT_KEY_DROP
-//            sorted      double [N][4]             (cos phi, sin phi, w, t) by key
+//            sorted      double [N][4]             (cos phi, sin phi, w, t) by key; for the NUFFT sums
+//                                                  (turns hi, lo, w, t)
 //   pieces   <= 1 bin each, <= piece_max points    (key, start, len)
 //   partial  double [piece][8][Nl]                 (k, re/im) bin sums for every m
 //   fold     double [Nl][Nx/8][2 parity][8][8]     columns A, B' of eight nodes (fold.cu)

@@ -1,7 +1,6 @@
 // The FP64 Ylm / dYlm recurrences of one column m at one node x, step by step in l.
 //
-// Shared by the table build (tables.cu) and by the kernels that regenerate table values on
-// the fly (heavy.cu), so both produce bitwise the same numbers.  Every product and sum is a
+// Used by the table build (tables.cu).  Every product and sum is a
 // separately rounded __dmul_rn / __dadd_rn / __ddiv_rn in the order of the reference's
 // numpy/numba path:
 //   Y_mm        = prod_{k=1..m} (-sqrt(1 - 1/2k) sx)              sht/legendre_py.py:28-30

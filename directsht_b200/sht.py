@@ -103,8 +103,8 @@ class DirectSHT:
 
     def tune(self, piece_max=None, maps_per_pass=None, bin_sums=None):
         """Set tuning parameters (``dsht_plan_tune``); None leaves one unchanged, 0 (or
-        'auto') restores the automatic choice.  bin_sums picks the mixed levels' per-bin sums:
-        'nufft', 'tc' (direct tensor-core sums), 'fp64' (direct FP64 sums) or 'auto' (the
+        'auto') restores the automatic choice.  bin_sums picks the per-bin sums: 'nufft',
+        'tc' (direct tensor-core sums, mixed levels), 'fp64' (direct FP64 sums) or 'auto' (the
         default).  Returns the current values
         as a dict (bin_sums as its name)."""
         if piece_max is not None:

@@ -68,8 +68,10 @@ enum {
 };
 
 /* Arithmetic of a plan's transforms.
- *   DSHT_PREC_FP64  : FP64 CUDA-core per-bin sums and FP64 tables; agrees with the
- *                     reference's numpy path to about 1e-15 (tested at <= 1e-12 x max|alm|).
+ *   DSHT_PREC_FP64  : FP64 per-bin sums -- direct, or by a type-1 non-uniform FFT of the same
+ *                     accuracy where bins hold many points (DSHT_TUNE_BIN_SUMS) -- and FP64
+ *                     tables; agrees with the reference's numpy path to about 1e-15 (tested at
+ *                     <= 1e-12 x max|alm|).
  *   DSHT_PREC_MIXED : per-bin sums (see DSHT_TUNE_BIN_SUMS for the choice) by a type-1
  *                     non-uniform FFT in FP64 (each bin's points
  *                     spread onto a periodic grid of 4 x 2^ceil(log2 Nl) cells with a width-12
@@ -108,11 +110,16 @@ int dsht_get_precision(dsht_plan_t plan, int* precision);
 /* Tuning of a plan (no counterpart in the reference; results do not depend on it beyond
  * the stated precision).  DSHT_TUNE_PIECE_MAX: points per bin piece of the per-bin sums, a
  * multiple of 32 in [256, 65536], 0 = chosen from N and the method (the direct sums, FP64 and
- * tensor-core, cap it at 2048; the NUFFT sums default to 8192).  DSHT_TUNE_MAPS_PER_PASS:
+ * tensor-core, cap it at 2048; the NUFFT sums at 4096, the default there, or 2048 where their
+ * grid has fewer than 4096 cells).  DSHT_TUNE_MAPS_PER_PASS:
  * maps or point sets that share one read of the tables in a multi-transform call, 1..8,
- * 0 = the most (8 with the tensor-core contraction, 4 with the FP64 one).  DSHT_TUNE_BIN_SUMS: the bin sums of the mixed levels, DSHT_BIN_SUMS_NUFFT,
- * DSHT_BIN_SUMS_TC (the direct int8-slice tensor-core sums) or DSHT_BIN_SUMS_FP64 (the direct
- * FP64 CUDA-core sums of the fp64 level); AUTO (the default) chooses per transform (so the
+ * 0 = the most (8 with the tensor-core contraction, 4 with the FP64 one).  DSHT_TUNE_BIN_SUMS:
+ * the bin sums, DSHT_BIN_SUMS_NUFFT,
+ * DSHT_BIN_SUMS_TC (the direct int8-slice tensor-core sums, mixed levels only) or
+ * DSHT_BIN_SUMS_FP64 (the direct FP64 CUDA-core sums).  At the FP64 level AUTO (the default)
+ * takes the NUFFT sums from N Nl >= 44 n (Nx - 1) for a grid of n cells, n = 4 x 2^ceil(log2 Nl)
+ * (8 x up to Nl = 256), and the direct sums below.  At the mixed levels AUTO chooses per
+ * transform (so the
  * transforms of one batch call may differ) from its points per bin key on average: the
  * NUFFT sums from 512 (N >= 2048 (Nx - 1)), where their fixed cost per bin piece pays off,
  * the FP64 direct sums below 28 (N < 112 (Nx - 1): pieces of a few points, where the
@@ -120,7 +127,7 @@ int dsht_get_precision(dsht_plan_t plan, int* precision);
  * tensor-core sums in between.  Workspace sizes depend on all three: query them after
  * tuning. */
 enum { DSHT_TUNE_PIECE_MAX = 1, DSHT_TUNE_MAPS_PER_PASS = 2, DSHT_TUNE_BIN_SUMS = 3 };
-/* Values of DSHT_TUNE_BIN_SUMS: the bin-sum method of the mixed levels. */
+/* Values of DSHT_TUNE_BIN_SUMS. */
 enum { DSHT_BIN_SUMS_AUTO = 0, DSHT_BIN_SUMS_NUFFT = 1, DSHT_BIN_SUMS_TC = 2, DSHT_BIN_SUMS_FP64 = 3 };
 int dsht_plan_tune(dsht_plan_t plan, int param, int value);
 int dsht_plan_get_tune(dsht_plan_t plan, int param, int* value);
@@ -303,8 +310,8 @@ int dsht_test_stall_next_contraction(void);
 int dsht_test_point_keys(dsht_plan_t plan, const double* theta, const double* phi, int64_t N, int mode,
                          uint32_t* keys, unsigned* flags, void* stream);
 
-/* Test hook, no counterpart in the reference: the host-side tables of the NUFFT bin sums for
- * Nl <= 2048 -- *logn = log2 of the grid cells, poly[12][12] the monomial coefficients (in
+/* Test hook, no counterpart in the reference: the host-side tables of the mixed levels' NUFFT bin
+ * sums for Nl <= 2048 -- *logn = log2 of the grid cells, poly[12][12] the monomial coefficients (in
  * s = 2f - 1) of the kernel values at the 12 cells next to a point of fractional cell offset
  * f, dinv[Nl] = 1 / Psi(m).  Needs no GPU. */
 int dsht_test_nufft_tables(int Nl, int* logn, double* poly, double* dinv);
