@@ -50,3 +50,14 @@ def test_threads_and_streams():
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_pinned_views_are_copied_directly():
+    """A numpy view of pinned memory keeps the link's rate: one copy, no staging, the same bytes."""
+    import torch
+    from directsht_b200.hostcopy import to_device
+    p = torch.empty(3 << 20, dtype=torch.uint8).pin_memory()
+    a = p.numpy()
+    a[:] = np.arange(a.size, dtype=np.int64) % 251
+    d = to_device(a, torch.device("cuda"))
+    assert torch.equal(d.cpu(), p)
