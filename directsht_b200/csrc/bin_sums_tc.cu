@@ -481,7 +481,9 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
     const int sign = ri ? -1 : 1;  // an im lane sends its D[im, Ri] negated: the re lane subtracts it
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const int m0 = Cf * a + cbase;
-    const int vec_out = (Nl & 7) == 0 ? 8 : (Nl & 3) == 0 ? 4 : 1;  // floats per store (m0, cb: multiples of 8)
+    // floats per store (m0 and cb are multiples of 8; a caller's workspace may be 16-byte aligned only)
+    const bool sectors = (Nl & 7) == 0 && (reinterpret_cast<uintptr_t>(partial) & 31) == 0;
+    const int vec_out = sectors ? 8 : (Nl & 3) == 0 ? 4 : 1;
     uint32_t piece_iter = 0;
     for (int piece = blockIdx.x; piece < npieces; piece += gridDim.x, ++piece_iter) {
       // D q^2 / 2^8 = 2^24 W0 + 2^16 W1 + 2^8 W2 + W3 is an exact integer below 2^50, so
