@@ -36,7 +36,7 @@ fold_kernel(int Nl, int Nx, int nbins, int ngroups, double dx, const Src src, co
   const int m = m0 + lane, j = j0 + warp;
   double* out = stage + lane * kRowDoubles + (warp >> 3) * 128 + ((warp & 7) >> 1) * 2 + (warp & 1);
   const double x = (double)j * dx;
-  const double bf = dx / (1.0 - x * x);
+  const double bf = j < Nx ? dx / (1.0 - x * x) : 0.0;  // (a padding node may lie at x = 1)
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     double acc[2][4];

@@ -61,3 +61,24 @@ def test_no_points_in_range_gives_zeros():
     from directsht_b200 import DirectSHT
     got = DirectSHT(140, 40)(np.full(5, np.nan), np.zeros(5), np.ones(5))
     assert not got.any()
+
+
+# grids whose padding nodes (beyond Nx, up to a whole group of eight) include x = 1
+@pytest.mark.parametrize("precision", ["fp64", "mixed_f64_tables", "mixed"])
+@pytest.mark.parametrize("Nl,Nx,xmax", [(20, 4, 0.75), (20, 10, 0.75), (20, 17, 0.8), (20, 19, 0.9), (40, 49, 0.96),
+                                        (40, 100, 0.99)])
+def test_padding_nodes_at_x_equal_to_one(Nl, Nx, xmax, precision):
+    from directsht_b200 import DirectSHT
+    dx = xmax / (Nx - 1)
+    assert any(j * dx == 1.0 for j in range(Nx, (Nx + 7) // 8 * 8))
+    rng = np.random.default_rng(Nx)
+    th, ph = _sky(rng, 600)  # below the 1024 points from which the mixed levels leave the FP64 stages
+    w = rng.normal(size=(2, 600))
+    tab = O.build_tables(Nl, Nx, xmax)
+    d = DirectSHT(Nl, Nx, xmax, precision=precision)
+    maps = d.call_maps(th, ph, w)
+    for k in range(2):
+        ref = O.direct_sht(tab, th, ph, w[k])
+        tol = 1e-12 * np.abs(ref).max()
+        assert np.abs(d(th, ph, w[k]) - ref).max() <= tol
+        assert np.abs(maps[k] - ref).max() <= tol
