@@ -352,7 +352,7 @@ int run_after_sort(dsht_plan_s* p, int64_t N, int mode, double* alm, const Works
   if (mode == DSHT_MODE_CALL) {
     RotMaps rm{};
     rm.rot[0] = ws.alm_pol;
-    rm.io[0] = alm;
+    rm.add[0] = rm.out[0] = alm;
     rm.flags[0] = ws.flags;
     launch_rotate_back(g, rm, 1, rotation_tables(p->rot_tab, g.Nl), s);
   }
@@ -427,7 +427,7 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
       out.equ[k] = items[pass[k]].alm;
       out.pol[k] = ws.alm_pol + nlm2 * k;
       rm.rot[k] = out.pol[k];
-      rm.io[k] = items[pass[k]].alm;
+      rm.add[k] = rm.out[k] = items[pass[k]].alm;
       rm.flags[k] = ws.slot_flags + k;
       so.slot[k] = ws.slot_flags + k;
       so.status[k] = items[pass[k]].status;
@@ -477,7 +477,7 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
     StatusOut so{};
     for (size_t k = 0; k < pend.size(); ++k) {
       rm.rot[k] = ws.alm_pol + nlm2 * k;
-      rm.io[k] = items[pend[k]].alm;
+      rm.add[k] = rm.out[k] = items[pend[k]].alm;
       rm.flags[k] = ws.slot_flags + k;
       so.slot[k] = ws.slot_flags + k;
       so.status[k] = items[pend[k]].status;
@@ -1018,12 +1018,10 @@ int dsht_rotate_back(dsht_plan_t p, const double* alm_rot, const double* alm_add
                      void* stream) {
   if (!p || !alm_rot || !alm_out) return set_error(DSHT_ERR_INVALID, "invalid arguments");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const size_t bytes = sizeof(double) * 2 * p->g.Nlm;
-  if (!alm_add) DSHT_CUDA_OK(cudaMemsetAsync(alm_out, 0, bytes, s));
-  else if (alm_add != alm_out) DSHT_CUDA_OK(cudaMemcpyAsync(alm_out, alm_add, bytes, cudaMemcpyDeviceToDevice, s));
   RotMaps rm{};
   rm.rot[0] = alm_rot;
-  rm.io[0] = alm_out;
+  rm.add[0] = alm_add;
+  rm.out[0] = alm_out;
   launch_rotate_back(p->g, rm, 1, rotation_tables(p->rot_tab, p->g.Nl), s);
   DSHT_CUDA_OK(cudaGetLastError());
   return DSHT_OK;

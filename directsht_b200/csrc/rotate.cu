@@ -129,7 +129,7 @@ __global__ void rotation_alpha_kernel(int Nl, const double* __restrict__ sc, dou
   al[at] = k >= 1 ? sc[at] / (sqrt((double)(l + k) * (double)(l - k + 1)) * sc[at + 1]) : 0.0;
 }
 
-// Columns m = m0, m0 + blockDim, ... (C of them, one parity) of degree l: io[map] += R(rot[map]).
+// Columns m = m0, m0 + blockDim, ... (C of them, one parity) of degree l: out[map] = add[map] + R(rot[map]).
 // al: [i], S: [map][i] the coefficients of this parity's alternating real and imaginary rows, both
 // padded with zeros.
 template <int kMaps, int C>
@@ -198,9 +198,10 @@ __device__ __forceinline__ void rotate_columns(int Nl, int l, int m0, int map0, 
 #pragma unroll
     for (int g = 0; g < kMaps; ++g) {
       if (g < nm && (!maps.flags[map0 + g] || (*maps.flags[map0 + g] & kFlagHasPolar))) {
-        double* out = maps.io[map0 + g];
-        out[at] += ((m & 1) ? s[j][g][1] : s[j][g][0]) * f;
-        out[at + 1] += ((m & 1) ? s[j][g][0] : s[j][g][1]) * f;
+        const double* add = maps.add[map0 + g];
+        double* out = maps.out[map0 + g];
+        out[at] = (add ? add[at] : 0.0) + ((m & 1) ? s[j][g][1] : s[j][g][0]) * f;
+        out[at + 1] = (add ? add[at + 1] : 0.0) + ((m & 1) ? s[j][g][0] : s[j][g][1]) * f;
       }
     }
   }

@@ -207,7 +207,7 @@ int dsht_enqueue_batch(dsht_plan_t plan, int ntrans, const double* const* theta,
 
 /* alm_out = alm_add + R(alm_rot): alm of points rotated by +90 deg about y rotated back to
  * the original frame with Wigner d(pi/2) (DEVICE pointers, 2*Nlm doubles each; alm_add may be
- * NULL for zeros, alm_out may alias alm_add).  Replaces healpy's
+ * NULL for zeros, alm_out may be alm_rot or alm_add).  Replaces healpy's
  * Rotator(rot=(0,90,0), eulertype='ZYZ', inv=True).rotate_alm at sht/sht.py:138-139. */
 int dsht_rotate_back(dsht_plan_t plan, const double* alm_rot, const double* alm_add, double* alm_out,
                      void* stream);

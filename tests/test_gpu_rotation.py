@@ -58,3 +58,30 @@ def test_maps_equal_single_rotations(nmaps):
     for k in range(nmaps):
         ref = d(th, ph, w[k])
         assert np.abs(got[k] - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("Nl", [1, 64, 65, 300, 1030])
+def test_rotate_back_in_place(Nl):
+    """alm_out may be any of the inputs: the result is that of separate arrays, bit for bit."""
+    import torch
+    from directsht_b200 import DirectSHT
+    from directsht_b200 import _lib as L
+    rng = np.random.default_rng(Nl)
+    d = DirectSHT(Nl, 2)
+    a, b = (torch.from_numpy(_random_alm(rng, Nl)).cuda() for _ in range(2))
+
+    def rotate(rot, add, out):
+        L.check(d._lib.dsht_rotate_back(d._plan, L.ptr(rot), None if add is None else L.ptr(add), L.ptr(out), None))
+        torch.cuda.synchronize()
+        return out
+
+    new = lambda: torch.full_like(a, float("nan"))
+    sum_ab, rot_a, sum_aa = rotate(a, b, new()), rotate(a, None, new()), rotate(a, a, new())
+    x, y = a.clone(), b.clone()
+    assert torch.equal(rotate(x, y, x), sum_ab) and torch.equal(y, b)
+    y = b.clone()
+    assert torch.equal(rotate(a, y, y), sum_ab)
+    x = a.clone()
+    assert torch.equal(rotate(x, None, x), rot_a)
+    x = a.clone()
+    assert torch.equal(rotate(x, x, x), sum_aa)
