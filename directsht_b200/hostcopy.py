@@ -23,7 +23,7 @@ def _chunks(nbytes):
 
 def _buffers(count):
     n = min(_BUFFERS, count)
-    return ([torch.empty(_CHUNK, dtype=torch.uint8, pin_memory=True) for _ in range(n)],
+    return ([torch.empty(_CHUNK, dtype=torch.uint8, device="cpu", pin_memory=True) for _ in range(n)],
             [torch.cuda.Event() for _ in range(n)])
 
 
@@ -52,7 +52,7 @@ def to_host(t: torch.Tensor) -> np.ndarray:
     nbytes = t.numel() * t.element_size()
     if nbytes < _MIN_BYTES or not t.is_contiguous():
         return t.cpu().numpy()
-    out = torch.empty(t.shape, dtype=t.dtype)
+    out = torch.empty(t.shape, dtype=t.dtype, device="cpu")
     flat = (torch.view_as_real(t) if t.is_complex() else t).reshape(-1).view(torch.uint8)
     dst = (torch.view_as_real(out) if t.is_complex() else out).reshape(-1).view(torch.uint8)
     parts = _chunks(nbytes)

@@ -61,3 +61,12 @@ def test_pinned_views_are_copied_directly():
     a[:] = np.arange(a.size, dtype=np.int64) % 251
     d = to_device(a, torch.device("cuda"))
     assert torch.equal(d.cpu(), p)
+
+
+def test_other_default_device():
+    """Programs that make CUDA the default device (or float32 the default type) get the same copies."""
+    import torch
+    from directsht_b200.hostcopy import to_device, to_host
+    a = np.random.default_rng(1).normal(size=700001)
+    with torch.device("cuda"):
+        np.testing.assert_array_equal(to_host(to_device(a, "cuda")), a)
