@@ -296,9 +296,9 @@ static int build_digits(dsht_plan_s* p) {
   return DSHT_OK;
 }
 
-FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol) {
+FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol, unsigned* flags) {
   return FoldOut{ws.fold + (size_t)k * fold_stride(g.Nx) * g.Nl, ws.live + (size_t)k * ((g.Nx + 15) / 16), equ, pol,
-                 ws.tc_next};
+                 flags, ws.tc_next};
 }
 
 Geometry make_geometry(int Nl, int Nx, double xmax) {
@@ -337,16 +337,17 @@ int run_after_sort(dsht_plan_s* p, int64_t N, int mode, double* alm, const Works
     TcOut out{};
     out.equ[0] = alm;
     out.pol[0] = ws.alm_pol;
+    out.flags[0] = ws.flags;
     if (int rc = launch_contract_tc(g, p->tmDig, p->tc_items, p->tc_nitems, p->rexp, fdig, 4, ws.cexp, 1, out,
-                                    ws.flags, ws.tc_next, s))
+                                    ws.tc_next, s))
       return rc;
   } else {
     mark(DSHT_STAGE_FOLD);
     FoldIn in{};
-    in.map[0] = fold_slot(g, ws, 0, alm, ws.alm_pol);
+    in.map[0] = fold_slot(g, ws, 0, alm, ws.alm_pol, ws.flags);
     launch_fold(g, w2, in.map[0], s);
     mark(DSHT_STAGE_CONTRACT);
-    launch_contract_fp64(g, p->tmY, in, 1, ws.tc_next, ws.flags, s);
+    launch_contract_fp64(g, p->tmY, in, 1, ws.tc_next, s);
   }
   mark(DSHT_STAGE_ROTATE);
   if (mode == DSHT_MODE_CALL) {
@@ -426,6 +427,7 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
     for (size_t k = 0; k < pass.size(); ++k) {
       out.equ[k] = items[pass[k]].alm;
       out.pol[k] = ws.alm_pol + nlm2 * k;
+      out.flags[k] = ws.slot_flags + k;
       rm.rot[k] = out.pol[k];
       rm.add[k] = rm.out[k] = items[pass[k]].alm;
       rm.flags[k] = ws.slot_flags + k;
@@ -434,7 +436,7 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
     }
     prof_mark(p, DSHT_STAGE_CONTRACT, s);
     if (int rc = launch_contract_tc(g, p->tmDig, p->tc_items, p->tc_nitems, p->rexp, fdig, fcols, ws.cexp,
-                                    (int)pass.size(), out, ws.slot_flags, ws.tc_next, s))
+                                    (int)pass.size(), out, ws.tc_next, s))
       return rc;
     prof_mark(p, DSHT_STAGE_ROTATE, s);
     if (mode == DSHT_MODE_CALL) launch_rotate_back(g, rm, (int)pass.size(), rotation_tables(p->rot_tab, g.Nl), s);
@@ -462,14 +464,14 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
     if (int rc = sort_and_sum(p, item, *sorted_item >= 0, more, mode, ws, ws.slot_flags + slot, w2, s)) return rc;
     *sorted_item = i;
     prof_mark(p, DSHT_STAGE_FOLD, s);
-    in.map[nfold] = fold_slot(g, ws, nfold, item.alm, ws.alm_pol + nlm2 * slot);
+    in.map[nfold] = fold_slot(g, ws, nfold, item.alm, ws.alm_pol + nlm2 * slot, w2.flags);
     launch_fold(g, w2, in.map[nfold], s);
     ++nfold;
     pend.push_back(i);
     const bool rotate = pend.size() >= (size_t)kMaxRot || li + 1 == list.size();
     if (nfold == ws.fp64_maps || rotate) {
       prof_mark(p, DSHT_STAGE_CONTRACT, s);
-      launch_contract_fp64(g, p->tmY, in, nfold, ws.tc_next, w2.flags, s);
+      launch_contract_fp64(g, p->tmY, in, nfold, ws.tc_next, s);
       nfold = 0;
     }
     if (!rotate) continue;

@@ -117,8 +117,7 @@ struct StreamLayout {
 template <int G>
 __global__ void __launch_bounds__(kThreads, 1)
 contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_constant__ TableMaps tm,
-                     const FoldIn in, int nstage,
-                     unsigned* __restrict__ next_item, unsigned* __restrict__ err) {
+                     const FoldIn in, int nstage, unsigned* __restrict__ next_item, int stall) {
   using L = StreamLayout<G>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -142,6 +141,13 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
     *abort_flag = 0;
     tc::mbar_fence_init();
   }
+  auto timed_out = [&]() {  // the alm of every map of the pass are invalid
+    for (int k = 0; k < G; ++k) atomicOr(in.map[k].flags, kFlagTimeout);
+  };
+  auto fail = [&]() {
+    *abort_flag = 1;
+    timed_out();
+  };
   bool some = false;
   for (int t = tid; t < nstage; t += blockDim.x) {
     uint8_t any = 0;
@@ -166,7 +172,9 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
         if (item < nitems) item_of(item, Nl, &m, &g);
         else item = -1;
         item_ring[j % kItemRing] = item < 0 ? -1 : m << 8 | g;  // g < 16384 / kRows
-        tc::mbar_arrive(&item_full[j % kItemRing]);  // releases the ring entry
+        // releases the ring entry (stall, a test hook: block 0 never releases its first one, so the
+        // consumers' bounded wait runs out)
+        if (!(stall && blockIdx.x == 0 && j == 0)) tc::mbar_arrive(&item_full[j % kItemRing]);
         if (item < 0) break;
         const int l0 = m + g * kRows;
         const int row0 = (int)hp_index(l0, m, Nl);
@@ -177,8 +185,7 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
           const int s = n % kStages;
           const uint32_t use = n / kStages;
           if (use > 0 && !tc::mbar_wait(&empty[s], (use - 1) & 1, abort_flag)) {
-            *abort_flag = 1;
-            atomicOr(err, kFlagTimeout);
+            fail();
             break;
           }
           const int j0 = t * kStageNodes;
@@ -210,7 +217,7 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
         const long long t0 = clock64();
         while (!tc::mbar_try_wait_for(&full[i % kStages], (i / kStages) & 1, 10000u))
           if (clock64() - t0 > (1ll << 31)) {
-            atomicOr(err, kFlagTimeout);
+            timed_out();
             break;
           }
       }
@@ -230,8 +237,7 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
     uint32_t n = 0, iter = 0;
     for (;; ++iter) {
       if (*abort_flag || !tc::mbar_wait(&item_full[iter % kItemRing], (iter / kItemRing) & 1, abort_flag)) {
-        *abort_flag = 1;
-        if (lane == 0) atomicOr(err, kFlagTimeout);
+        if (lane == 0) fail();
         break;
       }
       const int item = item_ring[iter % kItemRing];
@@ -275,8 +281,7 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
         const uint32_t use = n / kStages;
         bool ok = !*abort_flag;
         if (ok && !tc::mbar_wait(&full[s], use & 1, abort_flag)) {
-          *abort_flag = 1;
-          atomicOr(err, kFlagTimeout);
+          fail();
           ok = false;
         }
         if (ok && on0) {
@@ -358,8 +363,7 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(ex_full);
       if (!tc::mbar_wait(ex_full, iter & 1, abort_flag)) {
-        *abort_flag = 1;
-        if (lane == 0) atomicOr(err, kFlagTimeout);
+        if (lane == 0) fail();
         break;
       }
       if (q < 2) {
@@ -424,8 +428,7 @@ int encode_table(CUtensorMap* tm, const void* base, const Geometry& g, int box_r
 }
 
 template <int G>
-void launch_g(const Geometry& g, const TableMaps& tm, const FoldIn& in, unsigned* next_item, unsigned* flags,
-              cudaStream_t s) {
+void launch_g(const Geometry& g, const TableMaps& tm, const FoldIn& in, unsigned* next_item, cudaStream_t s) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -436,7 +439,7 @@ void launch_g(const Geometry& g, const TableMaps& tm, const FoldIn& in, unsigned
   const int bytes = StreamLayout<G>::bytes(nstage);
   cudaFuncSetAttribute(contract_fp64_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   contract_fp64_kernel<G><<<(unsigned)grid, kThreads, bytes, s>>>(g.Nl, g.Nx, g.dx, nitems, tm, in, nstage,
-                                                                  next_item, flags);
+                                                                  next_item, take_stall());
   count_launches(1);
 }
 
@@ -449,12 +452,12 @@ int make_table_tmaps(TableMaps* tm, const void* base, const Geometry& g) {
 }
 
 void launch_contract_fp64(const Geometry& g, const TableMaps& tm, const FoldIn& in, int nmaps, unsigned* next_item,
-                          unsigned* flags, cudaStream_t s) {
+                          cudaStream_t s) {
   switch (nmaps) {
-    case 1: launch_g<1>(g, tm, in, next_item, flags, s); break;
-    case 2: launch_g<2>(g, tm, in, next_item, flags, s); break;
-    case 3: launch_g<3>(g, tm, in, next_item, flags, s); break;
-    default: launch_g<4>(g, tm, in, next_item, flags, s); break;
+    case 1: launch_g<1>(g, tm, in, next_item, s); break;
+    case 2: launch_g<2>(g, tm, in, next_item, s); break;
+    case 3: launch_g<3>(g, tm, in, next_item, s); break;
+    default: launch_g<4>(g, tm, in, next_item, s); break;
   }
 }
 

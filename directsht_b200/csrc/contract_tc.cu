@@ -76,8 +76,8 @@ template <int NC>
 __global__ void __launch_bounds__(kTcThreads, 1)
 contract_tc_kernel(int Nl, int nchunks, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const uint32_t* __restrict__ items, int nitems, const int16_t* __restrict__ rexp,
-                   const int16_t* __restrict__ cexp, int ncols, const TcOut out, unsigned* __restrict__ err,
-                   unsigned* __restrict__ next_item, int stall) {
+                   const int16_t* __restrict__ cexp, int ncols, const TcOut out, unsigned* __restrict__ next_item,
+                   int stall) {
   using L = TcLayout<NC>;
   constexpr int S = L::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -111,9 +111,12 @@ contract_tc_kernel(int Nl, int nchunks, const __grid_constant__ CUtensorMap tmA,
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  auto timed_out = [&]() {  // the alm of every map of the pass are invalid
+    for (int k = 0; k < ncols / 4; ++k) atomicOr(out.flags[k], kFlagTimeout);
+  };
   auto fail = [&]() {
     *abort_flag = 1;
-    atomicOr(err, kFlagTimeout);
+    timed_out();
   };
 
   if (warp == 0) {
@@ -155,7 +158,7 @@ contract_tc_kernel(int Nl, int nchunks, const __grid_constant__ CUtensorMap tmA,
         const long long t0 = clock64();
         while (!tc::mbar_try_wait_for(&full[i % S], (i / S) & 1, 10000u))
           if (clock64() - t0 > (1ll << 31)) {
-            atomicOr(err, kFlagTimeout);
+            timed_out();
             break;
           }
       }
@@ -221,7 +224,7 @@ contract_tc_kernel(int Nl, int nchunks, const __grid_constant__ CUtensorMap tmA,
       const long long t0 = clock64();
       while (!tc::mbar_try_wait_for(drain, 0, 10000u))
         if (clock64() - t0 > (1ll << 31)) {
-          atomicOr(err, kFlagTimeout);
+          timed_out();
           break;
         }
     }
@@ -284,8 +287,7 @@ contract_tc_kernel(int Nl, int nchunks, const __grid_constant__ CUtensorMap tmA,
   if (warp == 1) tc::tmem_dealloc(tmem, L::kTmemCols);
 }
 
-// Test hook (dsht_test_stall_next_contraction): the next launch leaves one wait unsatisfied.
-std::atomic<int> g_stall_next{0};
+std::atomic<bool> g_stall_next{false};
 
 PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
@@ -317,8 +319,8 @@ int make_digit_tmap(CUtensorMap* tm, const void* base, int64_t kp, int64_t rows,
 
 template <int NC>
 int tc_launch(const Geometry& g, const CUtensorMap& tmA, const uint8_t* fdig, int fdig_cols, const uint32_t* items,
-              int nitems, const int16_t* rexp, const int16_t* cexp, int ncols, const TcOut& out, unsigned* flags,
-              unsigned* next_item, cudaStream_t s) {
+              int nitems, const int16_t* rexp, const int16_t* cexp, int ncols, const TcOut& out, unsigned* next_item,
+              cudaStream_t s) {
   using L = TcLayout<NC>;
   alignas(64) CUtensorMap tmB;
   const int kp = digit_kp(g.Nx);
@@ -332,15 +334,16 @@ int tc_launch(const Geometry& g, const CUtensorMap& tmA, const uint8_t* fdig, in
   const int grid = nitems < sms ? nitems : sms;
   auto kern = contract_tc_kernel<NC>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
-  const int stall = g_stall_next.exchange(0);
   cudaMemsetAsync(next_item, 0, sizeof(unsigned), s);
-  kern<<<grid, kTcThreads, L::kBytes, s>>>(g.Nl, kp / kChunk, tmA, tmB, items, nitems, rexp, cexp, ncols, out, flags,
-                                           next_item, stall);
+  kern<<<grid, kTcThreads, L::kBytes, s>>>(g.Nl, kp / kChunk, tmA, tmB, items, nitems, rexp, cexp, ncols, out,
+                                           next_item, take_stall());
   count_launches(1);
   return DSHT_OK;
 }
 
 }  // namespace
+
+bool take_stall() { return g_stall_next.exchange(false); }
 
 int tc_fold_cols(int nmaps) { return nmaps <= 4 ? 16 : nmaps <= 8 ? 32 : 64; }
 
@@ -360,13 +363,13 @@ std::vector<uint32_t> tc_items(int Nl) {
 
 int launch_contract_tc(const Geometry& g, const CUtensorMap& tmA, const uint32_t* items, int nitems,
                        const int16_t* rexp, const uint8_t* fdig, int fdig_cols, const int16_t* cexp, int nmaps,
-                       const TcOut& out, unsigned* flags, unsigned* next_item, cudaStream_t s) {
+                       const TcOut& out, unsigned* next_item, cudaStream_t s) {
   if (nmaps < 1 || nmaps > kTcMaxMaps || 4 * nmaps > fdig_cols)
     return set_error(DSHT_ERR_INVALID, "tensor-core pass of %d maps (%d fold columns)", nmaps, fdig_cols);
   const int nc = tc_fold_cols(nmaps);
   const int ncols = 4 * nmaps;
   auto go = [&](auto launch) {
-    return launch(g, tmA, fdig, fdig_cols, items, nitems, rexp, cexp, ncols, out, flags, next_item, s);
+    return launch(g, tmA, fdig, fdig_cols, items, nitems, rexp, cexp, ncols, out, next_item, s);
   };
   if (nc == 16) return go(tc_launch<16>);
   if (nc == 32) return go(tc_launch<32>);
@@ -376,6 +379,6 @@ int launch_contract_tc(const Geometry& g, const CUtensorMap& tmA, const uint32_t
 }  // namespace dsht
 
 extern "C" int dsht_test_stall_next_contraction(void) {
-  dsht::g_stall_next.store(1);
+  dsht::g_stall_next.store(true);
   return DSHT_OK;
 }

@@ -46,13 +46,14 @@ struct Geometry {
 };
 
 // Output pointers of one tensor-core contraction pass (contract_tc.cu): map k's equatorial
-// alm to equ[k], its rotated-polar alm to pol[k] (2 Nlm doubles each).
+// alm to equ[k], its rotated-polar alm to pol[k] (2 Nlm doubles each); a wait that runs out is
+// recorded in every map's flags[k].
 constexpr int kTcMaxMaps = 8;
 struct TcOut {
   double* equ[kTcMaxMaps];
   double* pol[kTcMaxMaps];
+  unsigned* flags[kTcMaxMaps];
 };
-
 
 // One pass of the FP64 contraction: each map's fold, its equatorial and rotated polar alm.
 constexpr int kFp64Maps = 4;
@@ -67,6 +68,7 @@ struct FoldOut {
   uint8_t* live;  // [ceil(Nx/16)] any point feeds a node of the block of 16
   double* equ;    // equatorial alm, rotated polar alm
   double* pol;
+  unsigned* flags;      // the map's flag word: a wait of the contraction that runs out is recorded there
   unsigned* next_item;  // the contraction's work counter (cleared by the fold)
 };
 struct FoldIn {
@@ -139,7 +141,7 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
 // Workspace of a call of ntrans transforms of up to N points on a plan.
 size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws);
 // The fold of map k of an FP64 contraction pass and where its alm go.
-FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol);
+FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol, unsigned* flags);
 int default_piece_max(const Geometry& g, int64_t N);
 int plan_piece_max(const dsht_plan_s* p, int64_t N);
 // How a transform of N points runs on a plan: tensor-core bin sums (tc), tensor-core
@@ -196,11 +198,14 @@ int make_table_digit_tmap(CUtensorMap* tm, const uint8_t* dig, int Nx, int64_t N
 std::vector<uint32_t> tc_items(int Nl);
 int launch_contract_tc(const Geometry& g, const CUtensorMap& tmA, const uint32_t* items, int nitems,
                        const int16_t* rexp, const uint8_t* fdig, int fdig_cols, const int16_t* cexp, int nmaps,
-                       const TcOut& out, unsigned* flags, unsigned* next_item, cudaStream_t s);
+                       const TcOut& out, unsigned* next_item, cudaStream_t s);
+// Test hook (dsht_test_stall_next_contraction): whether this launch, of either contraction, is to leave one
+// wait unsatisfied.
+bool take_stall();
 
 // FP64 contraction of the Y table (contract_fp64.cu) for nmaps <= kFp64Maps folds.
 void launch_contract_fp64(const Geometry& g, const TableMaps& tm, const FoldIn& in, int nmaps, unsigned* next_item,
-                          unsigned* flags, cudaStream_t s);
+                          cudaStream_t s);
 // 2D tensor maps of an FP64 table (node x row), boxes of 16 nodes x 8 to 128 rows.
 int make_table_tmaps(TableMaps* tm, const void* base, const Geometry& g);
 // An FP64 table in the JAX path's layout out[m][l - m][j] (Nl x Nl x Nx doubles, zeros
