@@ -353,7 +353,7 @@ int run_after_sort(dsht_plan_s* p, int64_t N, int mode, double* alm, const Works
   if (mode == DSHT_MODE_CALL) {
     RotMaps rm{};
     rm.rot[0] = ws.alm_pol;
-    rm.add[0] = rm.out[0] = alm;
+    rm.out[0] = alm;
     rm.flags[0] = ws.flags;
     launch_rotate_back(g, rm, 1, rotation_tables(p->rot_tab, g.Nl), s);
   }
@@ -429,7 +429,7 @@ static int run_class_digits(dsht_plan_s* p, const Item* items, const std::vector
       out.pol[k] = ws.alm_pol + nlm2 * k;
       out.flags[k] = ws.slot_flags + k;
       rm.rot[k] = out.pol[k];
-      rm.add[k] = rm.out[k] = items[pass[k]].alm;
+      rm.out[k] = items[pass[k]].alm;
       rm.flags[k] = ws.slot_flags + k;
       so.slot[k] = ws.slot_flags + k;
       so.status[k] = items[pass[k]].status;
@@ -479,7 +479,7 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
     StatusOut so{};
     for (size_t k = 0; k < pend.size(); ++k) {
       rm.rot[k] = ws.alm_pol + nlm2 * k;
-      rm.add[k] = rm.out[k] = items[pend[k]].alm;
+      rm.out[k] = items[pend[k]].alm;
       rm.flags[k] = ws.slot_flags + k;
       so.slot[k] = ws.slot_flags + k;
       so.status[k] = items[pend[k]].status;
@@ -1022,8 +1022,9 @@ int dsht_rotate_back(dsht_plan_t p, const double* alm_rot, const double* alm_add
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   RotMaps rm{};
   rm.rot[0] = alm_rot;
-  rm.add[0] = alm_add;
   rm.out[0] = alm_out;
+  rm.add = alm_add;
+  rm.sum = true;
   launch_rotate_back(p->g, rm, 1, rotation_tables(p->rot_tab, p->g.Nl), s);
   DSHT_CUDA_OK(cudaGetLastError());
   return DSHT_OK;

@@ -77,14 +77,15 @@ struct FoldIn {
 // Doubles of one m of an FP64 fold: 16 per node, nodes in groups of eight.
 __host__ __device__ inline size_t fold_stride(int Nx) { return (size_t)((Nx + 7) / 8) * 128; }
 
-// Maps of one batched rotation: out[k] = add[k] + R(rot[k]) when *flags[k] has polar points (add null:
-// zeros).  out[k] may be add[k] or rot[k].
+// Maps of one batched rotation: out[k] += R(rot[k]) when *flags[k] has polar points; or (sum) of a lone
+// one: out[0] = add + R(rot[0]), add null for zeros, out[0] any of the others.
 constexpr int kMaxRot = 8;
 struct RotMaps {
   const double* rot[kMaxRot];
-  const double* add[kMaxRot];
   double* out[kMaxRot];
   const unsigned* flags[kMaxRot];
+  const double* add;
+  bool sum;
 };
 
 // Flag words of finished transforms: *all |= *slot[k]; status[k] (if set) = *slot[k].
@@ -222,8 +223,8 @@ struct RotTables {
 size_t rotation_table_bytes(int Nl);
 RotTables rotation_tables(void* base, int Nl);
 void launch_rotation_tables(const Geometry& g, const RotTables& t, cudaStream_t s);
-// alm out[k] = add[k] + R(rot[k]) for k < nmaps <= kMaxRot (out[k] of a map without polar points is left as
-// it is; flags null: rotate anyway).
+// alm out[k] += R(rot[k]) for k < nmaps <= kMaxRot (a map without polar points is left as it is; flags
+// null: rotate anyway), or the sum of a lone map.
 void launch_rotate_back(const Geometry& g, const RotMaps& maps, int nmaps, const RotTables& t, cudaStream_t s);
 
 // Hint: bring [p, p + bytes) into L2 (cp.async.bulk.prefetch.L2, 16-byte aligned chunks of at

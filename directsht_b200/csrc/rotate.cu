@@ -129,10 +129,10 @@ __global__ void rotation_alpha_kernel(int Nl, const double* __restrict__ sc, dou
   al[at] = k >= 1 ? sc[at] / (sqrt((double)(l + k) * (double)(l - k + 1)) * sc[at + 1]) : 0.0;
 }
 
-// Columns m = m0, m0 + blockDim, ... (C of them, one parity) of degree l: out[map] = add[map] + R(rot[map]).
+// Columns m = m0, m0 + blockDim, ... (C of them, one parity) of degree l: out[map] += R(rot[map]), or (kAdd) out = add + R(rot).
 // al: [i], S: [map][i] the coefficients of this parity's alternating real and imaginary rows, both
 // padded with zeros.
-template <int kMaps, int C>
+template <int kMaps, int C, bool kAdd>
 __device__ __forceinline__ void rotate_columns(int Nl, int l, int m0, int map0, int nm, const RotMaps& maps,
                                                const double* al, const double* S, int stride,
                                                const double* __restrict__ start, const int* __restrict__ start_e) {
@@ -198,10 +198,16 @@ __device__ __forceinline__ void rotate_columns(int Nl, int l, int m0, int map0, 
 #pragma unroll
     for (int g = 0; g < kMaps; ++g) {
       if (g < nm && (!maps.flags[map0 + g] || (*maps.flags[map0 + g] & kFlagHasPolar))) {
-        const double* add = maps.add[map0 + g];
         double* out = maps.out[map0 + g];
-        out[at] = (add ? add[at] : 0.0) + ((m & 1) ? s[j][g][1] : s[j][g][0]) * f;
-        out[at + 1] = (add ? add[at + 1] : 0.0) + ((m & 1) ? s[j][g][0] : s[j][g][1]) * f;
+        const double re = ((m & 1) ? s[j][g][1] : s[j][g][0]) * f, im = ((m & 1) ? s[j][g][0] : s[j][g][1]) * f;
+        if constexpr (kAdd) {
+          const double* add = maps.add;
+          out[at] = (add ? add[at] : 0.0) + re;
+          out[at + 1] = (add ? add[at + 1] : 0.0) + im;
+        } else {
+          out[at] += re;
+          out[at + 1] += im;
+        }
       }
     }
   }
@@ -209,7 +215,7 @@ __device__ __forceinline__ void rotate_columns(int Nl, int l, int m0, int map0, 
 
 // Maps blockIdx.y kMaps + g of degree l = Nl - 1 - blockIdx.x; a map without polar points is skipped
 // (its rotated alm are zero).  C: most columns per thread at a time.
-template <int kMaps, int C>
+template <int kMaps, int C, bool kAdd>
 __global__ void __launch_bounds__(kRotThreads)
 rotate_back_kernel(int Nl, int nmaps, const RotMaps maps, const double* __restrict__ al_t,
                    const double* __restrict__ sc_t, const double* __restrict__ start,
@@ -253,7 +259,7 @@ rotate_back_kernel(int Nl, int nmaps, const RotMaps maps, const double* __restri
     const int left = (l - first) / kRotThreads + 1;  // columns of the warp's first lane from here on
     auto run = [&](auto columns) {
       constexpr int n = decltype(columns)::value < C ? decltype(columns)::value : C;
-      rotate_columns<kMaps, n>(Nl, l, m0, map0, nm, maps, al, Sp, pad, start, start_e);
+      rotate_columns<kMaps, n, kAdd>(Nl, l, m0, map0, nm, maps, al, Sp, pad, start, start_e);
     };
     switch (min(left, C)) {
       case 1: run(std::integral_constant<int, 1>{}); break;
@@ -264,12 +270,12 @@ rotate_back_kernel(int Nl, int nmaps, const RotMaps maps, const double* __restri
   }
 }
 
-template <int kMaps, int C>
+template <int kMaps, int C, bool kAdd = false>
 void rotate_launch(const Geometry& g, const RotMaps& maps, int nmaps, const RotTables& t, cudaStream_t s) {
   const size_t smem = sizeof(double) * (size_t)(((g.Nl + 3) & ~3) + 2) * (1 + 2 * kMaps);
-  cudaFuncSetAttribute(rotate_back_kernel<kMaps, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(rotate_back_kernel<kMaps, C, kAdd>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   dim3 grid(g.Nl, (nmaps + kMaps - 1) / kMaps);
-  rotate_back_kernel<kMaps, C><<<grid, kRotThreads, smem, s>>>(g.Nl, nmaps, maps, t.al, t.sc, t.start, t.start_e);
+  rotate_back_kernel<kMaps, C, kAdd><<<grid, kRotThreads, smem, s>>>(g.Nl, nmaps, maps, t.al, t.sc, t.start, t.start_e);
   count_launches(1);
 }
 
@@ -296,7 +302,8 @@ void launch_rotate_back(const Geometry& g, const RotMaps& maps, int nmaps, const
   // maps with two columns 694 (registers: fewer CTAs per SM).
   auto bytes = [&](int k) { return sizeof(double) * (size_t)(((g.Nl + 3) & ~3) + 2) * (1 + 2 * k); };
   const size_t lim = 227 * 1024;
-  if (nmaps > 2 && bytes(4) <= lim) rotate_launch<4, 3>(g, maps, nmaps, t, s);
+  if (maps.sum) rotate_launch<1, 4, true>(g, maps, 1, t, s);
+  else if (nmaps > 2 && bytes(4) <= lim) rotate_launch<4, 3>(g, maps, nmaps, t, s);
   else if (nmaps == 2 && bytes(2) <= lim) rotate_launch<2, 2>(g, maps, nmaps, t, s);
   else rotate_launch<1, 4>(g, maps, nmaps, t, s);
 }
