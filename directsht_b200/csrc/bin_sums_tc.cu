@@ -238,7 +238,8 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
     // half 1 (the heavier) on warps 6-7, i.e. sub-partitions 2-3, where no B slicer warp runs
     const int p = (tid - kSlicers) & 63, half = ((tid - kSlicers) >> 6) ^ 1;
     uint32_t g = 0;
-    for (int piece = blockIdx.x; piece < npieces && !*abort_flag; piece += gridDim.x) {
+    bool ok = true;  // (after a wait that ran out the warps go on without waiting, to stay whole)
+    for (int piece = blockIdx.x; piece < npieces; piece += gridDim.x) {
       const int64_t start = piece_start[piece];
       const int len = piece_len[piece];
       const int nblk = (len + kBK - 1) / kBK;
@@ -266,9 +267,9 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
         t0 = t1;
         if (b + 2 < nblk) load(b + 2, c1, s1, w1, t1);
         const int buf = g & 1;
-        if (g >= 2 && !tc::mbar_wait(&aempty[buf], ((g >> 1) - 1) & 1, abort_flag)) {
+        if (ok && g >= 2 && !tc::mbar_wait(&aempty[buf], ((g >> 1) - 1) & 1, abort_flag)) {
           fail();
-          break;
+          ok = false;
         }
         int4* eb = reinterpret_cast<int4*>(eb_of(buf) + p * kEbStride);  // pairs of c
         float2* ea = ea_of(buf);
@@ -491,11 +492,8 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
       // (through the bit pattern of 1.5 2^52: no conversion-pipe instruction).
       const double fs = tc_scale(piecemax[piece]) * kKScale[k] / (kQ * kQ) * 256.0;
       float* out = partial + ((size_t)piece * 8 + 2 * k + ri) * Nl;
-      bool ok = !*abort_flag;
-      if (ok && !tc::mbar_wait(done, piece_iter & 1, abort_flag)) {
-        fail();
-        ok = false;
-      }
+      const bool ok = tc::warp_wait(done, piece_iter & 1, abort_flag);
+      if (!ok && lane == 0) fail();
       tc::tc_fence_after();
 #pragma unroll 1
       for (int cb = 8 * set; cb < CH; cb += 8 * kEpiSets) {

@@ -236,7 +236,7 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
     row[1] = row[0] + 64;
     uint32_t n = 0, iter = 0;
     for (;; ++iter) {
-      if (*abort_flag || !tc::mbar_wait(&item_full[iter % kItemRing], (iter / kItemRing) & 1, abort_flag)) {
+      if (!tc::warp_wait(&item_full[iter % kItemRing], (iter / kItemRing) & 1, abort_flag)) {
         if (lane == 0) fail();
         break;
       }
@@ -279,11 +279,8 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
         if (!live[t]) continue;
         const int s = n % kStages;
         const uint32_t use = n / kStages;
-        bool ok = !*abort_flag;
-        if (ok && !tc::mbar_wait(&full[s], use & 1, abort_flag)) {
-          fail();
-          ok = false;
-        }
+        const bool ok = tc::warp_wait(&full[s], use & 1, abort_flag);
+        if (!ok && lane == 0) fail();
         if (ok && on0) {
           const uint8_t* st = smem + s * L::kStage;
           const int ng = min(kStageNodes / 8, (Nx - t * kStageNodes + 7) / 8);
@@ -362,7 +359,7 @@ contract_fp64_kernel(int Nl, int Nx, double dx, int64_t nitems, const __grid_con
       // every consumer warp has written (a bounded wait: a warp that gave up never arrives)
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(ex_full);
-      if (!tc::mbar_wait(ex_full, iter & 1, abort_flag)) {
+      if (!tc::warp_wait(ex_full, iter & 1, abort_flag)) {
         if (lane == 0) fail();
         break;
       }

@@ -233,7 +233,7 @@ contract_tc_kernel(int Nl, int nchunks, const __grid_constant__ CUtensorMap tmA,
     // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 -----------------------------
     const int q = warp & 3;
     for (uint32_t iter = 0;; ++iter) {
-      if (*abort_flag || !tc::mbar_wait(&item_full[iter % kItemRing], (iter / kItemRing) & 1, abort_flag)) {
+      if (!tc::warp_wait(&item_full[iter % kItemRing], (iter / kItemRing) & 1, abort_flag)) {
         if (lane == 0) fail();
         break;
       }
@@ -241,7 +241,7 @@ contract_tc_kernel(int Nl, int nchunks, const __grid_constant__ CUtensorMap tmA,
       if (it < 0) break;
       const uint32_t b = L::kBufs == 2 ? (iter & 1) : 0;
       const uint32_t use_b = L::kBufs == 2 ? (iter >> 1) : iter;
-      if (*abort_flag || !tc::mbar_wait(&tfull[b], use_b & 1, abort_flag)) {
+      if (!tc::warp_wait(&tfull[b], use_b & 1, abort_flag)) {
         if (lane == 0) fail();
         break;
       }

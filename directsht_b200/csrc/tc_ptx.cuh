@@ -64,6 +64,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+// The same for a whole warp: true for all its lanes or for none, so that what the warp does together --
+// mma.sync, tcgen05.ld, shuffles, __syncwarp -- may depend on it.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const volatile int* abort) {
+  if (__all_sync(0xffffffffu, mbar_try_wait_for(bar, parity, 10000u))) return true;
+  return __all_sync(0xffffffffu, !*abort && mbar_wait(bar, parity, abort));
+}
+
 // Make this thread's generic-proxy shared-memory writes visible to the async proxy
 // (tcgen05.mma reads its operands through it).
 __device__ __forceinline__ void fence_async_smem() {
