@@ -62,8 +62,16 @@ int default_piece_max(const Geometry& g, int64_t N) {
   return (int)p;
 }
 
+// Most pieces, beyond one per key, that the direct sums of a transform of at most n points have: pieces of
+// piece_max points, or of default_piece_max(N) (N / 256 of them up to 2048, then N / 2048).
+static int64_t direct_pieces(int64_t n, int piece_max) {
+  const int64_t least = (n + 2047) / 2048;
+  if (piece_max > 0) return std::max<int64_t>(least, (n + piece_max - 1) / piece_max);
+  return std::max(least, std::min<int64_t>(2048, (n + 255) / 256));
+}
+
 size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws, bool multi,
-                        int tc_maps, int fp64_maps, int nu_grid) {
+                        int tc_maps, int fp64_maps, int nu_grid, int64_t direct_extra) {
   size_t off = 0;
   auto take = [&](size_t bytes) -> uint8_t* {
     uint8_t* p = base ? base + off : nullptr;
@@ -71,16 +79,9 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
     return p;
   };
   const int64_t n = N > 0 ? N : 1;
-  // Pieces of a transform of up to n points.  A workspace laid out for the NUFFT sums' large
-  // pieces also serves smaller transforms (of a batch, or of later calls), which may take the direct
-  // sums, with N below the NUFFT threshold: their pieces of default_piece_max(N) number at
-  // most min(2048, N / 256) or N / 2048 beyond one per key.
-  int64_t extra = (n + piece_max - 1) / piece_max;
-  if (nu_grid) {
-    const int64_t direct_n = std::min<int64_t>(n, (int64_t)kNufftMinPerKey * g.nkeys);
-    extra = std::max(extra, std::min<int64_t>(2048, (direct_n + 255) / 256));
-    extra = std::max<int64_t>(extra, (direct_n + 2047) / 2048);
-  }
+  // Pieces of a transform of up to n points: of this size, and those of the smaller transforms that
+  // the workspace also serves (of a batch, or of later calls) on the direct sums.
+  const int64_t extra = std::max<int64_t>((n + piece_max - 1) / piece_max, direct_extra);
   const int64_t pmax = std::min<int64_t>(g.nkeys, n) + extra;
   Workspace w{};
   w.key = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * n));
@@ -134,6 +135,26 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
   return off;
 }
 
+// Fewest points of a transform that takes the NUFFT sums on this plan; the one rule for the choice of the
+// sums and for the sizes of workspaces.
+static int64_t plan_nufft_from(const dsht_plan_s* p) {
+  constexpr int64_t never = INT64_MAX;
+  const bool mixed = p->precision != DSHT_PREC_FP64;
+  const int t = p->tune_bin_sums, cls = mixed ? kNuMixed : kNuFp64;
+  if (!p->nu_tab[cls] || t == DSHT_BIN_SUMS_FP64) return never;
+  if (mixed) {
+    // A NUFFT node pays a fixed FFT and little per point (plan_bin_method).
+    if (t == DSHT_BIN_SUMS_TC) return never;
+    return std::max<int64_t>(DSHT_MIXED_MIN_POINTS,
+                             t == DSHT_BIN_SUMS_NUFFT ? 0 : (int64_t)kNufftMinPerKey * p->g.nkeys);
+  }
+  if (t == DSHT_BIN_SUMS_NUFFT) return 0;
+  // The direct sums cost Nl per point, a node's transform n log n: measured (full sky) equal at 45
+  // points per key for n = 4 Nl, 60-73 for n = 7 Nl, 65-110 for n = 8 Nl.
+  const int64_t n = (int64_t)1 << nufft_logn(p->g.Nl, kNuFp64);
+  return (11 * n * p->g.nkeys + p->g.Nl - 1) / p->g.Nl;
+}
+
 // The mixed levels' bin-sum method for one transform of N points (chosen per transform, so
 // the transforms of one batch call may differ).  AUTO compares the average points per bin
 // key with two measured crossovers: a NUFFT node pays a fixed FFT and little per point, so it wins
@@ -144,21 +165,15 @@ size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* ba
 int plan_bin_method(const dsht_plan_s* p, int64_t N) {
   const int t = p->tune_bin_sums;
   if (t == DSHT_BIN_SUMS_FP64 || t == DSHT_BIN_SUMS_TC) return t;
-  if (p->nu_tab[kNuMixed] && (t == DSHT_BIN_SUMS_NUFFT || N >= (int64_t)kNufftMinPerKey * p->g.nkeys))
-    return DSHT_BIN_SUMS_NUFFT;
+  if (N >= plan_nufft_from(p)) return DSHT_BIN_SUMS_NUFFT;
   if (t == DSHT_BIN_SUMS_AUTO && N < (int64_t)kFp64MaxPerKey * p->g.nkeys) return DSHT_BIN_SUMS_FP64;
   return DSHT_BIN_SUMS_TC;
 }
 
 // Accuracy class of a transform's NUFFT sums, -1 for the direct sums.
 int plan_nufft_class(const dsht_plan_s* p, int64_t N) {
-  if (plan_route(p, N).tc) return plan_bin_method(p, N) == DSHT_BIN_SUMS_NUFFT ? kNuMixed : -1;
-  if (p->precision != DSHT_PREC_FP64 || !p->nu_tab[kNuFp64] || p->tune_bin_sums == DSHT_BIN_SUMS_FP64) return -1;
-  if (p->tune_bin_sums == DSHT_BIN_SUMS_NUFFT) return kNuFp64;
-  // The direct sums cost Nl per point, a node's transform n log n: measured (full sky) equal at 45
-  // points per key for n = 4 Nl, 60-73 for n = 7 Nl, 65-110 for n = 8 Nl.
-  const int64_t n = (int64_t)1 << nufft_logn(p->g.Nl, kNuFp64);
-  return (double)N * p->g.Nl >= 11.0 * (double)n * p->g.nkeys ? kNuFp64 : -1;
+  if (N < plan_nufft_from(p)) return -1;
+  return p->precision == DSHT_PREC_FP64 ? kNuFp64 : kNuMixed;
 }
 
 // Pieces of the direct sums stay at or below 2048 points (the tensor path's S32 sums stay
@@ -577,8 +592,12 @@ size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* b
   // maps per tensor-core contraction pass (digit tables): up to kTcMaxMaps unless tuned
   const int tc = multi ? std::min(std::max(ntrans, 1), p->tune_maps_per_pass > 0 ? p->tune_maps_per_pass
                                                                                   : kTcMaxMaps) : 1;
+  const int64_t direct_n = std::min<int64_t>(N, std::max<int64_t>(plan_nufft_from(p), 1) - 1);
+  const int direct_piece = p->tune_piece_max > 0 ? std::min(p->tune_piece_max, 2048) : 0;
+  // a batch's smaller transforms, or smaller later calls where this one takes the NUFFT sums
+  const int64_t cover = multi || direct_n < N ? direct_pieces(direct_n, direct_piece) : 0;
   return workspace_layout(p->g, N, plan_piece_max(p, N), base, ws, multi, tc, std::min(tc, kFp64Maps),
-                          plan_nufft_grid(p, N));
+                          plan_nufft_grid(p, N), cover);
 }
 
 }  // namespace dsht
@@ -922,6 +941,26 @@ int dsht_test_point_keys(dsht_plan_t p, const double* theta, const double* phi, 
   DSHT_CUDA_OK(cudaMemcpyAsync(flags, ws.flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
   DSHT_CUDA_OK(cudaStreamSynchronize(s));
   DSHT_CUDA_OK(cudaGetLastError());
+  return DSHT_OK;
+}
+
+int dsht_test_layout(int Nl, int Nx, int precision, int bin_sums, int piece_max, int64_t N, int ntrans, int64_t n,
+                     int64_t* out) {
+  if (Nl < 1 || Nx < 2 || N < 1 || ntrans < 0 || n < 1 || n > N || !out)
+    return set_error(DSHT_ERR_INVALID, "invalid arguments");
+  dsht_plan_s p;  // never launched: the tables only have to be there
+  double there = 0.0;
+  p.g = make_geometry(Nl, Nx, 0.75);
+  p.precision = precision;
+  p.tune_bin_sums = bin_sums;
+  p.tune_piece_max = piece_max;
+  if (Nl <= 2048) p.nu_tab[0] = p.nu_tab[1] = &there;
+  Workspace ws;
+  out[0] = out[1] = (int64_t)call_layout(&p, N, std::max(ntrans, 1), ntrans > 0, nullptr, &ws);
+  out[2] = ws.pmax;
+  out[3] = plan_nufft_class(&p, n);
+  out[4] = plan_piece_max(&p, n);
+  out[5] = plan_nufft_grid(&p, n);
   return DSHT_OK;
 }
 

@@ -136,9 +136,10 @@ struct Workspace {
 
 // multi: add the records of multi-transform calls (gather indices, rotation and flag slots);
 // tc_maps: maps one tensor-core contraction pass holds (fold digit columns), fp64_maps: maps one
-// FP64 contraction pass holds; nu_grid: CTAs of the NUFFT sums (0: none).
-size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws,
-                        bool multi = false, int tc_maps = 1, int fp64_maps = 1, int nu_grid = 0);
+// FP64 contraction pass holds; nu_grid: CTAs of the NUFFT sums (0: none); direct_extra: pieces beyond
+// one per key that smaller transforms on the same workspace may have.
+size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws, bool multi,
+                        int tc_maps, int fp64_maps, int nu_grid, int64_t direct_extra);
 // Workspace of a call of ntrans transforms of up to N points on a plan.
 size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws);
 // The fold of map k of an FP64 contraction pass and where its alm go.

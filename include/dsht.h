@@ -301,6 +301,15 @@ int dsht_profile_read(dsht_plan_t plan, double* ms, int64_t* calls, int reset);
  * shared the launch.  Lets a test check that a stalled pipeline is reported instead of hanging. */
 int dsht_test_stall_next_contraction(void);
 
+/* Test hook, no counterpart in the reference: how a workspace is laid out, without a device.  For a plan
+ * (Nl, Nx) at a precision level with the tuned bin_sums and piece_max (0: automatic), out[0] = bytes of
+ * the workspace for N points (ntrans = 0: dsht_workspace_size; > 0: dsht_workspace_size_batch of that many
+ * transforms), out[1] = bytes that a call of N points asks for, out[2] = bin pieces that call has room
+ * for; and for a transform of n <= N points on it out[3] = class of its NUFFT sums (-1: direct sums),
+ * out[4] = points per piece, out[5] = CTAs of the NUFFT sums. */
+int dsht_test_layout(int Nl, int Nx, int precision, int bin_sums, int piece_max, int64_t N, int ntrans, int64_t n,
+                     int64_t* out);
+
 /* Test hook, no counterpart in the reference: the sort key of every point as the transform
  * computes it (DEVICE pointers; keys[N] uint32, flags one unsigned), so tests can check the
  * binning index for index.  key = set * (Nx - 1) + bin with set 0/1 for equatorial points
