@@ -55,7 +55,7 @@ static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // Points per bin piece: at most 2048 (the S32 sums of the tensor path stay exact), at
 // least 256, and about N/2048 in between.  Smaller pieces keep the fixed-point scale of
 // the tensor path (the piece's largest |w h_k|) closer to its typical weight.
-int default_piece_max(const Geometry& g, int64_t N) {
+static int default_piece_max(int64_t N) {
   int64_t p = (N + 2047) / 2048;
   if (p < 256) p = 256;
   if (p > 2048) p = 2048;
@@ -70,78 +70,88 @@ static int64_t direct_pieces(int64_t n, int piece_max) {
   return std::max(least, std::min<int64_t>(2048, (n + 255) / 256));
 }
 
-size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws, bool multi,
-                        int tc_maps, int fp64_maps, int nu_grid, int64_t direct_extra) {
+// What a workspace has room for.
+struct LayoutSpec {
+  int64_t n;        // points
+  int64_t pieces;   // pieces of the lists
+  int piece_max;
+  int nu_grid;      // CTAs of the NUFFT sums (0: none)
+  bool piece_sums;  // sums per piece (direct sums) besides the sums per node slot of the NUFFT
+  bool maxima;      // the pieces' largest |w h_k|
+  bool wsums;       // the pieces' sums of |w|
+  bool multi;       // gather indices, rotation and flag slots of multi-transform calls
+  int tc_maps;      // maps of a tensor-core contraction pass (fold digit columns; 0: none)
+  int fp64_maps;    // maps of an FP64 contraction pass (0: none)
+};
+
+static size_t workspace_layout(const Geometry& g, const LayoutSpec& spec, uint8_t* base, Workspace* ws) {
   size_t off = 0;
   auto take = [&](size_t bytes) -> uint8_t* {
     uint8_t* p = base ? base + off : nullptr;
     off = align_up(off + bytes, 256);
     return p;
   };
-  const int64_t n = N > 0 ? N : 1;
-  // Pieces of a transform of up to n points: of this size, and those of the smaller transforms that
-  // the workspace also serves (of a batch, or of later calls) on the direct sums.
-  const int64_t extra = std::max<int64_t>((n + piece_max - 1) / piece_max, direct_extra);
-  const int64_t pmax = std::min<int64_t>(g.nkeys, n) + extra;
+  const int64_t n = spec.n, pmax = spec.pieces;
   Workspace w{};
   w.key = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * n));
   w.pay = reinterpret_cast<double*>(take(sizeof(double) * kRec * n));
-  const bool maps = multi;
-  if (maps) {
-    w.sidx = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * n));
-  }
+  if (spec.multi) w.sidx = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * n));
   w.count = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
   w.flags = base ? w.count + g.nkeys : nullptr;  // cleared with the counts
   w.offset = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
-  w.cursor = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
+  if (spec.multi) w.cursor = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
   w.piece_first = reinterpret_cast<int*>(take(sizeof(int) * (g.nkeys + 1)));
   w.piece_key = reinterpret_cast<int*>(take(sizeof(int) * pmax));
   w.piece_start = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * pmax));
   w.piece_len = reinterpret_cast<int*>(take(sizeof(int) * pmax));
-  w.piecemax = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * pmax));
-  w.wsum = reinterpret_cast<double*>(take(sizeof(double) * pmax));
+  if (spec.maxima || spec.nu_grid) w.piecemax = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * pmax));
+  if (spec.wsums) w.wsum = reinterpret_cast<double*>(take(sizeof(double) * pmax));
   w.npieces = reinterpret_cast<int*>(take(sizeof(int)));
-  if (maps) {
+  if (spec.multi) {
     w.slot_flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * kMaxRot));
     w.all_flags = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
   }
-  size_t sums = 8 * (size_t)pmax;
-  if (nu_grid) {
-    w.piece_cta = reinterpret_cast<int*>(take(sizeof(int) * pmax));
-    w.cta_first = reinterpret_cast<int*>(take(sizeof(int) * (nu_grid + 1)));
+  size_t sums = spec.piece_sums ? 8 * (size_t)pmax : 0;
+  if (spec.nu_grid) {
+    w.piece_cta = reinterpret_cast<int*>(w.piecemax);  // a transform uses one of the two
+    w.cta_first = reinterpret_cast<int*>(take(sizeof(int) * (spec.nu_grid + 1)));
     w.node_first = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (g.nkeys + 1)));
     // a slot per node with points, two more per CTA
     const int64_t nodes = std::min<int64_t>(2 * std::min<int64_t>(g.nkeys, n), g.nkeys + kSets);
-    sums = std::max<size_t>(sums, 4 * (size_t)(nodes + 2 * nu_grid));
+    sums = std::max<size_t>(sums, 4 * (size_t)(nodes + 2 * spec.nu_grid));
   }
   w.partial = reinterpret_cast<double*>(take(sizeof(double) * (size_t)g.Nl * sums));
   // The FP64 folds of a contraction pass, or the tensor-core route's fold digits ([Nl][2][4][4 tc_maps]
-  // [Kp] int8), whichever is larger: a call's route uses one of them.
-  w.tc_maps = std::max(1, std::min(tc_maps, kTcMaxMaps));
-  const size_t fold_bytes = sizeof(double) * fold_stride(g.Nx) * (size_t)g.Nl * fp64_maps;
-  const size_t fdig_bytes = (size_t)g.Nl * 8 * 4 * w.tc_maps * (size_t)digit_kp(g.Nx);
+  // [Kp] int8), whichever is larger: a pass uses one of them.
+  const size_t fold_bytes = sizeof(double) * fold_stride(g.Nx) * (size_t)g.Nl * spec.fp64_maps;
+  const size_t fdig_bytes = (size_t)g.Nl * 8 * 4 * spec.tc_maps * (size_t)digit_kp(g.Nx);
   w.fold = reinterpret_cast<double*>(take(std::max(fold_bytes, fdig_bytes)));
-  w.fp64_maps = fp64_maps;
-  w.live = take((size_t)fp64_maps * ((g.Nx + 15) / 16));
-  w.cexp = reinterpret_cast<int16_t*>(take(sizeof(int16_t) * 2 * w.tc_maps));
-  w.cmax = reinterpret_cast<unsigned long long*>(take(sizeof(unsigned long long) * 2 * w.tc_maps));
+  // a single transform's sort is done before its fold is written (fold: at least 64 bytes per node)
+  if (!spec.multi) w.cursor = reinterpret_cast<uint32_t*>(w.fold);
+  w.tc_maps = spec.tc_maps;
+  w.fp64_maps = spec.fp64_maps;
+  if (spec.fp64_maps) w.live = take((size_t)spec.fp64_maps * ((g.Nx + 15) / 16));
+  if (spec.tc_maps) {
+    w.cexp = reinterpret_cast<int16_t*>(take(sizeof(int16_t) * 2 * spec.tc_maps));
+    w.cmax = reinterpret_cast<unsigned long long*>(take(sizeof(unsigned long long) * 2 * spec.tc_maps));
+  }
   w.tc_next = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
-  w.alm_pol = reinterpret_cast<double*>(take(sizeof(double) * 2 * (size_t)g.Nlm * (maps ? kMaxRot : 1)));
+  w.alm_pol = reinterpret_cast<double*>(take(sizeof(double) * 2 * (size_t)g.Nlm * (spec.multi ? kMaxRot : 1)));
   w.npts = n;
   w.pmax = pmax;
-  w.piece_max = piece_max;
+  w.piece_max = spec.piece_max;
   w.bytes = off;
   if (ws) *ws = w;
   return off;
 }
 
-// Fewest points of a transform that takes the NUFFT sums on this plan; the one rule for the choice of the
-// sums and for the sizes of workspaces.
-static int64_t plan_nufft_from(const dsht_plan_s* p) {
+// Fewest points of a transform that takes the NUFFT sums on this plan at a precision level; the one rule
+// for the choice of the sums and for the sizes of workspaces.
+static int64_t plan_nufft_from(const dsht_plan_s* p, int level) {
   constexpr int64_t never = INT64_MAX;
-  const bool mixed = p->precision != DSHT_PREC_FP64;
-  const int t = p->tune_bin_sums, cls = mixed ? kNuMixed : kNuFp64;
-  if (!p->nu_tab[cls] || t == DSHT_BIN_SUMS_FP64) return never;
+  const bool mixed = level != DSHT_PREC_FP64;
+  const int t = p->tune_bin_sums;
+  if (p->g.Nl > 2048 || t == DSHT_BIN_SUMS_FP64) return never;
   if (mixed) {
     // A NUFFT node pays a fixed FFT and little per point (plan_bin_method).
     if (t == DSHT_BIN_SUMS_TC) return never;
@@ -162,46 +172,46 @@ static int64_t plan_nufft_from(const dsht_plan_s* p) {
 // piece and 0.2-0.3 ns per point (device-wide), the FP64 direct sums little per piece and 1-2 ns
 // per point, so below kFp64MaxPerKey points per key (pieces of a few points) the FP64 sums are the
 // fastest.  (The tensor-core sums quantise, so the NUFFT threshold also decides the accuracy.)
-int plan_bin_method(const dsht_plan_s* p, int64_t N) {
+static int plan_bin_method(const dsht_plan_s* p, int64_t N, int level) {
   const int t = p->tune_bin_sums;
   if (t == DSHT_BIN_SUMS_FP64 || t == DSHT_BIN_SUMS_TC) return t;
-  if (N >= plan_nufft_from(p)) return DSHT_BIN_SUMS_NUFFT;
+  if (N >= plan_nufft_from(p, level)) return DSHT_BIN_SUMS_NUFFT;
   if (t == DSHT_BIN_SUMS_AUTO && N < (int64_t)kFp64MaxPerKey * p->g.nkeys) return DSHT_BIN_SUMS_FP64;
   return DSHT_BIN_SUMS_TC;
 }
 
 // Accuracy class of a transform's NUFFT sums, -1 for the direct sums.
-int plan_nufft_class(const dsht_plan_s* p, int64_t N) {
-  if (N < plan_nufft_from(p)) return -1;
-  return p->precision == DSHT_PREC_FP64 ? kNuFp64 : kNuMixed;
+static int plan_nufft_class(const dsht_plan_s* p, int64_t N, int level) {
+  if (N < plan_nufft_from(p, level)) return -1;
+  return level == DSHT_PREC_FP64 ? kNuFp64 : kNuMixed;
 }
 
 // Pieces of the direct sums stay at or below 2048 points (the tensor path's S32 sums stay
 // exact); the NUFFT sums' at or below what their sort holds.
-int plan_piece_max(const dsht_plan_s* p, int64_t N) {
-  const int cls = plan_nufft_class(p, N);
+static int plan_piece_max(const dsht_plan_s* p, int64_t N, int level) {
+  const int cls = plan_nufft_class(p, N, level);
   if (cls >= 0) {
     const int most = nufft_piece(p->g.Nl, cls);
     return p->tune_piece_max > 0 ? std::min(p->tune_piece_max, most) : most;
   }
-  const int pm = p->tune_piece_max > 0 ? p->tune_piece_max : default_piece_max(p->g, N);
+  const int pm = p->tune_piece_max > 0 ? p->tune_piece_max : default_piece_max(N);
   return std::min(pm, 2048);
 }
 
 // CTAs of the NUFFT sums of N points, 0 for the direct sums: no more than there can be pieces.
-int plan_nufft_grid(const dsht_plan_s* p, int64_t N) {
-  const int cls = plan_nufft_class(p, N);
+static int plan_nufft_grid(const dsht_plan_s* p, int64_t N, int level) {
+  const int cls = plan_nufft_class(p, N, level);
   if (cls < 0) return 0;
-  const int64_t pm = plan_piece_max(p, N);
+  const int64_t pm = plan_piece_max(p, N, level);
   const int64_t pieces = std::min<int64_t>(p->g.nkeys, N) + (N + pm - 1) / pm;
   return (int)std::max<int64_t>(1, std::min<int64_t>(nufft_grid(p->g.Nl, cls), pieces));
 }
 
 // Sets the workspace for a transform of N points: its piece size and its NUFFT run, if any.
 void route_workspace(const dsht_plan_s* p, int64_t N, Workspace& w) {
-  const int cls = plan_nufft_class(p, N);
-  w.piece_max = plan_piece_max(p, N);
-  w.nu_grid = plan_nufft_grid(p, N);
+  const int cls = plan_nufft_class(p, N, p->precision);
+  w.piece_max = plan_piece_max(p, N, p->precision);
+  w.nu_grid = plan_nufft_grid(p, N, p->precision);
   w.nu_piece_cost = cls >= 0 ? nufft_piece_cost(p->g.Nl, cls) : 0;
 }
 
@@ -211,15 +221,15 @@ int launch_bin_sums(const dsht_plan_s* p, Workspace& w, int64_t N, cudaStream_t 
   const Route rt = plan_route(p, N);
   w.partial_f32 = 0;
   if (w.nu_grid) {
-    const int cls = plan_nufft_class(p, N);
+    const int cls = plan_nufft_class(p, N, p->precision);
     const NufftTables t{cls, p->nu_tab[cls], p->nu_tab[cls] + p->g.Nl + (p->g.Nl & 1)};
     return launch_bin_sums_nufft(p->g, w, t, s);
   }
-  if (rt.tc && plan_bin_method(p, N) == DSHT_BIN_SUMS_TC) {
+  if (rt.tc && plan_bin_method(p, N, p->precision) == DSHT_BIN_SUMS_TC) {
     w.partial_f32 = 1;
     return launch_bin_sums_tc(p->g, w, s);  // piece maxima and |w| sums first
   }
-  if (rt.tc || rt.digits) launch_piece_maxima(w, s);  // the |w| sums (fold digit scales)
+  if (rt.digits) launch_piece_maxima(w, s);  // the |w| sums (fold digit scales)
   launch_bin_sums_fp64(p->g, w, s);
   return DSHT_OK;
 }
@@ -236,14 +246,15 @@ static int build_nufft(dsht_plan_s* p, int cls) {
   return DSHT_OK;
 }
 
-Route plan_route(const dsht_plan_s* p, int64_t N) {
+static Route level_route(const dsht_plan_s* p, int64_t N, int level, bool digit_tables) {
   Route r{};
-  r.tc = p->precision != DSHT_PREC_FP64 && N >= DSHT_MIXED_MIN_POINTS;
+  r.tc = level != DSHT_PREC_FP64 && N >= DSHT_MIXED_MIN_POINTS;
   // The digit tables serve tensor-core transforms at the MIXED level and every transform
   // of a plan that holds no FP64 tables; everything else contracts the FP64 tables.
-  r.digits = p->tmdig && ((r.tc && p->precision == DSHT_PREC_MIXED) || !p->Yv);
+  r.digits = digit_tables && ((r.tc && level == DSHT_PREC_MIXED) || !p->Yv);
   return r;
 }
+Route plan_route(const dsht_plan_s* p, int64_t N) { return level_route(p, N, p->precision, p->tmdig); }
 
 // Builds the digit tables of rows [row0, row0 + nrows) from FP64 tables (Healpy order)
 // held at Yv, Yd for exactly those rows.
@@ -586,18 +597,62 @@ static int ensure_plan_workspace(dsht_plan_s* p, size_t bytes) {
   return DSHT_OK;
 }
 
-// Workspace of a call: single transforms use the lean layout; multi-transform calls add
-// the gather records, fold digit columns of a contraction pass, rotation and flag slots.
-size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws) {
-  // maps per tensor-core contraction pass (digit tables): up to kTcMaxMaps unless tuned
-  const int tc = multi ? std::min(std::max(ntrans, 1), p->tune_maps_per_pass > 0 ? p->tune_maps_per_pass
-                                                                                  : kTcMaxMaps) : 1;
-  const int64_t direct_n = std::min<int64_t>(N, std::max<int64_t>(plan_nufft_from(p), 1) - 1);
+// Room that one transform of N points needs at a level.
+static LayoutSpec single_spec(const dsht_plan_s* p, int64_t N, int level, bool digit_tables) {
+  const Route rt = level_route(p, N, level, digit_tables);
+  LayoutSpec s{};
+  s.n = std::max<int64_t>(N, 1);
+  s.piece_max = plan_piece_max(p, N, level);
+  s.pieces = std::min<int64_t>(p->g.nkeys, s.n) + (s.n + s.piece_max - 1) / s.piece_max;
+  s.nu_grid = plan_nufft_grid(p, N, level);
+  s.piece_sums = s.nu_grid == 0;
+  s.maxima = s.piece_sums && (rt.digits || (rt.tc && plan_bin_method(p, N, level) == DSHT_BIN_SUMS_TC));
+  s.wsums = rt.digits;
+  s.tc_maps = rt.digits ? 1 : 0;
+  s.fp64_maps = rt.digits ? 0 : 1;
+  return s;
+}
+
+// Room for ntrans transforms of up to N points each: every smaller one may take the direct sums, in smaller
+// pieces; digit tables or not.
+static LayoutSpec multi_spec(const dsht_plan_s* p, int64_t N, int ntrans, int level) {
+  LayoutSpec s = single_spec(p, N, level, false);
+  const int64_t direct_n = std::min<int64_t>(N, std::max<int64_t>(plan_nufft_from(p, level), 1) - 1);
   const int direct_piece = p->tune_piece_max > 0 ? std::min(p->tune_piece_max, 2048) : 0;
-  // a batch's smaller transforms, or smaller later calls where this one takes the NUFFT sums
-  const int64_t cover = multi || direct_n < N ? direct_pieces(direct_n, direct_piece) : 0;
-  return workspace_layout(p->g, N, plan_piece_max(p, N), base, ws, multi, tc, std::min(tc, kFp64Maps),
-                          plan_nufft_grid(p, N), cover);
+  s.pieces = std::max(s.pieces, std::min<int64_t>(p->g.nkeys, s.n) + direct_pieces(direct_n, direct_piece));
+  s.multi = s.piece_sums = true;
+  s.maxima = s.wsums = level != DSHT_PREC_FP64;
+  // transforms per read of the tables: the most unless tuned
+  s.tc_maps = std::min(std::max(ntrans, 1), p->tune_maps_per_pass > 0 ? p->tune_maps_per_pass : kTcMaxMaps);
+  s.fp64_maps = std::min(s.tc_maps, kFp64Maps);
+  return s;
+}
+
+size_t call_layout(const dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws) {
+  return workspace_layout(p->g, multi ? multi_spec(p, N, ntrans, p->precision)
+                                      : single_spec(p, N, p->precision, p->tmdig), base, ws);
+}
+
+// Bytes for calls of up to N points at any precision level of the plan: a size asked for once stays good
+// below each change of method and after dsht_set_precision.  (A call itself asks for its own layout only.)
+static size_t reported_size(const dsht_plan_s* p, int64_t N, int ntrans, bool multi) {
+  size_t most = 0;
+  for (int level : {DSHT_PREC_FP64, DSHT_PREC_MIXED, DSHT_PREC_MIXED_F64_TABLES}) {
+    if (!p->Yv && level != DSHT_PREC_MIXED) continue;
+    if (p->g.Nl > 2048 && level != DSHT_PREC_FP64) continue;
+    if (multi) {
+      most = std::max(most, workspace_layout(p->g, multi_spec(p, N, ntrans, level), nullptr, nullptr));
+      continue;
+    }
+    // the largest sizes below each change of method, where less is needed above it
+    const int64_t from = plan_nufft_from(p, level), below[] = {N, from - 1, DSHT_MIXED_MIN_POINTS - 1};
+    for (int64_t n : below)
+      if (n >= 0 && n <= N) {
+        const LayoutSpec s = single_spec(p, n, level, level == DSHT_PREC_MIXED && p->g.Nx <= kTcMaxNx);
+        most = std::max(most, workspace_layout(p->g, s, nullptr, nullptr));
+      }
+  }
+  return most;
 }
 
 }  // namespace dsht
@@ -793,7 +848,7 @@ int dsht_plan_info(dsht_plan_t p, int* Nl, int* Nx, double* xmax, int64_t* Nlm) 
 
 int dsht_workspace_size(dsht_plan_t p, int64_t N, size_t* bytes) {
   if (!p || !bytes || N < 0) return set_error(DSHT_ERR_INVALID, "invalid arguments");
-  *bytes = call_layout(p, N, 1, false, nullptr, nullptr);
+  *bytes = reported_size(p, N, 1, false);
   return DSHT_OK;
 }
 
@@ -951,16 +1006,18 @@ int dsht_test_layout(int Nl, int Nx, int precision, int bin_sums, int piece_max,
   dsht_plan_s p;  // never launched: the tables only have to be there
   double there = 0.0;
   p.g = make_geometry(Nl, Nx, 0.75);
+  p.Yv = &there;
   p.precision = precision;
+  p.tmdig = precision == DSHT_PREC_MIXED && Nx <= kTcMaxNx;
   p.tune_bin_sums = bin_sums;
   p.tune_piece_max = piece_max;
-  if (Nl <= 2048) p.nu_tab[0] = p.nu_tab[1] = &there;
   Workspace ws;
-  out[0] = out[1] = (int64_t)call_layout(&p, N, std::max(ntrans, 1), ntrans > 0, nullptr, &ws);
+  out[0] = (int64_t)reported_size(&p, N, std::max(ntrans, 1), ntrans > 0);
+  out[1] = (int64_t)call_layout(&p, N, std::max(ntrans, 1), ntrans > 0, nullptr, &ws);
   out[2] = ws.pmax;
-  out[3] = plan_nufft_class(&p, n);
-  out[4] = plan_piece_max(&p, n);
-  out[5] = plan_nufft_grid(&p, n);
+  out[3] = plan_nufft_class(&p, n, precision);
+  out[4] = plan_piece_max(&p, n, precision);
+  out[5] = plan_nufft_grid(&p, n, precision);
   return DSHT_OK;
 }
 
@@ -972,7 +1029,7 @@ int dsht_execute(dsht_plan_t p, const double* theta, const double* phi, const do
 int dsht_workspace_size_maps(dsht_plan_t p, int64_t N, int nmaps, size_t* bytes) {
   if (!p || !bytes || N < 0 || nmaps < 1) return set_error(DSHT_ERR_INVALID, "invalid arguments");
   // float32 single maps take the multi-transform layout too; size for it.
-  *bytes = call_layout(p, N, nmaps, true, nullptr, nullptr);
+  *bytes = reported_size(p, N, nmaps, true);
   return DSHT_OK;
 }
 
@@ -992,7 +1049,7 @@ int dsht_enqueue_maps(dsht_plan_t p, const double* theta, const double* phi, con
 
 int dsht_workspace_size_batch(dsht_plan_t p, int64_t max_N, int ntrans, size_t* bytes) {
   if (!p || !bytes || max_N < 0 || ntrans < 1) return set_error(DSHT_ERR_INVALID, "invalid arguments");
-  *bytes = call_layout(p, max_N, ntrans, true, nullptr, nullptr);
+  *bytes = reported_size(p, max_N, ntrans, true);
   return DSHT_OK;
 }
 

@@ -99,17 +99,17 @@ struct Workspace {
   uint32_t* key;        // [N]
   double* pay;          // [N][4] sorted records (cos phi, sin phi, w, t)
   uint32_t* sidx;       // [N] input index of each sorted slot (multi-map transforms)
-  uint32_t* piecemax;   // [pmax] largest |w h_k| of the piece's points (float bits)
-  double* wsum;         // [pmax] sum of |w| of the piece's points (fold digit scales)
+  uint32_t* piecemax;   // [pmax] largest |w h_k| of the piece's points (float bits; tensor-core sums)
+  double* wsum;         // [pmax] sum of |w| of the piece's points (fold digit scales), or null
   uint32_t* count;      // [nkeys + 1]
   uint32_t* offset;     // [nkeys + 1]
-  uint32_t* cursor;     // [nkeys]
+  uint32_t* cursor;     // [nkeys] (of a single transform in the place of its fold, which is written later)
   int* piece_first;     // [nkeys + 1]  first piece of each key (exclusive scan)
   int* piece_key;       // [pmax]
   int64_t* piece_start; // [pmax]
   int* piece_len;       // [pmax]
   int* npieces;         // [1]
-  int* piece_cta;       // [pmax] NUFFT sums: the CTA that takes each piece
+  int* piece_cta;       // [pmax] NUFFT sums: the CTA that takes each piece (the place of piecemax)
   int* cta_first;       // [nu_grid + 1] first piece of every CTA
   uint32_t* node_first; // [nkeys + 1] nodes with points before each key (those of its left node included)
   int nu_grid;          // CTAs of the NUFFT sums (0: the direct sums of this call leave sums per piece)
@@ -134,18 +134,10 @@ struct Workspace {
   size_t bytes;
 };
 
-// multi: add the records of multi-transform calls (gather indices, rotation and flag slots);
-// tc_maps: maps one tensor-core contraction pass holds (fold digit columns), fp64_maps: maps one
-// FP64 contraction pass holds; nu_grid: CTAs of the NUFFT sums (0: none); direct_extra: pieces beyond
-// one per key that smaller transforms on the same workspace may have.
-size_t workspace_layout(const Geometry& g, int64_t N, int piece_max, uint8_t* base, Workspace* ws, bool multi,
-                        int tc_maps, int fp64_maps, int nu_grid, int64_t direct_extra);
 // Workspace of a call of ntrans transforms of up to N points on a plan.
-size_t call_layout(dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws);
+size_t call_layout(const dsht_plan_s* p, int64_t N, int ntrans, bool multi, uint8_t* base, Workspace* ws);
 // The fold of map k of an FP64 contraction pass and where its alm go.
 FoldOut fold_slot(const Geometry& g, const Workspace& ws, int k, double* equ, double* pol, unsigned* flags);
-int default_piece_max(const Geometry& g, int64_t N);
-int plan_piece_max(const dsht_plan_s* p, int64_t N);
 // How a transform of N points runs on a plan: tensor-core bin sums (tc), tensor-core
 // contraction of the digit tables (digits), else the FP64 table streamed by TMA.
 struct Route {

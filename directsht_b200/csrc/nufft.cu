@@ -397,7 +397,7 @@ nufft_nodes_kernel(const NuArgs a, const EsPoly<W, DEG> es) {
 #pragma unroll
     for (int i = 0; i < kWarps; ++i) t += wred[i];
     t *= 1.0 + (double)len * 0x1p-52;
-    if (tid == 0) a.wsum[p] = t;
+    if (tid == 0 && a.wsum) a.wsum[p] = t;
     return t;
   };
   // the same for pieces [p, q), nothing overlapped

@@ -572,7 +572,7 @@ piecemax_kernel(const double* __restrict__ pay, const int* __restrict__ npieces_
     }
     if (lane == 0) {
       piecemax[pc] = mx;
-      wsum[pc] = ws;
+      if (wsum) wsum[pc] = ws;
     }
   }
 }
