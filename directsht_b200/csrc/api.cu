@@ -7,6 +7,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -48,6 +49,22 @@ int set_error(int code, const char* fmt, ...) {
 int set_cuda_error(cudaError_t e, const char* what, const char* file, int line) {
   return set_error(e == cudaErrorMemoryAllocation ? DSHT_ERR_NOMEM : DSHT_ERR_CUDA, "%s failed: %s (%s:%d)",
                    what, cudaGetErrorString(e), file, line);
+}
+
+cudaError_t allow_shared_memory(const void* kernel) {
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done;
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({kernel, dev})) return cudaSuccess;
+  cudaFuncAttributes a;
+  if ((e = cudaFuncGetAttributes(&a, kernel)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+  if (e == cudaSuccess) done.insert({kernel, dev});
+  return e;
 }
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

@@ -548,8 +548,7 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
 template <int CH>
 int launch_ch(const Geometry& g, const Workspace& ws, int Cf, cudaStream_t s) {
   using Lay = Layout<CH>;
-  cudaError_t e =
-      cudaFuncSetAttribute(bin_sums_tc_kernel<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::kBytes);
+  cudaError_t e = allow_shared(bin_sums_tc_kernel<CH>);
   if (e != cudaSuccess) return set_cuda_error(e, "bin_sums_tc attributes", __FILE__, __LINE__);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);

@@ -434,7 +434,7 @@ void launch_g(const Geometry& g, const TableMaps& tm, const FoldIn& in, unsigned
   for (int m = 0; m < g.Nl; ++m) nitems += (g.Nl - m + kRows - 1) / kRows;
   const int64_t grid = nitems < sms ? nitems : sms;
   const int bytes = StreamLayout<G>::bytes(nstage);
-  cudaFuncSetAttribute(contract_fp64_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  allow_shared(contract_fp64_kernel<G>);
   contract_fp64_kernel<G><<<(unsigned)grid, kThreads, bytes, s>>>(g.Nl, g.Nx, g.dx, nitems, tm, in, nstage,
                                                                   next_item, take_stall());
   count_launches(1);

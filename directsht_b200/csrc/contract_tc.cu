@@ -333,7 +333,7 @@ int tc_launch(const Geometry& g, const CUtensorMap& tmA, const uint8_t* fdig, in
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = nitems < sms ? nitems : sms;
   auto kern = contract_tc_kernel<NC>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+  allow_shared(kern);
   cudaMemsetAsync(next_item, 0, sizeof(unsigned), s);
   kern<<<grid, kTcThreads, L::kBytes, s>>>(g.Nl, kp / kChunk, tmA, tmB, items, nitems, rexp, cexp, ncols, out,
                                            next_item, take_stall());

@@ -112,7 +112,7 @@ extern "C" int dsht_mode_coupling(int Nl, const double* W, int nW, double* M, vo
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (Nl <= kMaxNl) {
     const int bytes = 5 * Nl * (int)sizeof(double);
-    DSHT_CUDA_OK(cudaFuncSetAttribute(mode_coupling_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    DSHT_CUDA_OK(allow_shared(mode_coupling_kernel));
     mode_coupling_kernel<<<Nl, kThreads, bytes, s>>>(Nl, W, nW, M);
   } else {
     const int64_t n = (int64_t)Nl * Nl;

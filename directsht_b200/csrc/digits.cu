@@ -300,7 +300,7 @@ void launch_fold_digits(const Geometry& g, const Workspace& ws, const unsigned l
   constexpr int kStageBytes = kFoldM * 2 * 4 * 4 * 2 * kStageRow;
   with_node_source(g, ws, [&](auto src) {
     auto kern = fold_digits_kernel<decltype(src)>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
+    allow_shared(kern);
     kern<<<grid, kFoldM * kFoldNodes, kStageBytes, s>>>(g.Nl, g.Nx, Kp, src, cmax, cexp, map, ncols, fdig);
   });
   count_launches(1);

@@ -145,6 +145,15 @@ struct Route {
 };
 Route plan_route(const dsht_plan_s* p, int64_t N);
 
+// Lets a kernel take all the dynamic shared memory beside its static one, once per kernel and device.  (Set
+// to a launch's own size before every launch, threads with plans of different sizes could come between
+// the setting and the launch of one another, and the larger launch failed.)
+cudaError_t allow_shared_memory(const void* kernel);
+template <typename... Args>
+cudaError_t allow_shared(void (*kernel)(Args...)) {
+  return allow_shared_memory(reinterpret_cast<const void*>(kernel));
+}
+
 // Kernels launched by api.cu (each file owns its launch helpers).
 void launch_tables(const Geometry& g, double* Yv, double* Yd, cudaStream_t s);
 void launch_points(const Geometry& g, const double* theta, const double* phi, const void* w, int w_f32,

@@ -83,7 +83,7 @@ void launch_fold(const Geometry& g, const Workspace& ws, const FoldOut& out, cud
   constexpr int kBytes = kFoldM * kRowDoubles * (int)sizeof(double);
   with_node_source(g, ws, [&](auto src) {
     auto kern = fold_kernel<decltype(src)>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+    allow_shared(kern);
     kern<<<grid, 32 * kFoldNodes, kBytes, s>>>(g.Nl, g.Nx, g.nbins, ngroups, g.dx, src, ws.offset, out);
   });
   count_launches(1);

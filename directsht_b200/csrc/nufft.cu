@@ -825,7 +825,7 @@ template <int W, int DEG, int T, bool TWO, int R1>
 int nufft_launch(const Workspace& ws, const NuArgs& a, const EsPoly<W, DEG>& es, cudaStream_t s) {
   auto kern = nufft_nodes_kernel<W, DEG, T, TWO, R1>;
   const int bytes = NuLayout<T, TWO>(a.logn).bytes(a.logn);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  const cudaError_t e = allow_shared(kern);
   if (e != cudaSuccess) return set_cuda_error(e, "nufft attributes", __FILE__, __LINE__);
   kern<<<(unsigned)ws.nu_grid, T, bytes, s>>>(a, es);
   count_launches(1);

@@ -592,7 +592,7 @@ void launch_points(const Geometry& g, const double* theta, const double* phi, co
   cudaMemsetAsync(ws.count, 0, sizeof(uint32_t) * (g.nkeys + 1), s);  // the flags follow the counts
   const size_t hsmem = sizeof(uint32_t) * g.nkeys;
   const size_t csmem = hsmem + sizeof(uint32_t) * kQueueRounds * kCountUnroll * kPointThreads;
-  cudaFuncSetAttribute(count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
+  allow_shared(count_kernel);
   if (N > 0) {
     int64_t blocks = (N + kPointThreads * 2 * kCountUnroll - 1) / (kPointThreads * 2 * kCountUnroll);
     if (blocks > 148 * 4) blocks = 148 * 4;  // fewer, longer blocks: fewer per-block key flushes
@@ -603,7 +603,7 @@ void launch_points(const Geometry& g, const double* theta, const double* phi, co
                                                                 ws.flags, guard);
     count_launches(1);
   }
-  cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem);
+  allow_shared(scan_kernel);
   scan_kernel<<<1, kScanThreads, hsmem, s>>>(g.nkeys, g.nbins, ws.piece_max, ws.pmax, ws.count, ws.offset,
                                          ws.cursor, ws.piece_first, ws.piece_key, ws.piece_start,
                                          ws.piece_len, ws.npieces, ws.node_first, ws.piece_cta, ws.cta_first,
@@ -615,7 +615,7 @@ void launch_points(const Geometry& g, const double* theta, const double* phi, co
     const int tile = scatter_tile(N, std::max(1, resident));
     const int64_t blocks = (N + tile - 1) / tile;
     auto go = [&](auto kern, const auto* wp) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem);
+      allow_shared(kern);
       kern<<<(unsigned)blocks, kPointThreads, ssmem, s>>>(g, tile, theta, phi, wp, N, ws.key, ws.cursor, ws.pay,
                                                           ws.sidx);
     };

@@ -273,7 +273,7 @@ rotate_back_kernel(int Nl, int nmaps, const RotMaps maps, const double* __restri
 template <int kMaps, int C, bool kAdd = false>
 void rotate_launch(const Geometry& g, const RotMaps& maps, int nmaps, const RotTables& t, cudaStream_t s) {
   const size_t smem = sizeof(double) * (size_t)(((g.Nl + 3) & ~3) + 2) * (1 + 2 * kMaps);
-  cudaFuncSetAttribute(rotate_back_kernel<kMaps, C, kAdd>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_shared(rotate_back_kernel<kMaps, C, kAdd>);
   dim3 grid(g.Nl, (nmaps + kMaps - 1) / kMaps);
   rotate_back_kernel<kMaps, C, kAdd><<<grid, kRotThreads, smem, s>>>(g.Nl, nmaps, maps, t.al, t.sc, t.start, t.start_e);
   count_launches(1);

@@ -76,7 +76,7 @@ void launch_table_mlayout(const Geometry& g, const double* t64, double* out, cud
 template <typename TO>
 static void tables_launch(const Geometry& g, TO* Yv, TO* Yd, int m0, int m1, cudaStream_t s) {
   const size_t smem = (size_t)g.Nl * sizeof(Coef) + (size_t)(g.Nl + 1) * sizeof(double);
-  cudaFuncSetAttribute(table_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_shared(table_kernel<TO>);
   dim3 grid((g.Nx + kTableThreads - 1) / kTableThreads, m1 - m0);
   table_kernel<TO><<<grid, kTableThreads, smem, s>>>(g.Nl, g.Nx, g.pitch, g.dx, Yv, Yd, m0, hp_index(m0, m0, g.Nl));
   count_launches(1);
