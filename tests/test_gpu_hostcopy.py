@@ -70,3 +70,22 @@ def test_other_default_device():
     a = np.random.default_rng(1).normal(size=700001)
     with torch.device("cuda"):
         np.testing.assert_array_equal(to_host(to_device(a, "cuda")), a)
+
+
+@pytest.mark.parametrize("threads", [1, 2, 4])
+def test_any_number_of_host_threads(threads):
+    """Few intra-op threads take the direct copies up to 32 MB and the staged ones above (out, or from two
+    threads in): the same bytes either way."""
+    import torch
+    from directsht_b200 import hostcopy as H
+    keep = torch.get_num_threads()
+    try:
+        torch.set_num_threads(threads)
+        small, large = H._LARGE - 8, H._LARGE + 8
+        assert [H._staged(small, 2), H._staged(large, 2), H._staged(small, 1), H._staged(large, 1)] == \
+            [threads >= 4, threads >= 2, threads >= 4, True]
+        for nbytes in (H._MIN_BYTES - 8, H._MIN_BYTES, small, large):
+            a = np.random.default_rng(threads).normal(size=nbytes // 8)
+            np.testing.assert_array_equal(H.to_host(H.to_device(a, "cuda")), a)
+    finally:
+        torch.set_num_threads(keep)
