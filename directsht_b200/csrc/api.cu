@@ -258,8 +258,15 @@ static int build_nufft(dsht_plan_s* p, int cls) {
   nufft_host_tables(p->g.Nl, cls, t, tw);
   if (p->g.Nl & 1) t.push_back(0.0);  // the twiddles start on 16 bytes
   t.insert(t.end(), tw.begin(), tw.end());
-  DSHT_CUDA_OK(cudaMalloc(&p->nu_tab[cls], sizeof(double) * t.size()));
-  DSHT_CUDA_OK(cudaMemcpy(p->nu_tab[cls], t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
+  double* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, sizeof(double) * t.size());
+  if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    cudaGetLastError();
+    return set_cuda_error(e, "tables of the NUFFT sums", __FILE__, __LINE__);
+  }
+  p->nu_tab[cls] = d;
   return DSHT_OK;
 }
 
@@ -703,18 +710,20 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
     cudaFree(p->rot_tab);
     cudaFree(p->Yv);
     cudaFree(p->Yd);
+    cudaFree(p->nu_tab[kNuFp64]);
     cudaFreeHost(p->h_flags);
     delete p;
     cudaGetLastError();
     return set_cuda_error(e, what, __FILE__, __LINE__);
   };
+  int rc = DSHT_OK;
   cudaError_t e = cudaMallocHost(&p->h_flags, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc(&p->rot_tab, rotation_table_bytes(Nl));
   if (e != cudaSuccess) return fail(e, "plan allocation");
   launch_rotation_tables(p->g, rotation_tables(p->rot_tab, Nl), 0);
   if (f32_only) {
     // compact plan: the digit tables alone, built from FP64 columns a few m at a time
-    int rc = build_digits(p);
+    rc = build_digits(p);
     if (!rc) rc = build_nufft(p, kNuMixed);
     if (rc) {
       dsht_plan_destroy(p);
@@ -729,12 +738,12 @@ int dsht_plan_create(int Nl, int Nx, double xmax, int flags, dsht_plan_t* plan) 
     if (e == cudaSuccess) e = cudaMalloc(&p->Yd, tb);
     if (e != cudaSuccess) return fail(e, "plan allocation");
     launch_tables(p->g, p->Yv, p->Yd, 0);
+    rc = build_nufft(p, kNuFp64);  // formed on the host while the device builds the tables
   }
   e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(e, "table build");
-  int rc = make_table_tmaps(&p->tmY, p->Yv, p->g);
-  if (!rc) rc = build_nufft(p, kNuFp64);
+  if (!rc) rc = make_table_tmaps(&p->tmY, p->Yv, p->g);
   if (rc) {
     dsht_plan_destroy(p);
     return rc;
