@@ -63,8 +63,7 @@ constexpr int kAnchorWarps = 4;         // warps 6-9: FP64 anchors, one block ah
 constexpr int kBThreads = 64;           // slicer threads 0-63: B tiles, 64-191: A tiles
 constexpr int kSlicers = 32 * kSlicerWarps;
 constexpr int kMmaWarp = kSlicerWarps + kAnchorWarps;  // warp 10: MMA issuer
-constexpr int kEpiWarps = 4;            // warps 11-: epilogue (4 per set of TMEM lanes 0-127)
-constexpr int kEpiSets = kEpiWarps / 4;
+constexpr int kEpiWarps = 4;            // warps 11-14: epilogue (a quarter of TMEM lanes 0-127 each)
 constexpr int kThreads = 32 * (kMmaWarp + 1 + kEpiWarps);
 constexpr int kM = 128;
 constexpr float kQf = 4193280.0f;       // 2^22 - 2^10: |X| < 2^22, so X >> 16 fits int8
@@ -470,12 +469,12 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
     }
     __syncwarp();
   } else {
-    // ==== epilogue warps: one warp per TMEM lane quarter and set of columns ==============
+    // ==== epilogue warps: one warp per TMEM lane quarter ================================
     // Lane r holds row r = 2 (16 k + a) + ri of D.  For every c:
     //   Vr = D[re, Rr] - D[im, Ri],  Vi = D[re, Ri] + D[im, Rr],
     // so each lane sends its D[., Ri] to its neighbour (lane r ^ 1) and keeps D[., Rr]:
     // the re lane writes Vr, the im lane Vi, for m = Cf a + cbase + c.
-    const int quarter = warp & 3, set = (warp - kMmaWarp - 1) >> 2;
+    const int quarter = warp & 3;
     const int r = 32 * quarter + lane;  // TMEM lane == GEMM row
     const int ri = r & 1, j = r >> 1;
     const int k = j >> 4, a = j & 15;
@@ -496,7 +495,7 @@ bin_sums_tc_kernel(int Nl, int Cf, const double* __restrict__ pay, const int* __
       if (!ok && lane == 0) fail();
       tc::tc_fence_after();
 #pragma unroll 1
-      for (int cb = 8 * set; cb < CH; cb += 8 * kEpiSets) {
+      for (int cb = 0; cb < CH; cb += 8) {
         long long T[2][8];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {

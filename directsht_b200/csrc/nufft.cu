@@ -145,11 +145,7 @@ __device__ __forceinline__ void dft4(double2& x0, double2& x1, double2& x2, doub
 
 template <int R>
 __device__ __forceinline__ void dft(double2 (&x)[R]) {
-  if constexpr (R == 2) {
-    const double2 a = x[0], b = x[1];
-    x[0] = make_double2(a.x + b.x, a.y + b.y);
-    x[1] = make_double2(a.x - b.x, a.y - b.y);
-  } else if constexpr (R == 4) {
+  if constexpr (R == 4) {
     dft4(x[0], x[1], x[2], x[3]);
   } else {
     constexpr int R2 = R / 4;
@@ -295,7 +291,6 @@ struct NuLayout {
 struct NuArgs {
   int Nl, logn, nbins;
   const double* pay;
-  const int* npieces;
   const int64_t* piece_start;
   const int* piece_len;
   const int* piece_key;
@@ -864,7 +859,6 @@ int launch_bin_sums_nufft(const Geometry& g, const Workspace& ws, const NufftTab
   a.logn = nufft_logn(g.Nl, t.cls);
   a.nbins = g.nbins;
   a.pay = ws.pay;
-  a.npieces = ws.npieces;
   a.piece_start = ws.piece_start;
   a.piece_len = ws.piece_len;
   a.piece_key = ws.piece_key;
