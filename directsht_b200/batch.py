@@ -222,6 +222,12 @@ def _profile_key(batch: TransformBatch, key) -> str:
     return f"{key[0]}x{key[1]}x{key[2]}|n={len(idx)}|" + ",".join(str(int(b)) for b in buckets)
 
 
+def piece_candidates(mixed: bool):
+    """Points per bin piece that autotune times; 0 is the automatic choice.  The NUFFT sums take at most
+    2048 or 4096 (their automatic choice), the direct sums at most 2048."""
+    return (0, 512, 1024) if mixed else (0, 512, 1024, 2048)
+
+
 def default_cache_path() -> str:
     base = os.environ.get("DSHT_TUNE_CACHE") or os.path.join(os.path.expanduser("~"), ".cache", "directsht_b200",
                                                               "autotune.json")
@@ -250,8 +256,7 @@ def autotune(batch: TransformBatch, path: str | None = None, reps: int = 2, verb
         plan = batch.cache.get(*key)
         f32 = plan.precision == "mixed"
         n = len(batch.groups[key])
-        # the NUFFT bin sums of mixed plans pay one FFT per piece: larger pieces
-        pieces = [0, 4096, 16384] if f32 else [0, 512, 1024, 2048]
+        pieces = piece_candidates(f32)
         per_pass = [0, 4] if f32 else [0]  # mixed plans: 8 (0) or 4 transforms per table read
         streams = [s for s in (1, 2, 4) if s <= n]
         best = None

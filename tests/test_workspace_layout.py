@@ -98,3 +98,12 @@ def test_what_fits_the_fixed_scratch_per_piece_fits_it():
             for N in {lo, max(1, lo - rng.randrange(300)), rng.randrange(1, lo + 1), min(lo, 1023), min(lo, 1024)}:
                 if _per_piece_layout(Nl, Nx, N, level) <= scratch:
                     assert layout(Nl, Nx, level, N, 0, 1)["bytes"] <= scratch, (Nl, Nx, N, level)
+
+
+def test_autotune_times_pieces_that_differ():
+    from directsht_b200.batch import piece_candidates
+    for level in LEVELS:
+        cand = piece_candidates(level == L.DSHT_PREC_MIXED)
+        for Nl, Nx, N in ((200, 100, 1_000_000), (1024, 300, 2_000_000), (2048, 4096, 9_000_000), (500, 1000, 100_000)):
+            got = [layout(Nl, Nx, level, N, 1, N, piece_max=c)["piece"] for c in cand if c < 2048]
+            assert len(set(got)) == len(got), (level, Nl, Nx, N, got)
