@@ -79,3 +79,29 @@ def test_gpu_mode_coupling_edges(Nl, nW):
     M = mode_coupling_matrix(Nl, W)
     ref = O.mode_coupling_closed_form(Nl, full)
     assert np.abs(M - ref).max() <= 1e-12 * max(np.abs(ref).max(), 1e-300)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Nl,tol", [(5700, 1e-12), (5701, 1e-9)])
+def test_gpu_mode_coupling_on_both_sides_of_the_table_limit(Nl, tol):
+    """Up to Nl = 5700 the binomials are tabulated in shared memory (a few 1e-15); above, each symbol is
+    walked from a first value by lgamma, whose arguments give values up to 1e5: 4 ulp of each of the six,
+    1.5e-10 of the entry, and 5700 steps of a dozen roundings, 8e-12 (all terms of a positive W add)."""
+    import ctypes as ct
+
+    import torch
+    from directsht_b200 import _lib as L
+    W = np.random.default_rng(Nl).uniform(0.5, 1.5, 2 * Nl - 1)
+    Wd, M = torch.from_numpy(W).cuda(), torch.empty((Nl, Nl), dtype=torch.float64, device="cuda")
+    L.check(L.load().dsht_mode_coupling(Nl, L.ptr(Wd), len(W), L.ptr(M), ct.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    n = np.arange(1, 2 * Nl - 1, dtype=np.longdouble)
+    q = np.concatenate([[np.longdouble(1)], np.cumprod((2 * n - 1) / (2 * n))])  # C(2n, n) / 4^n
+    for l1 in (0, 1, 2850, Nl - 2, Nl - 1):
+        row = M[l1].cpu().numpy()
+        for l2 in (0, 1, 17, 2850, 4000, Nl - 1):
+            a, b = max(l1, l2), min(l1, l2)
+            i = np.arange(b + 1)
+            l3, g = a - b + 2 * i, a + i
+            w2 = q[g - l1] * q[g - l2] * q[g - l3] / (q[g] * (2 * g + 1))
+            ref = float(((2 * l3 + 1) * W[l3] * w2).sum() * (2 * l2 + 1) / (4 * np.pi))
+            assert abs(row[l2] - ref) <= tol * ref, (l1, l2)
