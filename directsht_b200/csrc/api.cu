@@ -545,9 +545,9 @@ static int run_class_fp64(dsht_plan_s* p, const Item* items, const std::vector<i
 // Several transforms in one call: multi-map transforms (one point set, the later maps marked
 // same_points) and batches of independent transforms on one plan.  Each point set is
 // classified and sorted once; a same_points item only gathers its weights into the sorted
-// payload.  Bin sums and the fold run per item.  On the digit tables the contraction runs
-// in passes of up to ws.tc_maps items that share one read of the tables
-// (run_class_digits); on the FP64 tables once per item.  Equatorial alm go straight to
+// payload.  Bin sums and the fold run per item.  The contraction runs in passes of items that
+// share one read of the tables: up to ws.tc_maps on the digit tables (run_class_digits), up to
+// ws.fp64_maps on the FP64 table (run_class_fp64).  Equatorial alm go straight to
 // item.alm, polar alm to a rotation slot, and one batched rotation per kMaxRot slots adds
 // them back.  Items with N < DSHT_MIXED_MIN_POINTS on a mixed plan run the FP64 bin sums,
 // in their own class.

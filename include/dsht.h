@@ -144,7 +144,7 @@ int dsht_plan_info(dsht_plan_t plan, int* Nl, int* Nx, double* xmax, int64_t* Nl
 /* Healpy index m(2Nl-1-m)/2 + l (sht/sht.py:58-67). */
 int64_t dsht_index(int Nl, int ell, int m);
 
-/* Bytes of device workspace dsht_execute needs for N points. */
+/* Bytes of device workspace for dsht_execute of N points, at every precision level of the plan. */
 int dsht_workspace_size(dsht_plan_t plan, int64_t N, size_t* bytes);
 
 /* Forward transform of N points given by DEVICE pointers theta, phi, w (float64).
@@ -219,7 +219,7 @@ int dsht_rotate_back(dsht_plan_t plan, const double* alm_rot, const double* alm_
  * cudaMalloc/cudaFree.  Same arguments and results as dsht_execute (DEVICE pointers), but
  * all scratch lives in one fixed device array of dsht_noalloc_scratch_bytes() = 64 MiB
  * that every GPU loading this library holds until exit; problems whose workspace is larger
- * return DSHT_ERR_NOMEM.  With the default piece size, Nl=256, Nx=512, N=1e5 fits (63.8 MB);
+ * return DSHT_ERR_NOMEM.  With the default piece size, Nl=256, Nx=512, N=1e5 fits (60.9 MB);
  * a plan tuned to smaller pieces (DSHT_TUNE_PIECE_MAX) needs more: check a problem with
  * dsht_workspace_size(plan, N) <= dsht_noalloc_scratch_bytes() beforehand.  Like
  * dsht_execute, each call waits for its stream once at the end to read the error flags,
