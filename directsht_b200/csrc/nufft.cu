@@ -271,6 +271,10 @@ __device__ __forceinline__ void fft_node(double2* z, int logn, const double2* __
 
 constexpr int kMeta = 64;  // descriptors of upcoming pieces kept in shared memory
 
+// The FP64 class's kernel values carry this power of two: a grid's transform sums the several cells of
+// every point, and weights near the largest double must not overflow there where their sums do not.
+constexpr double kRange = 0x1p-8;
+
 // Shared memory of a launch: the grids, the twiddles, the sorted points' indices, then the warps'
 // staging areas, which the cell counters share.
 template <int T, bool TWO>
@@ -619,7 +623,7 @@ nufft_nodes_kernel(const NuArgs a, const EsPoly<W, DEG> es) {
   // Finishes a node: its sums to a slot, the grid cleared.
   auto emit = [&](double2* z, int64_t slot_out, double scale) {
     __syncthreads();
-    fft_node<R1>(z, logn, tws, Nl, kExact ? 1.0 / scale : 1.0, a.dinv, a.slots + (size_t)slot_out * 4 * Nl);
+    fft_node<R1>(z, logn, tws, Nl, kExact ? 1.0 / scale : 1.0 / kRange, a.dinv, a.slots + (size_t)slot_out * 4 * Nl);
     __syncthreads();
     clear(z);
   };
@@ -731,11 +735,11 @@ std::vector<double> make_es_poly(const EsShape& e) {
 }
 
 template <int W, int DEG>
-EsPoly<W, DEG> half_poly(const EsShape& e) {
+EsPoly<W, DEG> half_poly(const EsShape& e, double scale) {
   const std::vector<double> c = make_es_poly(e);
   EsPoly<W, DEG> P;
   for (int i = 0; i < W / 2; ++i)
-    for (int d = 0; d <= DEG; ++d) P.c[i][d] = c[(size_t)i * (DEG + 1) + d];
+    for (int d = 0; d <= DEG; ++d) P.c[i][d] = scale * c[(size_t)i * (DEG + 1) + d];
   return P;
 }
 
@@ -869,10 +873,11 @@ int launch_bin_sums_nufft(const Geometry& g, const Workspace& ws, const NufftTab
   a.slots = ws.partial;
   a.wsum = t.cls == kNuMixed ? ws.wsum : nullptr;
   if (t.cls == kNuMixed) {
-    static const EsPoly<12, 11> P = half_poly<12, 11>(es_shape(kNuMixed, 0));
+    static const EsPoly<12, 11> P = half_poly<12, 11>(es_shape(kNuMixed, 0), 1.0);
     return nufft_go(ws, a, P, s);
   }
-  static const EsPoly<16, 15> P2 = half_poly<16, 15>(es_shape(kNuFp64, 0)), P4 = half_poly<16, 15>(es_shape(kNuFp64, 1));
+  static const EsPoly<16, 15> P2 = half_poly<16, 15>(es_shape(kNuFp64, 0), kRange);
+  static const EsPoly<16, 15> P4 = half_poly<16, 15>(es_shape(kNuFp64, 1), kRange);
   return nufft_go(ws, a, g.Nl <= 256 ? P4 : P2, s);
 }
 

@@ -85,3 +85,18 @@ def test_weights_that_are_not_finite_reach_every_coefficient():
         d = DirectSHT(20, 12)
         d.tune(bin_sums="nufft")
         assert not np.isfinite(d(th, ph, w)).any()
+
+
+@pytest.mark.parametrize("scale", [2.0**1013, 2.0**-1000])
+def test_weights_at_the_ends_of_the_range(scale):
+    """Weights near the largest double (their sums still finite) and tiny ones: the alm are those of the
+    unscaled weights times the power of two, as with the direct sums."""
+    from directsht_b200 import DirectSHT
+    rng = np.random.default_rng(8)
+    th, ph, w = np.arccos(rng.uniform(-0.7, 0.7, 3000)), rng.uniform(0, 2 * np.pi, 3000), rng.normal(size=3000)
+    w[5] = 1000.0
+    d = DirectSHT(20, 12)
+    for method in ("fp64", "nufft"):
+        d.tune(bin_sums=method)
+        ref, got = d(th, ph, w), d(th, ph, w * scale) / scale
+        assert np.isfinite(ref).all() and np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max(), method
